@@ -668,7 +668,7 @@ def run_fft(args):
                                  for k, (c, t) in prof.items()}}
         solver.close()
     C = wl.nslice * wl.ngrid ** 2
-    alg = {"fft_rows_fwd": 32 * C, "fft_cols": 32 * C, "fft_rows_inv": 32 * C}
+    alg = {"fft_rows": 32 * C, "fft_cols": 32 * C}
     peak, kind = measured_peak()
     k = out["fft"]["kernels"]
     dom = max((n for n in k if n in alg), key=lambda n: k[n]["avg_ms"])

@@ -79,6 +79,28 @@ def test_fft_step_matches_oracle(ctx, ngrid, filt):
     assert synth.rel_err(got, ref) < 1e-12, synth.rel_err(got, ref)
 
 
+# every edge of the line transform and its tiles: 64 threads of four inputs
+# per line, four lines per CTA, up to 2 n - 1 = 511
+@pytest.mark.parametrize("ngrid", [2, 3, 63, 64, 65, 66, 128, 129, 192, 193, 254, 256])
+@pytest.mark.parametrize("filt", [None, (0.3, 0.25, 0.1)])
+def test_fft_step_at_the_edges_of_its_tiles(ctx, ngrid, filt):
+    nslice, gridmax = 2, 2e-4
+    off, p = synth.beam(nslice, 300, seed=ngrid, ragged=True)
+    cur = np.array([2000.0, 900.0])
+    cells = synth.field(nslice, ngrid, gridmax, seed=ngrid + 3, amplitude=1e12)
+    st = synth.und_step(kx=0.5 * synth.KU ** 2, ky=0.5 * synth.KU ** 2)
+    fc = synth.coupling()
+    ref = cells.copy()
+    xc, yc, sig = filt if filt else (0.0, 0.0, 0.0)
+    orc.fft_advance(ref, harm=1, gridmax=gridmax, xks=2 * np.pi / synth.LAMBDA0, delz=st.delz,
+                    fc=fc, enabled=True, step=st, off=off, current=cur, parts=p, first=1,
+                    xc=xc, yc=yc, sig=sig)
+    got = _gpu_fft_step(ctx, cells, harm=1, gridmax=gridmax, xlambda=synth.LAMBDA0, first=1,
+                        delz=st.delz, fc=fc, step=st, off=off, current=cur, parts=p,
+                        filt=filt)
+    assert synth.rel_err(got, ref) < 1e-12, synth.rel_err(got, ref)
+
+
 def test_fft_pure_diffraction_is_unitary_and_reversible(ctx):
     """No source: the propagator has |exp(i k2 dz)| = 1, so the power is kept,
     and a step of -dz undoes a step of +dz."""
