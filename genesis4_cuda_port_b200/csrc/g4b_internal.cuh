@@ -384,10 +384,16 @@ __device__ __forceinline__ void fence_tensormap_acquire(const void* map) {
 
 // Programmatic dependent launch (launch_pdl): block until the preceding
 // kernel of the stream has completed and its writes are visible (returns at
-// once in a kernel launched without the attribute).  No kernel triggers its
-// dependents early: they launch as its last CTAs exit, which hides the
-// launch latency and the ramp-up, not the tail.
+// once in a kernel launched without the attribute).  Kernels do not trigger
+// their dependents early (they launch as the last CTAs exit, which hides the
+// launch latency and the ramp-up, not the tail), with one exception that says
+// so: pdl_launch_dependents lets the next kernel start beside this one, and
+// that kernel itself waits (pdl_wait) before it ends, so that its completion
+// implies this one's.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ void bulk_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");

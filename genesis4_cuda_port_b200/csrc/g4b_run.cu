@@ -29,6 +29,7 @@
 #include <map>
 #include <new>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "g4b_internal.cuh"
@@ -40,6 +41,7 @@ constexpr int kStepThreads = 128;  // beam step: two particles per thread
 constexpr int kStepBlocks = 8;     // resident beam-step CTAs per SM (<= 64 registers)
 constexpr int kStepWarps = kStepThreads / 32;
 constexpr int kMaxBunch = 8;
+constexpr int kRunMaxNp = 65536;   // particles per slice (deposition scale)
 constexpr int kBeamRec = 23;  // reference stats order (DiagnosticCUDA.cpp:102-125)
 
 struct MixField {
@@ -481,11 +483,14 @@ struct DepField {
   float2* src;        // compact tiles, cap cells per slice
   int4* desc;
   int4* bbox;
-  int* mpred;         // [nslice][kDepSplit] M of the slice's previous deposition (0: none)
+  int* mpred;         // [nslice] M of the slice's previous deposition (0: none)
+  float* qpred;       // [nslice] largest charge weight of the previous deposition (0: none)
+  unsigned char* tiles;  // [nslice] DepTile, zero between launches (runs of few slices)
+  int tile_cells;
   size_t cap;
   int first, n, ld, nslice, harm, do_source;
   float gridmax, dgrid, inv_dgrid;
-  double fc, xks, dgrid_d;
+  double kscl;        // source scale times particles over current
 };
 
 struct DepArgs {
@@ -494,7 +499,6 @@ struct DepArgs {
   const double* th;
   const int64_t* off;
   const double* current;
-  float* qpred;       // [nslice][kDepSplit] largest charge weight of the previous deposition (0: none)
   DepField f[kRunFields];
   int nfield;
   float ax, ay, kx, ky, gradx, grady, gref_f;
@@ -509,105 +513,123 @@ struct BeamDiagArgs {
   const int64_t* off;
   int nbunch, need_aux;
   double gref;
-  double* beam_part;  // [nslice * kDepParts][23 + 2*nbunch] records
+  double* beam_hist;  // [nslice][23 + 2*nbunch] records of this step
 };
 
-// Beam diagnostics (DiagnosticCUDA.cpp:102-125), kDepParts CTAs per slice,
-// each over an equal share of the slice's particles: one pass with FP64
-// sums (the minima and maxima in FP32, exact for FP32 state) into a record
-// of the final layout; the finalize combines a slice's records in a fixed
-// order (sums, minima and maxima of records are the record of the union).
-// Independent of the deposition, so it runs beside it and the ADI passes.
-constexpr int kDepParts = 1;          // beam-diagnostic records per slice
+// Beam diagnostics (DiagnosticCUDA.cpp:102-125): FP64 sums, the minima and
+// maxima in FP32 (exact for FP32 state).  The order of the sums is fixed by
+// the slice alone, so any number of CTAs gives the same bits: a
+// unit of kDiagUnit consecutive particles is summed by one warp (eight per
+// lane in order, then the lanes in a tree), unit j belongs to group j mod
+// kDiagGroups, a group adds its units in order and the groups are added in a
+// tree, both with compensation (csum_*).
 constexpr int kDiagThreads = 256;
-constexpr int kDepDiagU = 8;          // particles in flight per thread
+constexpr int kDiagU = 8;             // particles of a unit per lane, all in flight
+constexpr int kDiagUnit = 32 * kDiagU;
+constexpr int kDiagGroups = 32;
+constexpr int kDiagSums = 12;         // x, x^2, y, y^2, px, px^2, py, py^2, x px, y py, dg, dg^2
 
-// U: particles in flight per thread (each thread adds its particles in the
-// same order for every U, so the sums do not depend on it)
-template <int NB, int U = kDepDiagU>
-__device__ __forceinline__ void diag_slice(const BeamDiagArgs& a, const int bs, const int part) {
-  __shared__ double dpart[kDiagThreads / 32][kBeamRec + 2 * kMaxBunch];
-  __shared__ double bcomp[kDiagThreads / 32][2 * kMaxBunch];  // bunching compensations
-  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
-  const int nall = (int)(a.off[bs + 1] - a.off[bs]);  // at most kRunMaxNp per slice
-  const int per = (nall + kDepParts - 1) / kDepParts;
-  const int first = min(part * per, nall);
-  const int64_t p0 = a.off[bs] + first;
-  const int np = min(per, nall - first);
-  const float2* xyp = a.xy + p0;
-  const float2* pxyp = a.pxy + p0;
-  const float* dgp = a.dg + p0;
-  const double* thp = a.th + p0;
-  const int rec = kBeamRec + 2 * a.nbunch;
-  double sm[12];  // sums of x, x^2, y, y^2, px, px^2, py, py^2, x px, y py, dg, dg^2
+// The groups' sums of a slice, in shared memory.
+template <int NB>
+struct DiagGroups {
+  static constexpr int Q = NB <= 2 ? 16 : 32;  // sums, padded: kDiagSums + 2 NB
+  double2 sum[kDiagGroups][Q];          // (sum, compensation)
+  float ext[kDiagGroups][10];           // per warp: min, max of x, px, y, py, dg
+};
+
+// This lane's sum of one unit: quantity lane / (32 / Q).  The lanes are added
+// in a butterfly that halves the quantities a lane carries at every level: 15
+// exchanges for 16 quantities where a tree per quantity takes 80.
+template <int NB>
+__device__ __forceinline__ double diag_unit(const BeamDiagArgs& a, const float2* xyp,
+                                            const float2* pxyp, const float* dgp,
+                                            const double* thp, const int np, const int p0,
+                                            float (&mn)[5], float (&mx)[5]) {
+  constexpr int Q = DiagGroups<NB>::Q;
+  const int lane = threadIdx.x & 31;
+  float2 lxy[kDiagU], lpp[kDiagU];
+  float ldg[kDiagU];
+  double lth[kDiagU];
 #pragma unroll
-  for (int k = 0; k < 12; ++k) sm[k] = 0.0;
+  for (int u = 0; u < kDiagU; ++u) {
+    const int p = p0 + 32 * u + lane;
+    if (p < np) {
+      lxy[u] = xyp[p];
+      lpp[u] = pxyp[p];
+      ldg[u] = dgp[p];
+      lth[u] = thp[p];
+    }
+  }
+  double v[Q];
+#pragma unroll
+  for (int k = 0; k < Q; ++k) v[k] = 0.0;
+#pragma unroll
+  for (int u = 0; u < kDiagU; ++u) {
+    if (p0 + 32 * u + lane >= np) break;
+    const double x = lxy[u].x, y = lxy[u].y, px = lpp[u].x, py = lpp[u].y;
+    const double d = ldg[u];
+    v[0] += x; v[1] = __fma_rn(x, x, v[1]);
+    v[2] += y; v[3] = __fma_rn(y, y, v[3]);
+    v[4] += px; v[5] = __fma_rn(px, px, v[5]);
+    v[6] += py; v[7] = __fma_rn(py, py, v[7]);
+    v[8] = __fma_rn(x, px, v[8]); v[9] = __fma_rn(y, py, v[9]);
+    v[10] += d; v[11] = __fma_rn(d, d, v[11]);
+    if (a.need_aux) {
+      const float f[5] = {lxy[u].x, lpp[u].x, lxy[u].y, lpp[u].y, ldg[u]};
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        mn[i] = fminf(mn[i], f[i]);
+        mx[i] = fmaxf(mx[i], f[i]);
+      }
+    }
+    float s1, c1;
+    __sincosf(reduce_angle(lth[u]), &s1, &c1);
+    float ch = c1, sh = s1;
+#pragma unroll
+    for (int h = 0; h < NB; ++h) {
+      if (h >= a.nbunch) break;
+      v[kDiagSums + 2 * h] += ch;
+      v[kDiagSums + 2 * h + 1] += sh;
+      const float nc = __fmaf_rn(ch, c1, -__fmul_rn(sh, s1));
+      const float ns = __fmaf_rn(sh, c1, __fmul_rn(ch, s1));
+      ch = nc;
+      sh = ns;
+    }
+  }
+#pragma unroll
+  for (int o = 16, h = Q / 2; o > 0; o >>= 1, h >>= 1) {
+    if (h > 0) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int k = 0; k < Q / 2; ++k) {
+        if (k >= h) break;
+        const double give = up ? v[k] : v[k + h];
+        v[k] = (up ? v[k + h] : v[k]) + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return v[0];
+}
+
+// The groups of slice bs by warp w of nw.
+template <int NB>
+__device__ __forceinline__ void diag_groups(const BeamDiagArgs& a, const int bs, const int w,
+                                            const int nw, DiagGroups<NB>& G) {
+  constexpr int Q = DiagGroups<NB>::Q;
+  const int lane = threadIdx.x & 31;
+  const int64_t p0 = a.off[bs];
+  const int np = (int)(a.off[bs + 1] - p0);  // at most kRunMaxNp per slice
   // minima / maxima of x, px, y, py (reference start values -+1e5) and dg
   float mn[5] = {1.0e5f, 1.0e5f, 1.0e5f, 1.0e5f, INFINITY};
   float mx[5] = {-1.0e5f, -1.0e5f, -1.0e5f, -1.0e5f, -INFINITY};
-  // bunching sums: each thread adds its FP32 terms (at most 256: 65536
-  // particles over 256 threads) in FP64, within 2^-45 of their magnitude;
-  // the warp and the CTA's warps add with compensation (csum_*)
-  double bre[NB], bim[NB];
-#pragma unroll
-  for (int h = 0; h < NB; ++h) bre[h] = bim[h] = 0.0;
-  // in a wider CTA only the first kDiagThreads threads sum (the same layout)
-  for (int pb = tid < kDiagThreads ? tid : np; pb < np; pb += U * kDiagThreads) {
-    float2 lxy[U], lpp[U];
-    float ldg[U];
-    double lth[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int p = pb + u * kDiagThreads;
-      if (p < np) {
-        lxy[u] = xyp[p];
-        lpp[u] = pxyp[p];
-        ldg[u] = dgp[p];
-        lth[u] = thp[p];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (pb + u * kDiagThreads >= np) break;
-      const double x = lxy[u].x, y = lxy[u].y, px = lpp[u].x, py = lpp[u].y;
-      const double d = ldg[u];
-      sm[0] += x; sm[1] = __fma_rn(x, x, sm[1]);
-      sm[2] += y; sm[3] = __fma_rn(y, y, sm[3]);
-      sm[4] += px; sm[5] = __fma_rn(px, px, sm[5]);
-      sm[6] += py; sm[7] = __fma_rn(py, py, sm[7]);
-      sm[8] = __fma_rn(x, px, sm[8]); sm[9] = __fma_rn(y, py, sm[9]);
-      sm[10] += d; sm[11] = __fma_rn(d, d, sm[11]);
-      if (a.need_aux) {
-        const float f[5] = {lxy[u].x, lpp[u].x, lxy[u].y, lpp[u].y, ldg[u]};
-#pragma unroll
-        for (int i = 0; i < 5; ++i) {
-          mn[i] = fminf(mn[i], f[i]);
-          mx[i] = fmaxf(mx[i], f[i]);
-        }
-      }
-      float s1, c1;
-      __sincosf(reduce_angle(lth[u]), &s1, &c1);
-      float ch = c1, sh = s1;
-#pragma unroll
-      for (int h = 0; h < NB; ++h) {
-        if (h >= a.nbunch) break;
-        bre[h] += ch;
-        bim[h] += sh;
-        const float nc = __fmaf_rn(ch, c1, -__fmul_rn(sh, s1));
-        const float ns = __fmaf_rn(sh, c1, __fmul_rn(ch, s1));
-        ch = nc;
-        sh = ns;
-      }
-    }
-  }
-  // per-warp records in the layout of the final one: [0] sum dg,
-  // [1] sum dg^2, [2..11] the sums of x .. y py, [13..22] minima / maxima
-  // of x, px, y, py, dg
-#pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    double t = sm[k];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (l == 0 && w < kDiagThreads / 32) dpart[w][k < 10 ? k + 2 : k - 10] = t;
+  for (int g = w; g < kDiagGroups; g += nw) {
+    double s = 0.0, c = 0.0;
+    for (int u0 = g * kDiagUnit; u0 < np; u0 += kDiagGroups * kDiagUnit)
+      ptx::csum_add(s, c, diag_unit<NB>(a, a.xy + p0, a.pxy + p0, a.dg + p0, a.th + p0, np, u0,
+                                        mn, mx));
+    if (lane % (32 / Q) == 0) G.sum[g][lane / (32 / Q)] = make_double2(s, c);
   }
 #pragma unroll
   for (int i = 0; i < 5; ++i) {
@@ -616,62 +638,73 @@ __device__ __forceinline__ void diag_slice(const BeamDiagArgs& a, const int bs, 
       lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
       hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
-    if (l == 0 && w < kDiagThreads / 32) {
-      dpart[w][13 + 2 * i] = lo;
-      dpart[w][14 + 2 * i] = hi;
+    if (lane == 0) {
+      G.ext[w][2 * i] = lo;
+      G.ext[w][2 * i + 1] = hi;
     }
-  }
-#pragma unroll
-  for (int h = 0; h < NB; ++h) {
-    if (h >= a.nbunch) break;
-    double tr = bre[h], trc = 0.0, ti = bim[h], tic = 0.0;
-    ptx::csum_warp(tr, trc, 32);
-    ptx::csum_warp(ti, tic, 32);
-    if (l == 0 && w < kDiagThreads / 32) {
-      dpart[w][kBeamRec + 2 * h] = tr;
-      dpart[w][kBeamRec + 2 * h + 1] = ti;
-      bcomp[w][2 * h] = trc;
-      bcomp[w][2 * h + 1] = tic;
-    }
-  }
-  __syncthreads();
-  if (tid < rec) {
-    // record (DiagnosticCUDA.cpp:102-125): [0] sum gamma, [1] sum gamma^2,
-    // [12] count, [21] / [22] min / max gamma from the dg extremes (gamma
-    // = gref + dg is monotonic in dg)
-    const double N = (double)np;
-    const int op = tid < 13 ? 0 : (tid < kBeamRec ? ((tid - 13) % 2 == 0 ? 1 : 2) : 0);
-    double t = N;
-    if (tid >= kBeamRec) {  // bunching: the warps' compensated partials
-      const int q = tid - kBeamRec;
-      double tc = bcomp[0][q];
-      t = dpart[0][tid];
-      for (int i = 1; i < kDiagThreads / 32; ++i) ptx::csum_merge(t, tc, dpart[i][tid], bcomp[i][q]);
-      t += tc;
-    } else if (tid != 12) {
-      t = dpart[0][tid];
-      for (int i = 1; i < kDiagThreads / 32; ++i) {
-        const double u = dpart[i][tid];
-        t = op == 0 ? t + u : (op == 1 ? fmin(t, u) : fmax(t, u));
-      }
-    }
-    if (tid == 0) t = __fma_rn(N, a.gref, t);
-    if (tid == 1) {
-      double sd = dpart[0][0];
-      for (int i = 1; i < kDiagThreads / 32; ++i) sd += dpart[i][0];
-      t = __fma_rn(__dmul_rn(N, a.gref), a.gref, __fma_rn(__dmul_rn(2.0, a.gref), sd, t));
-    }
-    if (tid == 21) t = fmin(1.0e7, a.gref + t);
-    if (tid == 22) t = fmax(1.0, a.gref + t);
-    if (tid >= 13 && tid < kBeamRec && !a.need_aux) t = 0.0;
-    a.beam_part[((size_t)bs * kDepParts + part) * rec + tid] = t;
   }
 }
 
-template <int NB>
+// The slice's record from the groups' sums and the warps' extremes, by a whole
+// CTA of T threads: a warp per quantity, a lane per group.
+template <int NB, int T>
+__device__ __forceinline__ void diag_record(const BeamDiagArgs& a, const int bs,
+                                            const DiagGroups<NB>& G) {
+  constexpr int kWarps = T / 32;
+  __shared__ double total[kDiagSums + 2 * kMaxBunch];
+  __shared__ float bound[10];
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  for (int q = w; q < kDiagSums + 2 * a.nbunch; q += kWarps) {
+    double2 t = G.sum[lane][q];
+    ptx::csum_warp(t.x, t.y, 32);
+    if (lane == 0) total[q] = t.x + t.y;
+  }
+  for (int q = w; q < 10; q += kWarps) {
+    float t = G.ext[lane < kWarps ? lane : 0][q];
+    for (int o = 16; o > 0; o >>= 1) {
+      const float u = __shfl_xor_sync(0xffffffffu, t, o);
+      t = q % 2 == 0 ? fminf(t, u) : fmaxf(t, u);
+    }
+    if (lane == 0) bound[q] = t;
+  }
+  __syncthreads();
+  const int rec = kBeamRec + 2 * a.nbunch;
+  if (tid >= rec) return;
+  // record (DiagnosticCUDA.cpp:102-125): [0] sum gamma, [1] sum gamma^2,
+  // [2..11] the sums of x .. y py, [12] count, [13..22] minima / maxima of x,
+  // px, y, py, gamma (gamma = gref + dg is monotonic in dg), then bunching
+  const double N = (double)(a.off[bs + 1] - a.off[bs]);
+  double t = N;
+  if (tid >= kBeamRec) {
+    t = total[kDiagSums + tid - kBeamRec];
+  } else if (tid >= 13) {
+    t = bound[tid - 13];
+    if (tid == 21) t = fmin(1.0e7, a.gref + t);
+    if (tid == 22) t = fmax(1.0, a.gref + t);
+    if (!a.need_aux) t = 0.0;
+  } else if (tid == 0) {
+    t = __fma_rn(N, a.gref, total[10]);
+  } else if (tid == 1) {
+    t = __fma_rn(__dmul_rn(N, a.gref), a.gref,
+                 __fma_rn(__dmul_rn(2.0, a.gref), total[10], total[11]));
+  } else if (tid != 12) {
+    t = total[tid - 2];
+  }
+  a.beam_hist[(size_t)bs * rec + tid] = t;
+}
+
+template <int NB, bool BESIDE>
 __global__ void __launch_bounds__(kDiagThreads, 2)
     beam_diag_kernel(const __grid_constant__ BeamDiagArgs a) {
-  diag_slice<NB>(a, blockIdx.x / kDepParts, blockIdx.x % kDepParts);
+  __shared__ DiagGroups<NB> G;
+  // launched beside the deposition (deposit_kernel): the beam step, whose
+  // output it reads, is complete; the wait for the deposition at its end makes
+  // this kernel's completion imply the deposition's
+  if (!BESIDE) ptx::pdl_wait();
+  diag_groups<NB>(a, blockIdx.x, threadIdx.x >> 5, kDiagThreads / 32, G);
+  __syncthreads();
+  diag_record<NB, kDiagThreads>(a, blockIdx.x, G);
+  if (BESIDE) ptx::pdl_wait();
 }
 
 // Deposition (adi_deposit_source_atomic, FieldSolverADICUDA.cpp:98-174),
@@ -696,19 +729,41 @@ __global__ void __launch_bounds__(kDiagThreads, 2)
 // approximation (absolute error below 2^-21.4 on that interval).  Every
 // rounding that could be fused differently is written out with intrinsics,
 // so the single-run and the batched kernels give the same bits.  The tile is
-// the slice's bounding box of touched cells (from K1); tiles larger than
-// kDepMaxCells are processed in row bands.
-constexpr int kDepThreads = 256;
-// CTAs per slice: CTA `part` takes the tile's row bands part, part +
-// kDepSplit, ... (a tile of one band leaves the second CTA idle; one of two
-// bands is done by two CTAs side by side instead of one after the other)
-constexpr int kDepSplit = 2;
-constexpr int kDepAccU = 4;           // particles in flight per thread
-constexpr int kDepWideThreads = 512;  // the deposition CTA of runs of few slices
-constexpr int kDepMaxCells = 8192;    // output cells per band (a multiple of 4)
+// the slice's bounding box of touched cells (from K1); larger tiles
+// are processed in row bands.
+//
+// A slice belongs to one CTA, which holds a band in shared memory; in runs of
+// few slices C CTAs take 1/C of its particles each and add to a tile in global
+// memory (DepTile), and the last of them to finish writes the source.  The
+// integer sums, hence the bits, are the same for every C.
+constexpr int kDepThreads = 512;
+constexpr double kDepUnit = 1073741824.0;  // 2^30
 constexpr int kDepMaxWidth = 896;     // tile width bound: mixed ngrid <= 880
-// re and im planes, then the counts per base cell ((hb + 1) bw <= cells + width)
-constexpr size_t kDepSmem = (size_t)(3 * kDepMaxCells + kDepMaxWidth) * 4;
+// Output cells per band (a multiple of 4) where two CTAs share an SM and where
+// one has it: re and im planes, then the counts per base cell ((hb + 1) bw <=
+// cells + width) in shared memory
+constexpr int kDepCells2 = 9216, kDepCells1 = 18432;
+constexpr size_t dep_smem(int cells) { return (size_t)(3 * cells + kDepMaxWidth) * 4; }
+// Tile of one slice: `cells` sums im 2^32 + re, the counts per base cell
+// (one row more), the bits of the largest charge weight and the CTAs done.
+constexpr int kDepTileCells = 65536;  // at most
+struct DepTile {
+  unsigned long long* sum;
+  int* hist;
+  int* qmax;
+  unsigned* done;
+};
+__host__ __device__ constexpr size_t dep_tile_bytes(int cells) {
+  return (size_t)cells * 8 + (size_t)(cells + kDepMaxWidth) * 4 + 128;
+}
+__device__ __forceinline__ DepTile dep_tile(unsigned char* tiles, int cells, int bs) {
+  DepTile t;
+  t.sum = reinterpret_cast<unsigned long long*>(tiles + bs * dep_tile_bytes(cells));
+  t.hist = reinterpret_cast<int*>(t.sum + cells);
+  t.qmax = t.hist + cells + kDepMaxWidth;
+  t.done = reinterpret_cast<unsigned*>(t.qmax + 1);
+  return t;
+}
 
 // Charge weight sqrt(faw2) / gamma of one particle (FP32).
 __device__ __forceinline__ float dep_charge(const DepArgs& a, const float2 xy, const float dg) {
@@ -720,281 +775,524 @@ __device__ __forceinline__ float dep_charge(const DepArgs& a, const float2 xy, c
   return __fdividef(sqrtf(faw2), a.gref_f + dg);
 }
 
-// T threads per CTA, U particles in flight per thread: the integer sums and
-// the maxima do not depend on either, so every instance gives the same bits.
-template <int T = kDepThreads, int U = kDepAccU>
-__device__ __forceinline__ void deposit_slice(const DepArgs& a, const int bs, const int part,
-                                              unsigned char* smem) {
-  __shared__ int4 sbox[kRunFields];
+// One field's source tile of one slice.
+struct DepSlice {
+  int bs, np, target;
+  const float2* xy;
+  const float* dg;
+  const double* th;
+  double scl;
+  int bx0, by0, bw, bh;
+  int m_use;     // bound M' of the contributions (0: no previous deposition)
+  float q_use;   // bound q' of the charge weights (0: no previous deposition)
+  MixField mf;
+  float fh, inv_bw;
+  __device__ __forceinline__ bool predicted() const {
+    return m_use > 0 && q_use > 0.f && q_use < 3.0e38f;
+  }
+  // the predicted bounds' M' q': the scale is 2^30 / (M' q')
+  __device__ __forceinline__ double bound() const { return (double)m_use * (double)q_use; }
+};
+
+// False (and no source, which thread 0 of the caller with `lead` writes): no
+// particle in the grid, no current, or a tile the kernels do not take.
+__device__ __forceinline__ bool dep_setup(const DepArgs& a, const DepField& F, const int bs,
+                                          const bool lead, DepSlice& d) {
+  d.bs = bs;
+  const int64_t p0 = a.off[bs];
+  d.np = (int)(a.off[bs + 1] - p0);  // at most kRunMaxNp per slice
+  d.xy = a.xy + p0;
+  d.dg = a.dg + p0;
+  d.th = a.th + p0;
+  d.target = (bs + F.first) % F.nslice;
+  const int4 bb = F.bbox[bs];
+  // M and qmax of this slice's previous deposition of this field bound the
+  // contributions of the single-pass form
+  const int mprev = F.mpred[bs];
+  d.m_use = mprev > 0 ? mprev + (mprev >> 2) + 4 : 0;
+  d.q_use = F.qpred[bs] * 1.015625f;
+  d.scl = 0.0;
+  if (d.np > 0) d.scl = F.kscl * a.current[bs] / (double)d.np;
+  d.bx0 = bb.x;
+  d.bw = bb.z - bb.x + 2;
+  d.by0 = bb.y;
+  d.bh = bb.w - bb.y + 2;
+  const bool none = bb.z < 0 || d.scl == 0.0;
+  if (!none && (d.bw & 1)) {  // even tile width keeps the rows 16-byte aligned
+    ++d.bw;
+    if (d.bx0 + d.bw > F.ld) --d.bx0;
+  }
+  const bool wide = !none && d.bw > kDepMaxWidth;  // excluded by g4b_run_create's ngrid limit
+  if (lead && threadIdx.x == 0) {
+    if (wide) atomicOr(a.err, kErrBadSlice);
+    F.desc[d.target] = none || wide ? make_int4(0, 0, 0, 0) : make_int4(d.bx0, d.by0, d.bw, d.bh);
+  }
+  if (none || wide) return false;
+  d.fh = (float)F.harm;
+  d.inv_bw = 1.0f / (float)d.bw;
+  d.mf.gridmax = F.gridmax;
+  d.mf.dgrid = F.dgrid;
+  d.mf.inv_dgrid = F.inv_dgrid;
+  d.mf.n = F.n;
+  return true;
+}
+
+// The rounded contributions of one particle of scaled charge weight q: (re, im)
+// of the lower corners (ix, ix + 1), then of the upper ones.
+__device__ __forceinline__ void dep_corners(const DepSlice& d, const float2 xy, const double th,
+                                            const float q, int (&c)[8]) {
+  float sn, cs;
+  __sincosf(reduce_angle((double)d.fh * th), &sn, &cs);
+  const float vre = sn * q, vim = cs * q;
+  int ix, iy;
+  float x0, y0;
+  cell_f(d.mf, xy.x, xy.y, ix, iy, x0, y0);  // the weights
+  const float w00 = x0 * y0, w10 = (1.f - x0) * y0, w01 = x0 * (1.f - y0),
+              w11 = (1.f - x0) * (1.f - y0);
+  c[0] = __float2int_rn(vre * w00);
+  c[1] = __float2int_rn(vim * w00);
+  c[2] = __float2int_rn(vre * w10);
+  c[3] = __float2int_rn(vim * w10);
+  c[4] = __float2int_rn(vre * w01);
+  c[5] = __float2int_rn(vim * w01);
+  c[6] = __float2int_rn(vre * w11);
+  c[7] = __float2int_rn(vim * w11);
+}
+
+// Adds the particles [plow, phigh) of the slice to the rows ylo .. ylo + hb - 1:
+// with `count` the counts per base cell (ext row iy - ylo + 1) and the largest
+// charge weight (qloc), with `add` the contributions at scale Sf of charge
+// weights capped at qc.  One particle per lane, the next one's loads in
+// flight.  Four consecutive particles of one base cell (a quiet-start beamlet,
+// nbins = 4 particles at one transverse position) are summed over their lanes,
+// each of which adds one corner, with one count (the same integer sums).
+// GLOBAL: to a DepTile; else to planes in shared memory.
+template <int T, bool GLOBAL>
+__device__ __forceinline__ void dep_pass(const DepArgs& a, const DepSlice& d, const int plow,
+                                         const int phigh, const int ylo, const int hb, int* are,
+                                         int* aim, unsigned long long* packed, int* hist,
+                                         const bool count,
+                                         const bool add, const float Sf, const float qc,
+                                         float& qloc) {
+  const int tid = threadIdx.x, l = tid & 31;
+  const int bw = d.bw, nout = hb * bw;
+  auto add2 = [&](int o, int re, int im) {
+    if (GLOBAL) {
+      atomicAdd(&packed[o], ((unsigned long long)(unsigned)im << 32) +
+                                (unsigned long long)(long long)re);
+    } else {
+      atomicAdd(&are[o], re);
+      atomicAdd(&aim[o], im);
+    }
+  };
+  float2 nxy = make_float2(0.f, 0.f);
+  float ndg = 0.f;
+  double nth = 0.0;
+  auto load = [&](int p) {
+    if (p < phigh) {
+      nxy = d.xy[p];
+      ndg = d.dg[p];
+      if (add) nth = d.th[p];
+    }
+  };
+  load(plow + tid);
+  for (int p = plow + tid; p - l < phigh; p += T) {  // whole warps
+    const float2 xy = nxy;
+    const float dg = ndg;
+    const double th = nth;
+    load(p + T);
+    int cid = -1, ix, iy;
+    float x0, y0;
+    if (p < phigh && cell_f(d.mf, xy.x, xy.y, ix, iy, x0, y0) && iy + 1 >= ylo && iy < ylo + hb) {
+      const int ex = ix - d.bx0;
+      if (ex < 0 || ex > bw - 2) {
+        if (count) atomicOr(a.err, kErrBadSlice);
+      } else {
+        cid = (iy - ylo + 1) * bw + ex;
+      }
+    }
+    const int lead = __shfl_sync(0xffffffffu, cid, l & ~3);
+    const unsigned match = __ballot_sync(0xffffffffu, cid >= 0 && cid == lead);
+    const bool same = ((match >> (l & ~3)) & 15u) == 15u;
+    if (count) {
+      const int n = same ? ((l & 3) == 0 ? 4 : 0) : (cid >= 0 ? 1 : 0);
+      if (n > 0) atomicAdd(&hist[cid], n);
+    }
+    // contributions to the lower corners (row ey - 1) and the upper ones, (re, im)
+    int c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (cid >= 0) {
+      const float qraw = dep_charge(a, xy, dg);
+      if (count) qloc = fmaxf(qloc, qraw);
+      if (add) dep_corners(d, xy, th, fminf(qraw, qc) * Sf, c);
+    }
+    if (!add) continue;
+    // a beamlet's sums: lane l ends with the corner of row (l & 2), column (l & 1)
+    const bool up = (l & 2) != 0, right = (l & 1) != 0;
+    int k[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      k[i] = (up ? c[4 + i] : c[i]) + __shfl_xor_sync(0xffffffffu, up ? c[i] : c[4 + i], 2);
+    const int re = (right ? k[2] : k[0]) + __shfl_xor_sync(0xffffffffu, right ? k[0] : k[2], 1);
+    const int im = (right ? k[3] : k[1]) + __shfl_xor_sync(0xffffffffu, right ? k[1] : k[3], 1);
+    if (same) {
+      if (up ? cid < nout : cid >= bw) add2((up ? cid : cid - bw) + (right ? 1 : 0), re, im);
+    } else if (cid >= 0) {
+      if (cid >= bw) {  // lower corners: output row ey = cid / bw - 1
+        add2(cid - bw, c[0], c[1]);
+        add2(cid - bw + 1, c[2], c[3]);
+      }
+      if (cid < nout) {  // upper corners: row ey + 1 inside the band
+        add2(cid, c[4], c[5]);
+        add2(cid + 1, c[6], c[7]);
+      }
+    }
+  }
+}
+
+// Counts and contributions to shared memory by threads that take a group of four
+// consecutive particles each (16-byte loads where the slice starts on a
+// multiple of four): more work in flight per thread, for CTAs that have an SM,
+// or half of one, to themselves at up to 128 registers.
+template <int T>
+__device__ __forceinline__ void dep_pass4(const DepArgs& a, const DepSlice& d, const int ylo,
+                                          const int hb, int* are, int* aim, int* hist,
+                                          const float Sf, const float qc, float& qloc) {
+  const int bw = d.bw, nout = hb * bw;
+  const bool wide = ((uintptr_t)d.dg & 15) == 0;  // d.dg + 4 g, hence d.xy and d.th too
+  auto add8 = [&](int cid, const int* v) {
+    if (cid >= bw) {  // lower corners: output row ey = cid / bw - 1
+      const int o = cid - bw;
+      atomicAdd(&are[o], v[0]);
+      atomicAdd(&aim[o], v[1]);
+      atomicAdd(&are[o + 1], v[2]);
+      atomicAdd(&aim[o + 1], v[3]);
+    }
+    if (cid < nout) {  // upper corners: row ey + 1 inside the band
+      atomicAdd(&are[cid], v[4]);
+      atomicAdd(&aim[cid], v[5]);
+      atomicAdd(&are[cid + 1], v[6]);
+      atomicAdd(&aim[cid + 1], v[7]);
+    }
+  };
+  for (int pg = 4 * threadIdx.x; pg < d.np; pg += 4 * T) {
+    float2 lxy[4];
+    float ldg[4];
+    double lth[4];
+    if (wide && pg + 3 < d.np) {
+      const float4 u = *reinterpret_cast<const float4*>(d.xy + pg);
+      const float4 v = *reinterpret_cast<const float4*>(d.xy + pg + 2);
+      const float4 q = *reinterpret_cast<const float4*>(d.dg + pg);
+      lxy[0] = make_float2(u.x, u.y);
+      lxy[1] = make_float2(u.z, u.w);
+      lxy[2] = make_float2(v.x, v.y);
+      lxy[3] = make_float2(v.z, v.w);
+      ldg[0] = q.x;
+      ldg[1] = q.y;
+      ldg[2] = q.z;
+      ldg[3] = q.w;
+      const double2 s = *reinterpret_cast<const double2*>(d.th + pg);
+      const double2 t = *reinterpret_cast<const double2*>(d.th + pg + 2);
+      lth[0] = s.x;
+      lth[1] = s.y;
+      lth[2] = t.x;
+      lth[3] = t.y;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (pg + u < d.np) {
+          lxy[u] = d.xy[pg + u];
+          ldg[u] = d.dg[pg + u];
+          lth[u] = d.th[pg + u];
+        }
+      }
+    }
+    int cid[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      cid[u] = -1;
+      int ix, iy;
+      float wx, wy;
+      if (pg + u < d.np && cell_f(d.mf, lxy[u].x, lxy[u].y, ix, iy, wx, wy) && iy + 1 >= ylo &&
+          iy < ylo + hb) {
+        const int ex = ix - d.bx0;
+        if (ex < 0 || ex > bw - 2) {
+          atomicOr(a.err, kErrBadSlice);
+        } else {
+          cid[u] = (iy - ylo + 1) * bw + ex;
+        }
+      }
+    }
+    const bool same = cid[0] >= 0 && cid[1] == cid[0] && cid[2] == cid[0] && cid[3] == cid[0];
+    if (same) {
+      atomicAdd(&hist[cid[0]], 4);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (cid[u] >= 0) atomicAdd(&hist[cid[u]], 1);
+    }
+    int sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (cid[u] < 0) continue;
+      const float qraw = dep_charge(a, lxy[u], ldg[u]);
+      qloc = fmaxf(qloc, qraw);
+      int c[8];
+      dep_corners(d, lxy[u], lth[u], fminf(qraw, qc) * Sf, c);
+      if (same) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sum[k] += c[k];
+      } else {
+        add8(cid[u], c);
+      }
+    }
+    if (same) add8(cid[0], sum);
+  }
+}
+
+// Block maximum of M and of the charge weight.
+template <int T>
+__device__ __forceinline__ void dep_max(int& M, float& q) {
   __shared__ int wsum[T / 32];
   __shared__ float wmax[T / 32];
-  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
-  const int64_t p0 = a.off[bs];
-  const int np = (int)(a.off[bs + 1] - p0);  // at most kRunMaxNp per slice
-  const float2* xyp = a.xy + p0;
-  const float* dgp = a.dg + p0;
-  const double* thp = a.th + p0;
-  if (tid < a.nfield) sbox[tid] = a.f[tid].bbox[bs];
-  const float qprev = a.qpred[bs * kDepSplit + part];
-  const float q_use = qprev * 1.015625f;  // 0 without a previous deposition
-  float q_seen = 0.f;
-  bool deposited = false;
-  __syncthreads();  // sbox is read by every thread below
+  M = __reduce_max_sync(0xffffffffu, M);
+  for (int o = 16; o > 0; o >>= 1) q = fmaxf(q, __shfl_xor_sync(0xffffffffu, q, o));
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+    wsum[threadIdx.x >> 5] = M;
+    wmax[threadIdx.x >> 5] = q;
+  }
+  __syncthreads();
+  M = wsum[0];
+  q = wmax[0];
+  for (int i = 1; i < T / 32; ++i) {
+    M = max(M, wsum[i]);
+    q = fmaxf(q, wmax[i]);
+  }
+}
 
-  // ---- deposition of every field with a source this step ----
+// Two neighbouring source cells (bw and the cell counts are even, the rows
+// 16-byte aligned).
+__device__ __forceinline__ void dep_write(float2* out, int2 re, int2 im, double unscale) {
+  *reinterpret_cast<float4*>(out) =
+      make_float4((float)((double)re.x * unscale), (float)((double)im.x * unscale),
+                  (float)((double)re.y * unscale), (float)((double)im.y * unscale));
+}
+
+// The rare passes (counts alone, or the contributions alone), out of line.
+template <int T>
+__device__ __noinline__ float dep_rare(const DepArgs& a, const DepSlice d, const int ylo,
+                                       const int hb, int* are, int* aim, int* hist,
+                                       const bool count, const float Sf, const float qc) {
+  float q = 0.f;
+  dep_pass<T, false>(a, d, 0, d.np, ylo, hb, are, aim, nullptr, hist, count, !count, Sf, qc, q);
+  return q;
+}
+
+// One field of a slice by a whole CTA, band by band of at most CELLS cells in
+// shared memory; FOUR: by dep_pass4.  With a prediction one pass takes counts,
+// qmax and contributions at the scale of the predicted bounds; it is kept if
+// neither counted bound exceeds its prediction (then no cell sum can have
+// overflowed and no charge was capped), else the contributions are redone at
+// the exact scale 2^30 / (M qmax).  Without one, a first pass only counts.  M
+// and qmax are the slice's, whatever its bands.
+template <int T, bool FOUR, int CELLS>
+__device__ __forceinline__ void deposit_field(const DepArgs& a, const DepField& F,
+                                              const DepSlice& d, unsigned char* smem) {
+  const int tid = threadIdx.x, bw = d.bw;
   int* are = reinterpret_cast<int*>(smem);        // [hb * bw] real parts
-  int* aim = are + kDepMaxCells;                  // [hb * bw] imaginary parts
-  int* hist = aim + kDepMaxCells;                 // [(hb + 1) * bw] counts per base cell
-  const double npd = (double)np;
+  int* aim = are + CELLS;                         // [hb * bw] imaginary parts
+  int* hist = aim + CELLS;                        // [(hb + 1) * bw] counts per base cell
+  const int hband = max(1, CELLS / bw);           // bw <= ngrid + 1 < CELLS
+  auto zero = [&](int* p, int n) {
+    for (int i = tid; i < (n + 3) >> 2; i += T) reinterpret_cast<int4*>(p)[i] = make_int4(0, 0, 0, 0);
+  };
+  int M = 0;
+  float qm = 0.f;
+  bool count = true, add = d.predicted();
+  double B = d.bound();  // the scale is kDepUnit / B
+  float qc = d.q_use;
+  for (;;) {
+    const float Sf = (float)(kDepUnit / B);
+    const double unscale = d.scl * (B * (1.0 / kDepUnit));
+    for (int yb = 0; yb < d.bh; yb += hband) {
+      const int hb = min(hband, d.bh - yb), nout = hb * bw;
+      __syncthreads();
+      if (count) zero(hist, (hb + 1) * bw);
+      if (add) {
+        zero(are, nout);
+        zero(aim, nout);
+      }
+      __syncthreads();
+      if (!(count && add))
+        qm = fmaxf(qm, dep_rare<T>(a, d, d.by0 + yb, hb, are, aim, hist, count, Sf, qc));
+      else if (FOUR)
+        dep_pass4<T>(a, d, d.by0 + yb, hb, are, aim, hist, Sf, qc, qm);
+      else
+        dep_pass<T, false>(a, d, 0, d.np, d.by0 + yb, hb, are, aim, nullptr, hist, true, true, Sf,
+                           qc, qm);
+      __syncthreads();
+      // the cells' sums, and the largest number M of contributions any output
+      // cell receives (its four base cells' counts); row of cell o: (o + 1/2)
+      // / bw in FP32 is never within nout 2^-23 / bw of an integer boundary,
+      // so the truncation is exact
+      float2* out = F.src + (size_t)d.target * F.cap + (size_t)yb * bw;
+      for (int o = 2 * tid; o < nout; o += 2 * T) {
+        if (add)
+          dep_write(out + o, *reinterpret_cast<const int2*>(are + o),
+                    *reinterpret_cast<const int2*>(aim + o), unscale);
+        if (!count) continue;
+        const int x = o - (int)(((float)o + 0.5f) * d.inv_bw) * bw;
+        const int2 up = *reinterpret_cast<const int2*>(hist + o),
+                   dn = *reinterpret_cast<const int2*>(hist + o + bw);
+        const int left = x > 0 ? hist[o - 1] + hist[o + bw - 1] : 0;
+        M = max(M, max(left + up.x + dn.x, up.x + dn.x + up.y + dn.y));
+      }
+    }
+    if (!count) break;
+    dep_max<T>(M, qm);
+    if (M == 0 || !(qm > 0.f) || !(qm < 3.0e38f)) {
+      if (M > 0) atomicOr(a.err, kErrFixedRange);  // non-finite charge
+      float2* out = F.src + (size_t)d.target * F.cap;
+      for (int i = tid; i < d.bh * bw; i += T) out[i] = make_float2(0.f, 0.f);
+      qm = 0.f;
+      break;
+    }
+    if (add && M <= d.m_use && qm <= d.q_use) break;
+    count = false;
+    add = true;
+    B = (double)M * (double)qm;
+    qc = qm;
+  }
+  if (tid == 0) {
+    F.mpred[d.bs] = M;
+    if (qm > 0.f) F.qpred[d.bs] = qm;
+  }
+}
+
+template <int T, bool FOUR, int CELLS>
+__device__ __forceinline__ void deposit_slice(const DepArgs& a, const int bs, unsigned char* smem) {
   for (int fi = 0; fi < a.nfield; ++fi) {
     const DepField& F = a.f[fi];
-    if (!F.do_source) continue;
-    const int target = (bs + F.first) % F.nslice;
-    const int4 bb = sbox[fi];
-    // adi_compute_slice_scl (src/Core/FieldSolverADICUDA.cpp:75-96)
-    double scl = 0.0;
-    if (npd > 0) {
-      scl = F.fc * 376.73031346177 * a.current[bs] * F.xks * a.delz;
-      scl /= 4.0 * 510998.95 * npd * F.dgrid_d * F.dgrid_d;
-    }
-    if (bb.z < 0 || scl == 0.0) {
-      if (tid == 0 && part == 0) F.desc[target] = make_int4(0, 0, 0, 0);
-      continue;
-    }
-    int bx0 = bb.x, bw = bb.z - bb.x + 2;
-    const int by0 = bb.y, bh = bb.w - bb.y + 2;
-    if (bw & 1) {  // even tile width keeps the rows 16-byte aligned
-      ++bw;
-      if (bx0 + bw > F.ld) --bx0;
-    }
-    if (bw > kDepMaxWidth) {  // excluded by g4b_run_create's ngrid limit
-      if (tid == 0 && part == 0) {
-        atomicOr(a.err, kErrBadSlice);
-        F.desc[target] = make_int4(0, 0, 0, 0);
-      }
-      continue;
-    }
-    if (tid == 0 && part == 0) F.desc[target] = make_int4(bx0, by0, bw, bh);
-    const int hband = max(1, kDepMaxCells / bw);  // bw <= ngrid + 1 < kDepMaxCells
-    const float fh = (float)F.harm;
-    // row of output cell o: (o + 1/2) / bw in FP32 is never within
-    // nout 2^-23 / bw of an integer boundary, so the truncation is exact
-    const float inv_bw = 1.0f / (float)bw;
-    MixField mf;
-    mf.gridmax = F.gridmax;
-    mf.dgrid = F.dgrid;
-    mf.inv_dgrid = F.inv_dgrid;
-    mf.n = F.n;
-    // M of this slice's previous deposition of this field (0: none yet)
-    // bounds the contributions of the single-pass form below
-    const int mprev = F.mpred[bs * kDepSplit + part];
-    const int m_use = mprev > 0 ? mprev + (mprev >> 2) + 4 : 0;
-    int m_seen = 0;
-    for (int yb = part * hband; yb < bh; yb += kDepSplit * hband) {
-      const int hb = min(hband, bh - yb);
-      const int ylo = by0 + yb;  // first grid row of this band
-      const int nout = hb * bw, nbase = (hb + 1) * bw;
-      // with `count` the counts per base cell (ext row iy - ylo + 1) and the
-      // largest charge weight (qloc), with `add` the contributions at scale
-      // Sf of charge weights capped at qc.  A thread takes groups of four
-      // consecutive particles: a quiet-start beamlet (nbins = 4 particles at
-      // one transverse position) when the four share a base cell, whose
-      // rounded contributions it sums in registers and adds, with its count,
-      // by one set of atomics instead of four (the same integer sums).
-      float qloc = 0.f;
-      auto add8 = [&](int cid, const int* v) {
-        if (cid >= bw) {  // lower corners: output row ey = cid / bw - 1
-          const int o = cid - bw;
-          atomicAdd(&are[o], v[0]);
-          atomicAdd(&aim[o], v[1]);
-          atomicAdd(&are[o + 1], v[2]);
-          atomicAdd(&aim[o + 1], v[3]);
-        }
-        if (cid < nout) {  // upper corners: row ey + 1 inside the band
-          atomicAdd(&are[cid], v[4]);
-          atomicAdd(&aim[cid], v[5]);
-          atomicAdd(&are[cid + 1], v[6]);
-          atomicAdd(&aim[cid + 1], v[7]);
-        }
-      };
-      auto pass = [&](const bool count, const bool add, const float Sf, const float qc) {
-        for (int g = tid; 4 * g < np; g += T) {
-          const int pg = 4 * g;
-          float2 lxy[4];
-          float ldg[4];
-          double lth[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (pg + u < np) {
-              lxy[u] = xyp[pg + u];
-              ldg[u] = dgp[pg + u];
-              if (add) lth[u] = thp[pg + u];
-            }
-          }
-          int cid[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            cid[u] = -1;
-            int ix, iy;
-            float wx, wy;
-            if (pg + u < np && cell_f(mf, lxy[u].x, lxy[u].y, ix, iy, wx, wy) &&
-                iy + 1 >= ylo && iy < ylo + hb) {
-              const int ex = ix - bx0;
-              if (ex < 0 || ex > bw - 2) {
-                if (count) atomicOr(a.err, kErrBadSlice);
-              } else {
-                cid[u] = (iy - ylo + 1) * bw + ex;
-              }
-            }
-          }
-          const bool same = cid[0] >= 0 && cid[1] == cid[0] && cid[2] == cid[0] &&
-                            cid[3] == cid[0];
-          if (count) {
-            if (same) {
-              atomicAdd(&hist[cid[0]], 4);
-            } else {
-#pragma unroll
-              for (int u = 0; u < 4; ++u)
-                if (cid[u] >= 0) atomicAdd(&hist[cid[u]], 1);
-            }
-          }
-          int sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (cid[u] < 0) continue;
-            const float qraw = dep_charge(a, lxy[u], ldg[u]);
-            if (count) qloc = fmaxf(qloc, qraw);
-            if (!add) continue;
-            const float q = fminf(qraw, qc) * Sf;
-            float sn, cs;
-            __sincosf(reduce_angle((double)fh * lth[u]), &sn, &cs);
-            const float vre = sn * q, vim = cs * q;
-            int ix, iy;
-            float x0, y0;
-            cell_f(mf, lxy[u].x, lxy[u].y, ix, iy, x0, y0);  // the weights again
-            const float w00 = x0 * y0, w10 = (1.f - x0) * y0, w01 = x0 * (1.f - y0),
-                        w11 = (1.f - x0) * (1.f - y0);
-            const int c[8] = {__float2int_rn(vre * w00), __float2int_rn(vim * w00),
-                              __float2int_rn(vre * w10), __float2int_rn(vim * w10),
-                              __float2int_rn(vre * w01), __float2int_rn(vim * w01),
-                              __float2int_rn(vre * w11), __float2int_rn(vim * w11)};
-            if (same) {
-#pragma unroll
-              for (int k = 0; k < 8; ++k) sum[k] += c[k];
-            } else {
-              add8(cid[u], c);
-            }
-          }
-          if (add && same) add8(cid[0], sum);
-        }
-      };
-      auto zero_acc = [&]() {
-        int4* r4 = reinterpret_cast<int4*>(are);
-        int4* i4 = reinterpret_cast<int4*>(aim);
-        for (int i = tid; i < (nout + 3) >> 2; i += T) {
-          r4[i] = make_int4(0, 0, 0, 0);
-          i4[i] = make_int4(0, 0, 0, 0);
-        }
-      };
-      __syncthreads();
-      {
-        int4* h4 = reinterpret_cast<int4*>(hist);
-        for (int i = tid; i < (nbase + 3) >> 2; i += T) h4[i] = make_int4(0, 0, 0, 0);
-      }
-      const bool single = m_use > 0 && q_use > 0.f && q_use < 3.0e38f;
-      double S = 0.0;
-      if (single) {
-        // one pass: counts, qmax and contributions at the scale of the
-        // predicted bounds; kept if neither counted bound exceeds its
-        // prediction (then no cell sum can have overflowed and no charge was
-        // capped), else redone below at the exact scale
-        S = 1073741824.0 / ((double)m_use * (double)q_use);  // 2^30 / (M' q')
-        zero_acc();
-        __syncthreads();
-        pass(true, true, (float)S, q_use);
-      } else {
-        __syncthreads();
-        pass(true, false, 0.f, 0.f);
-      }
-      __syncthreads();
-      // the largest number M of contributions any output cell receives
-      int mloc = 0;
-      for (int o = tid; o < nout; o += T) {
-        const int r = (int)(((float)o + 0.5f) * inv_bw), x = o - r * bw;
-        int m = hist[(r + 1) * bw + x] + hist[r * bw + x];
-        if (x > 0) m += hist[(r + 1) * bw + x - 1] + hist[r * bw + x - 1];
-        mloc = max(mloc, m);
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        mloc = max(mloc, __shfl_xor_sync(0xffffffffu, mloc, o));
-        qloc = fmaxf(qloc, __shfl_xor_sync(0xffffffffu, qloc, o));
-      }
-      if (l == 0) {
-        wsum[w] = mloc;
-        wmax[w] = qloc;
-      }
-      __syncthreads();
-      int M = wsum[0];
-      float qm = wmax[0];
-      for (int i = 1; i < T / 32; ++i) {
-        M = max(M, wsum[i]);
-        qm = fmaxf(qm, wmax[i]);
-      }
-      m_seen = max(m_seen, M);
-      float2* out = F.src + (size_t)target * F.cap + (size_t)yb * bw;
-      if (M == 0 || !(qm > 0.f) || !(qm < 3.0e38f)) {
-        if (M > 0) atomicOr(a.err, kErrFixedRange);  // non-finite charge
-        for (int i = tid; i < nout; i += T) out[i] = make_float2(0.f, 0.f);
-        continue;
-      }
-      q_seen = fmaxf(q_seen, qm);
-      deposited = true;
-      if (!single || M > m_use || qm > q_use) {
-        S = 1073741824.0 / ((double)M * (double)qm);  // 2^30 / (M qmax)
-        zero_acc();
-        __syncthreads();
-        pass(false, true, (float)S, qm);
-      }
-      __syncthreads();
-      const double unscale = scl / S;
-      for (int i = tid; i < nout; i += T)
-        out[i] = make_float2((float)((double)are[i] * unscale), (float)((double)aim[i] * unscale));
-    }
-    if (tid == 0 && part * hband < bh) F.mpred[bs * kDepSplit + part] = m_seen;
+    DepSlice d;
+    if (F.do_source && dep_setup(a, F, bs, true, d)) deposit_field<T, FOUR, CELLS>(a, F, d, smem);
   }
-  if (tid == 0 && deposited) a.qpred[bs * kDepSplit + part] = q_seen;
 }
 
-__global__ void __launch_bounds__(kDepThreads, 2) deposit_kernel(const __grid_constant__ DepArgs a) {
+// Part `rank` of C of a slice: the particles [rank, rank + 1) / C into the
+// slice's DepTile; the CTA whose count comes last reads it, writes the source
+// and leaves the tile zero for the next launch.  A field without a prediction,
+// one whose prediction fails and one larger than its tile are done by that CTA
+// in shared memory.
+
+template <int T>
+__device__ __forceinline__ void deposit_part(const DepArgs& a, const int bs, const int rank,
+                                             const int C, unsigned char* smem) {
+  __shared__ int last;
+  const int tid = threadIdx.x;
+  for (int fi = 0; fi < a.nfield; ++fi) {
+    const DepField& F = a.f[fi];
+    DepSlice d;
+    if (!F.do_source || !dep_setup(a, F, bs, rank == 0, d)) continue;
+    const int bw = d.bw, nout = d.bh * bw, nbase = (d.bh + 1) * bw;
+    const DepTile t = dep_tile(F.tiles, F.tile_cells, bs);
+    // true in the CTA of the slice that comes here last (every CTA has then
+    // read the prediction, which that one replaces)
+    auto is_last = [&]() {
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) last = atomicAdd(t.done, 1u) == (unsigned)C - 1u;
+      __syncthreads();
+      if (last) __threadfence();
+      return last != 0;
+    };
+    if (!d.predicted() || nout > F.tile_cells) {
+      if (is_last()) {
+        if (tid == 0) *t.done = 0;
+        deposit_field<T, false, kDepCells1>(a, F, d, smem);
+      }
+      continue;
+    }
+    const int share = (((d.np + 3) >> 2) + C - 1) / C * 4, plow = rank * share;
+    float qm = 0.f;
+    dep_pass<T, true>(a, d, plow, min(d.np, plow + share), d.by0, d.bh, nullptr, nullptr, t.sum,
+                      t.hist, true, true, (float)(kDepUnit / d.bound()), d.q_use, qm);
+    for (int o = 16; o > 0; o >>= 1) qm = fmaxf(qm, __shfl_xor_sync(0xffffffffu, qm, o));
+    if ((tid & 31) == 0 && qm > 0.f) atomicMax(t.qmax, __float_as_int(qm));
+    if (!is_last()) continue;
+    float2* out = F.src + (size_t)d.target * F.cap;
+    const double unscale = d.scl * (d.bound() * (1.0 / kDepUnit));
+    int M = 0;
+    for (int o = 2 * tid; o < nout; o += 2 * T) {
+      const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(t.sum + o));
+      const int x = o - (int)(((float)o + 0.5f) * d.inv_bw) * bw;
+      const int2 up = __ldcg(reinterpret_cast<const int2*>(t.hist + o)),
+                 dn = __ldcg(reinterpret_cast<const int2*>(t.hist + o + bw));
+      const int left = x > 0 ? __ldcg(t.hist + o - 1) + __ldcg(t.hist + o + bw - 1) : 0;
+      const int2 re = make_int2((int)(unsigned)v.x, (int)(unsigned)v.y);
+      dep_write(out + o, re,
+                make_int2((int)((v.x - re.x) >> 32), (int)((v.y - re.y) >> 32)), unscale);
+      M = max(M, max(left + up.x + dn.x, up.x + dn.x + up.y + dn.y));
+    }
+    qm = __int_as_float(__ldcg(t.qmax));
+    dep_max<T>(M, qm);  // (every cell has been read)
+    for (int o = 2 * tid; o < nbase; o += 2 * T) {
+      if (o < nout) *reinterpret_cast<int4*>(t.sum + o) = make_int4(0, 0, 0, 0);
+      *reinterpret_cast<int2*>(t.hist + o) = make_int2(0, 0);
+    }
+    if (tid == 0) {
+      *t.qmax = 0;
+      *t.done = 0;
+    }
+    if (M > d.m_use || !(qm <= d.q_use)) {
+      deposit_field<T, false, kDepCells1>(a, F, d, smem);
+    } else if (tid == 0) {
+      F.mpred[bs] = M;
+      F.qpred[bs] = qm;
+    }
+  }
+}
+
+// A CTA per slice.  BESIDE: lets the next kernel (beam_diag_kernel) start
+// beside this one, once every CTA runs or has ended.
+template <bool BESIDE>
+__global__ void __launch_bounds__(kDepThreads, 2)
+    deposit_kernel(const __grid_constant__ DepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   ptx::pdl_wait();
-  deposit_slice(a, blockIdx.x / kDepSplit, blockIdx.x % kDepSplit, smem);
+  if (BESIDE) ptx::pdl_launch_dependents();
+  deposit_slice<kDepThreads, false, kDepCells2>(a, blockIdx.x, smem);
 }
 
-// The beam diagnostics and the deposition of a slice by one CTA, one after
-// the other: the form of runs too small to fill the GPU (a graph branch for
-// their diagnostics would cost more to instantiate than it saves).  Runs of
-// fewer slices than SMs take T = 512 threads, twice the particles in flight
-// of a 256-thread CTA for the deposition; the diagnostics use the first
-// kDiagThreads threads, so every form gives the same bits.
+// Fewer slices than SMs: per slice one CTA for the beam diagnostics and the
+// others for the deposition, side by side.
 struct DepDiagLaunch {
   DepArgs d;
   BeamDiagArgs b;
+  int parts;
 };
+
+template <int NB, int T>
+__device__ __forceinline__ void deposit_diag_part(const DepArgs& d, const BeamDiagArgs& b,
+                                                  const int bs, const int part, const int parts,
+                                                  unsigned char* smem) {
+  if (part == parts - 1) {
+    DiagGroups<NB>& G = *reinterpret_cast<DiagGroups<NB>*>(smem);
+    diag_groups<NB>(b, bs, threadIdx.x >> 5, T / 32, G);
+    __syncthreads();
+    diag_record<NB, T>(b, bs, G);
+  } else if (parts == 2) {
+    deposit_slice<T, true, T == 512 ? kDepCells1 : kDepCells2>(d, bs, smem);
+  } else {
+    deposit_part<T>(d, bs, part, parts - 1, smem);
+  }
+}
 
 template <int NB, int T>
 __global__ void __launch_bounds__(T, 512 / T)
     deposit_diag_kernel(const __grid_constant__ DepDiagLaunch a) {
   extern __shared__ __align__(128) unsigned char smem[];
   ptx::pdl_wait();
-  const int bs = blockIdx.x / kDepSplit, part = blockIdx.x % kDepSplit;
-  // the last part takes the diagnostics: a tile of one band leaves it no
-  // deposition, so the slice's diagnostics and deposition run side by side
-  if (part == kDepSplit - 1) {
-    diag_slice<NB>(a.b, bs, 0);
-    __syncthreads();
-  }
-  deposit_slice<T, kDepAccU>(a.d, bs, part, smem);
+  deposit_diag_part<NB, T>(a.d, a.b, blockIdx.x / a.parts, blockIdx.x % a.parts, a.parts, smem);
 }
 
 // Batched forms: items[i] = (run, slice of that run).
@@ -1007,10 +1305,10 @@ struct DepBatchArgs {
 __global__ void __launch_bounds__(kDepThreads, 2)
     deposit_batch_kernel(const __grid_constant__ DepBatchArgs b) {
   extern __shared__ __align__(128) unsigned char smem[];
-  const int nitems = *b.nitems * kDepSplit;
+  const int nitems = *b.nitems;
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const int2 w = b.items[it / kDepSplit];
-    deposit_slice(b.args[w.x], w.y, it % kDepSplit, smem);
+    const int2 w = b.items[it];
+    deposit_slice<kDepThreads, false, kDepCells2>(b.args[w.x], w.y, smem);
     __syncthreads();
   }
 }
@@ -1021,15 +1319,65 @@ struct DiagBatchArgs {
   const int* nitems;
 };
 
+template <int NB, int T>
+__global__ void __launch_bounds__(T, 512 / T)
+    deposit_diag_batch_kernel(const __grid_constant__ DepBatchArgs b, const BeamDiagArgs* diag,
+                              const int parts) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int2 w = b.items[blockIdx.x / parts];
+  deposit_diag_part<NB, T>(b.args[w.x], diag[w.x], w.y, blockIdx.x % parts, parts, smem);
+}
+
 template <int NB>
 __global__ void __launch_bounds__(kDiagThreads, 2)
     beam_diag_batch_kernel(const __grid_constant__ DiagBatchArgs b) {
-  const int nitems = *b.nitems * kDepParts;  // (run, slice) items, kDepParts parts each
+  __shared__ DiagGroups<NB> G;
+  const int nitems = *b.nitems;
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const int2 w = b.items[it / kDepParts];
-    diag_slice<NB>(b.args[w.x], w.y, it % kDepParts);
+    const int2 w = b.items[it];
+    const BeamDiagArgs& a = b.args[w.x];
+    diag_groups<NB>(a, w.y, threadIdx.x >> 5, kDiagThreads / 32, G);
+    __syncthreads();
+    diag_record<NB, kDiagThreads>(a, w.y, G);
     __syncthreads();
   }
+}
+
+// How a launch over `nslice` slices is split.  parts > 0: that many CTAs per
+// slice, one of them for the diagnostics, of T threads: one CTA of 512 per SM
+// or two of 256; parts > 2: the deposition shared out over a tile in L2.  Else
+// one CTA per slice for the deposition and the diagnostics in a kernel of their
+// own: beside it, or in a branch of the graph where the slices fill the GPU
+// twice.  Measured, us per graph step of 8192 particles per slice (before: two
+// CTAs per slice below 296 slices, 256 threads of four particles above):
+//   slices  1 (151^2) 23.2 (28.3), 8 (201^2) 29.0, 16 33.0, 24 37.0 (two parts:
+//   26.3, 31.8, 34.4, 37.0: the adds to L2 cost more per particle than those to
+//   shared memory, so seven parts is where sharing stops to pay);
+//   50 48.6 (50.2), 64 55.3 (58.7), 100 82.2 (83.4), 147 104.5 (106.9);
+//   200 138 (143), 290 180 (191); 1024: the deposition 97 us (121).
+// A deposition waits on its loads, conversions and shared-memory atomics in
+// turn, so what pays is warps per SM: 32 with a particle per lane (64
+// registers) where two CTAs share an SM; four particles per thread at 128
+// registers where there is one.
+constexpr int kSplitMaxParts = 17;
+struct DepSplit {
+  int parts, T;
+  size_t smem() const { return dep_smem(T == 512 ? kDepCells1 : kDepCells2); }
+};
+static DepSplit dep_split(int nslice, int sm_count) {
+  if (nslice >= sm_count) return {0, 0};
+  const int parts = std::min(kSplitMaxParts, sm_count / nslice);
+  return parts >= 7 ? DepSplit{parts, 512} : DepSplit{2, 2 * nslice <= sm_count ? 512 : 256};
+}
+
+// fn(integral constant NB, integral constant T) of a split launch
+template <typename Fn>
+static void dep_dispatch(bool one, int T, Fn fn) {
+  using std::integral_constant;
+  if (one && T == 512) fn(integral_constant<int, 1>(), integral_constant<int, 512>());
+  else if (one) fn(integral_constant<int, 1>(), integral_constant<int, 256>());
+  else if (T == 512) fn(integral_constant<int, kMaxBunch>(), integral_constant<int, 512>());
+  else fn(integral_constant<int, kMaxBunch>(), integral_constant<int, 256>());
 }
 
 // ---------------------------------------------------------- diag finalize --
@@ -1040,21 +1388,17 @@ struct FinalizeArgs {
   int4* bbox[kRunFields];
   int nband[kRunFields];
   int first_after[kRunFields];
-  int nfield, nslice, rec;
-  const double* beam_part;  // [nslice * kDepParts][rec]
-  double* beam_hist;        // [nslice][rec] for this step
+  int nfield, nslice;
   double* field_hist;       // [nfield][nslice][9] for this step
 };
 
 // Per-slice reductions in fixed order: field diagnostics per beam slice
 // is = (nslice + storage - first) % nslice (src/Core/DiagnosticCUDA.cpp:320)
 // from the pass-Y band partials (one thread per slice and quantity, adding
-// the bands in order), the beam diagnostics from the deposition CTAs'
-// records; also resets the deposition boxes for the next step.
+// the bands in order); also resets the deposition boxes for the next step.
 __device__ __forceinline__ void finalize_range(const FinalizeArgs& a, int i0, int stride) {
   const int nf = a.nfield * a.nslice;
-  const int nb = a.nslice * a.rec;
-  for (int i = i0; i < 9 * nf + nb + nf; i += stride) {
+  for (int i = i0; i < 9 * nf + nf; i += stride) {
     if (i < 9 * nf) {
       const int j = i / 9, q = i - 9 * j;
       const int f = j / a.nslice, s = j - f * a.nslice;
@@ -1073,19 +1417,8 @@ __device__ __forceinline__ void finalize_range(const FinalizeArgs& a, int i0, in
       v += vc;
       const int is = (a.nslice + s - a.first_after[f]) % a.nslice;
       a.field_hist[((size_t)f * a.nslice + is) * 9 + q] = v;
-    } else if (i < 9 * nf + nb) {
-      const int j = i - 9 * nf;
-      const int s = j / a.rec, k = j - s * a.rec;
-      const int op = k < 13 ? 0 : (k < kBeamRec ? ((k - 13) % 2 == 0 ? 1 : 2) : 0);
-      const double* p = a.beam_part + (size_t)s * kDepParts * a.rec + k;
-      double t = p[0];
-      for (int b = 1; b < kDepParts; ++b) {
-        const double u = p[(size_t)b * a.rec];
-        t = op == 0 ? t + u : (op == 1 ? fmin(t, u) : fmax(t, u));
-      }
-      a.beam_hist[(size_t)s * a.rec + k] = t;
     } else {
-      const int j = i - 9 * nf - nb;
+      const int j = i - 9 * nf;
       const int f = j / a.nslice, s = j - f * a.nslice;
       a.bbox[f][s] = make_int4(1 << 30, 1 << 30, -1, -1);
     }
@@ -1155,6 +1488,9 @@ struct RunFieldState {
   int harm = 1;
   int4* d_bbox = nullptr;
   int* d_mpred = nullptr;       // [nslice] deposition contribution bound per slice
+  float* d_qpred = nullptr;     // [nslice] largest charge weight of the last deposition
+  unsigned char* d_tiles = nullptr;  // [nslice] DepTile of tile_cells (runs of few slices)
+  int tile_cells = 0;
   double* d_part = nullptr;
   int nband = 0;
   double accuslip = 0.0;        // host slippage model
@@ -1181,8 +1517,6 @@ struct g4b_run {
   std::vector<double> slip;
   // history of diagnostics: per step beam [nslice][rec] then fields
   double* d_hist = nullptr;
-  double* d_beam_part = nullptr;   // beam-diagnostic records per slice
-  float* d_qpred = nullptr;        // [nslice] largest charge weight of the last deposition
   // second stream and fork / join events of a captured step (diagnostics branch)
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -1202,7 +1536,6 @@ void g4b_chicane_matrix(double angle, double lb, double ld, double lt, double* m
 namespace {
 
 constexpr int kRunChunk = 2 * kStepThreads;  // particles per beam-step CTA
-constexpr int kRunMaxNp = 65536;              // particles per slice (deposition scale)
 
 // Every argument of one lattice step of one run.
 struct StepArgs {
@@ -1212,7 +1545,6 @@ struct StepArgs {
   BeamDiagArgs bd;
   AdiPlan adi[kRunFields];
   FinalizeArgs fa;
-  int nfin;
 };
 
 int plan_step(g4b_run* r, int i, StepPlan& p) {
@@ -1362,7 +1694,7 @@ int build_step(g4b_run* r, int i, const StepPlan& p, StepArgs& L) {
     b.nbunch = r->desc.nbunch;
     b.need_aux = 1;
     b.gref = gbase;
-    b.beam_part = r->d_beam_part;
+    b.beam_hist = step_hist;
     L.bd = b;
     DepArgs a{};
     a.xy = r->xy;
@@ -1370,7 +1702,6 @@ int build_step(g4b_run* r, int i, const StepPlan& p, StepArgs& L) {
     a.th = r->th;
     a.off = r->d_off;
     a.current = r->d_current;
-    a.qpred = r->d_qpred;
     a.nfield = r->nfield;
     a.ax = (float)st.ax;
     a.ay = (float)st.ay;
@@ -1388,6 +1719,8 @@ int build_step(g4b_run* r, int i, const StepPlan& p, StepArgs& L) {
       d.desc = F.f->desc;
       d.bbox = F.d_bbox;
       d.mpred = F.d_mpred;
+      d.qpred = F.d_qpred;
+      d.tiles = F.d_tiles;
       d.cap = (size_t)F.f->ngrid * F.f->ld;
       d.first = p.first_before[f];
       d.n = F.f->ngrid;
@@ -1398,9 +1731,10 @@ int build_step(g4b_run* r, int i, const StepPlan& p, StepArgs& L) {
       d.gridmax = (float)F.f->gridmax;
       d.dgrid = (float)F.f->dgrid;
       d.inv_dgrid = (float)(1.0 / F.f->dgrid);
-      d.dgrid_d = F.f->dgrid;
-      d.fc = p.fc[f];
-      d.xks = F.f->xks;
+      // adi_compute_slice_scl (src/Core/FieldSolverADICUDA.cpp:75-96)
+      d.kscl = p.fc[f] * 376.73031346177 * F.f->xks * st.delz /
+               (4.0 * 510998.95 * F.f->dgrid * F.f->dgrid);
+      d.tile_cells = F.tile_cells;
     }
     L.dd = a;
   }
@@ -1421,16 +1755,12 @@ int build_step(g4b_run* r, int i, const StepPlan& p, StepArgs& L) {
     a.nfield = r->nfield;
     a.nslice = r->nslice;
     a.field_hist = step_hist + r->rec_beam * r->nslice;
-    a.beam_hist = step_hist;
-    a.beam_part = r->d_beam_part;
-    a.rec = (int)r->rec_beam;
     for (int f = 0; f < r->nfield; ++f) {
       a.part[f] = r->fs[f].d_part;
       a.bbox[f] = r->fs[f].d_bbox;
       a.nband[f] = r->fs[f].nband;
       a.first_after[f] = p.first_after[f];
     }
-    L.nfin = 10 * r->nfield * r->nslice + r->nslice * (int)r->rec_beam;
     L.fa = a;
   }
   return G4B_OK;
@@ -1448,58 +1778,54 @@ int launch_single(g4b_run* r, const StepArgs& L) {
     G4B_CUDA_TRY(launch_pdl(kern, (unsigned)r->nchunk, kStepThreads, 0, c->stream, L.bs));
   }
   if (int rc = check_launch(c, "beam_step_kernel")) return rc;
-  // The beam diagnostics depend only on K1.  A run with slices enough to
-  // fill the GPU twice launches them as a kernel of their own: in a captured
-  // graph a branch beside the deposition and the ADI passes (on SMs those
-  // leave idle), joined before the finalize.  A smaller run computes them in
-  // the deposition's CTAs: the slice's last deposition part, before its band.
-  auto diag = [&](cudaStream_t st) {
-    LaunchScope ls(c, "run_beam_diag");
-    if (r->desc.nbunch == 1)
-      beam_diag_kernel<1><<<r->nslice * kDepParts, kDiagThreads, 0, st>>>(L.bd);
-    else
-      beam_diag_kernel<kMaxBunch><<<r->nslice * kDepParts, kDiagThreads, 0, st>>>(L.bd);
-    return check_launch(c, "beam_diag_kernel");
-  };
-  const bool own = r->nslice >= 2 * c->sm_count;
-  const bool branch = own && r->capturing;
+  // The beam diagnostics depend only on K1: see dep_split.  The branch (beside
+  // the deposition and the ADI passes, on SMs those leave idle, joined before
+  // the finalize) is for large runs: a fork per step takes a graph long to
+  // instantiate.
+  const DepSplit sp = dep_split(r->nslice, c->sm_count);
+  const bool one = r->desc.nbunch == 1;
+  const bool branch = r->nslice >= 2 * c->sm_count && r->capturing;
   if (branch) {
     G4B_CUDA_TRY(cudaEventRecord(r->ev_fork, c->stream));
     G4B_CUDA_TRY(cudaStreamWaitEvent(r->aux, r->ev_fork, 0));
-    if (int rc = diag(r->aux)) return rc;
+    {
+      LaunchScope ls(c, "run_beam_diag");
+      (one ? beam_diag_kernel<1, false> : beam_diag_kernel<kMaxBunch, false>)<<<
+          r->nslice, kDiagThreads, 0, r->aux>>>(L.bd);
+    }
+    if (int rc = check_launch(c, "beam_diag_kernel")) return rc;
     G4B_CUDA_TRY(cudaEventRecord(r->ev_join, r->aux));
   }
-  if (own) {
-    {
-      LaunchScope ls(c, "run_deposit");
-      G4B_CUDA_TRY(launch_pdl(deposit_kernel, (unsigned)(r->nslice * kDepSplit), kDepThreads,
-                              kDepSmem, c->stream, L.dd));
-    }
-    if (int rc = check_launch(c, "deposit_kernel")) return rc;
-    if (!branch)
-      if (int rc = diag(c->stream)) return rc;
-  } else {
+  if (sp.parts > 0) {
     LaunchScope ls(c, "run_deposit_diag");
-    const DepDiagLaunch dl{L.dd, L.bd};
-    const unsigned grid = (unsigned)(r->nslice * kDepSplit);
-    const bool wide = r->nslice * kDepSplit < c->sm_count;
-    const bool one = r->desc.nbunch == 1;
-    if (wide)
-      G4B_CUDA_TRY(launch_pdl(one ? deposit_diag_kernel<1, kDepWideThreads>
-                                  : deposit_diag_kernel<kMaxBunch, kDepWideThreads>,
-                              grid, kDepWideThreads, kDepSmem, c->stream, dl));
-    else
-      G4B_CUDA_TRY(launch_pdl(one ? deposit_diag_kernel<1, kDepThreads>
-                                  : deposit_diag_kernel<kMaxBunch, kDepThreads>,
-                              grid, kDepThreads, kDepSmem, c->stream, dl));
-    if (int rc = check_launch(c, "deposit_diag_kernel")) return rc;
+    const DepDiagLaunch dl{L.dd, L.bd, sp.parts};
+    cudaError_t e = cudaSuccess;
+    dep_dispatch(one, sp.T, [&](auto nb, auto t) {
+      e = launch_pdl(deposit_diag_kernel<decltype(nb)::value, decltype(t)::value>,
+                     (unsigned)(r->nslice * sp.parts), (unsigned)sp.T, sp.smem(), c->stream, dl);
+    });
+    G4B_CUDA_TRY(e);
+  } else {
+    LaunchScope ls(c, "run_deposit");
+    G4B_CUDA_TRY(launch_pdl(branch ? deposit_kernel<false> : deposit_kernel<true>,
+                            (unsigned)r->nslice, kDepThreads, dep_smem(kDepCells2), c->stream, L.dd));
+  }
+  if (int rc = check_launch(c, "deposit_kernel")) return rc;
+  if (sp.parts == 0 && !branch) {
+    {
+      LaunchScope ls(c, "run_beam_diag");
+      G4B_CUDA_TRY(launch_pdl(one ? beam_diag_kernel<1, true> : beam_diag_kernel<kMaxBunch, true>,
+                              (unsigned)r->nslice, kDiagThreads, 0, c->stream, L.bd));
+    }
+    if (int rc = check_launch(c, "beam_diag_kernel")) return rc;
   }
   for (int f = 0; f < r->nfield; ++f)
     if (int rc = adi_launch(r->fs[f].f, L.adi[f])) return rc;
   if (branch) G4B_CUDA_TRY(cudaStreamWaitEvent(c->stream, r->ev_join, 0));
   {
     LaunchScope ls(c, "run_diag_finalize");
-    G4B_CUDA_TRY(launch_pdl(diag_finalize_kernel, (unsigned)((L.nfin + 255) / 256), 256, 0,
+    G4B_CUDA_TRY(launch_pdl(diag_finalize_kernel,
+                            (unsigned)((10 * r->nfield * r->nslice + 255) / 256), 256, 0,
                             c->stream, L.fa));
   }
   return check_launch(c, "diag_finalize_kernel");
@@ -1612,7 +1938,12 @@ int g4b_run_create(g4b_ctx* c, const g4b_run_desc* d, const int64_t* off, g4b_ru
     r->bytes += F.f->bytes;
     F.nband = (F.f->ngrid + F.f->band_rows - 1) / F.f->band_rows;
     A((void**)&F.d_bbox, d->nslice * sizeof(int4));
-    A((void**)&F.d_mpred, d->nslice * kDepSplit * sizeof(int));
+    A((void**)&F.d_mpred, d->nslice * sizeof(int));
+    A((void**)&F.d_qpred, d->nslice * sizeof(float));
+    F.tile_cells = std::min((F.f->ngrid * F.f->ld + 3) / 4 * 4, kDepTileCells);
+    const size_t tiles =
+        dep_split(d->nslice, c->sm_count).parts > 2 ? d->nslice * dep_tile_bytes(F.tile_cells) : 0;
+    if (tiles) A((void**)&F.d_tiles, tiles);
     A((void**)&F.d_part, (size_t)d->nslice * F.nband * 9 * 8);
     if (e != cudaSuccess) {
       g4b_run_destroy(r);
@@ -1622,7 +1953,10 @@ int g4b_run_create(g4b_ctx* c, const g4b_run_desc* d, const int64_t* off, g4b_ru
     e = cudaMemcpyAsync(F.d_bbox, init.data(), init.size() * sizeof(int4),
                         cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess)
-      e = cudaMemsetAsync(F.d_mpred, 0, d->nslice * kDepSplit * sizeof(int), c->stream);
+      e = cudaMemsetAsync(F.d_mpred, 0, d->nslice * sizeof(int), c->stream);
+    if (e == cudaSuccess)
+      e = cudaMemsetAsync(F.d_qpred, 0, d->nslice * sizeof(float), c->stream);
+    if (e == cudaSuccess && tiles) e = cudaMemsetAsync(F.d_tiles, 0, tiles, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
       g4b_run_destroy(r);
@@ -1630,26 +1964,22 @@ int g4b_run_create(g4b_ctx* c, const g4b_run_desc* d, const int64_t* off, g4b_ru
     }
   }
   r->rec_beam = kBeamRec + 2 * d->nbunch;
-  A((void**)&r->d_beam_part, (size_t)d->nslice * kDepParts * r->rec_beam * 8);
-  A((void**)&r->d_qpred, d->nslice * kDepSplit * sizeof(float));
-  if (e == cudaSuccess)
-    e = cudaMemsetAsync(r->d_qpred, 0, d->nslice * kDepSplit * sizeof(float), c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     g4b_run_destroy(r);
     return cuda_fail(e, "g4b_run_create: device allocation");
   }
   r->step_doubles = (size_t)d->nslice * (r->rec_beam + 9 * d->nfield);
-  cudaFuncSetAttribute(deposit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)kDepSmem);
-  cudaFuncSetAttribute(deposit_diag_kernel<1, kDepThreads>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDepSmem);
-  cudaFuncSetAttribute(deposit_diag_kernel<kMaxBunch, kDepThreads>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDepSmem);
-  cudaFuncSetAttribute(deposit_diag_kernel<1, kDepWideThreads>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDepSmem);
-  cudaFuncSetAttribute(deposit_diag_kernel<kMaxBunch, kDepWideThreads>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDepSmem);
+  for (int k = 0; k < 4; ++k)
+    dep_dispatch(k & 1, k & 2 ? 512 : 256, [&](auto nb, auto t) {
+      cudaFuncSetAttribute(deposit_diag_kernel<decltype(nb)::value, decltype(t)::value>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)DepSplit{2, decltype(t)::value}.smem());
+    });
+  cudaFuncSetAttribute(deposit_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)dep_smem(kDepCells2));
+  cudaFuncSetAttribute(deposit_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)dep_smem(kDepCells2));
   *out = r;
   return G4B_OK;
 }
@@ -1662,7 +1992,7 @@ int g4b_run_destroy(g4b_run* r) {
   if (r->ev_join) cudaEventDestroy(r->ev_join);
   if (r->aux) cudaStreamDestroy(r->aux);
   void* ptrs[] = {r->xy, r->pxy, r->dg, r->th, r->d_off, r->d_chunks, r->d_current,
-                  r->d_eloss, r->d_hist, r->d_beam_part, r->d_qpred};
+                  r->d_eloss, r->d_hist};
   for (void* p : ptrs) dev_free(r->ctx, p);
   for (int f = 0; f < kRunFields; ++f) {
     RunFieldState& F = r->fs[f];
@@ -1670,6 +2000,8 @@ int g4b_run_destroy(g4b_run* r) {
     if (F.f) g4b_field_destroy(F.f);
     dev_free(r->ctx, F.d_bbox);
     dev_free(r->ctx, F.d_mpred);
+    dev_free(r->ctx, F.d_qpred);
+    dev_free(r->ctx, F.d_tiles);
     dev_free(r->ctx, F.d_part);
   }
   ctx_release(r->ctx);
@@ -1706,10 +2038,11 @@ int g4b_run_upload_beam(g4b_run* r, const double* x, const double* y, const doub
   }
   dev_free(r->ctx, stage);
   // a new beam: the next deposition counts before it accumulates
-  for (int f = 0; f < r->nfield && e == cudaSuccess; ++f)
-    e = cudaMemsetAsync(r->fs[f].d_mpred, 0, r->nslice * kDepSplit * sizeof(int), s);
-  if (e == cudaSuccess)
-    e = cudaMemsetAsync(r->d_qpred, 0, r->nslice * kDepSplit * sizeof(float), s);
+  for (int f = 0; f < r->nfield && e == cudaSuccess; ++f) {
+    e = cudaMemsetAsync(r->fs[f].d_mpred, 0, r->nslice * sizeof(int), s);
+    if (e == cudaSuccess)
+      e = cudaMemsetAsync(r->fs[f].d_qpred, 0, r->nslice * sizeof(float), s);
+  }
   const cudaError_t es = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "g4b_run_upload_beam");
   if (es != cudaSuccess) return cuda_fail(es, "g4b_run_upload_beam");
@@ -2255,26 +2588,37 @@ int batch_launch(g4b_batch* b, bool timed) {
   }
   if (int rc = check_launch(c, "beam_batch_kernel")) return rc;
   ev(1);
+  // few slices in all: several CTAs per slice, the diagnostics beside them
+  const DepSplit sp = dep_split(b->counts.dep, c->sm_count);
   {
     DepBatchArgs a{reinterpret_cast<const DepArgs*>(b->d_args + b->off_dd),
                    reinterpret_cast<const int2*>(b->d_items + b->off_dep), counts + 1};
     LaunchScope ls(c, "batch_deposit");
-    deposit_batch_kernel<<<b->grid[1], kDepThreads, kDepSmem, c->stream>>>(a);
+    if (sp.parts > 0)
+      dep_dispatch(b->nb_kind == 1, sp.T, [&](auto nb, auto t) {
+        deposit_diag_batch_kernel<decltype(nb)::value, decltype(t)::value>
+            <<<b->counts.dep * sp.parts, sp.T, sp.smem(), c->stream>>>(
+                a, reinterpret_cast<const BeamDiagArgs*>(b->d_args + b->off_bd), sp.parts);
+      });
+    else
+      deposit_batch_kernel<<<b->grid[1], kDepThreads, dep_smem(kDepCells2), c->stream>>>(a);
   }
   if (int rc = check_launch(c, "deposit_batch_kernel")) return rc;
   // branches (not while the tuner or the profiler times single kernels)
   const bool fork = !timed && !c->prof.on;
+  const DiagBatchArgs da{reinterpret_cast<const BeamDiagArgs*>(b->d_args + b->off_bd),
+                         reinterpret_cast<const int2*>(b->d_items + b->off_dep), counts + 1};
   auto diag = [&](cudaStream_t st) {
-    DiagBatchArgs a{reinterpret_cast<const BeamDiagArgs*>(b->d_args + b->off_bd),
-                    reinterpret_cast<const int2*>(b->d_items + b->off_dep), counts + 1};
     LaunchScope ls(c, "batch_beam_diag");
     if (b->nb_kind == 1)
-      beam_diag_batch_kernel<1><<<2 * c->sm_count, kDiagThreads, 0, st>>>(a);
+      beam_diag_batch_kernel<1><<<2 * c->sm_count, kDiagThreads, 0, st>>>(da);
     else
-      beam_diag_batch_kernel<kMaxBunch><<<2 * c->sm_count, kDiagThreads, 0, st>>>(a);
+      beam_diag_batch_kernel<kMaxBunch><<<2 * c->sm_count, kDiagThreads, 0, st>>>(da);
     return check_launch(c, "beam_diag_batch_kernel");
   };
-  if (fork) {
+  if (sp.parts > 0) {
+    // computed beside the deposition
+  } else if (fork) {
     G4B_CUDA_TRY(cudaEventRecord(b->ev_fork[0], c->stream));
     G4B_CUDA_TRY(cudaStreamWaitEvent(b->aux[0], b->ev_fork[0], 0));
     if (int rc = diag(b->aux[0])) return rc;
@@ -2315,7 +2659,7 @@ int batch_launch(g4b_batch* b, bool timed) {
         if (k % g4b_batch::kAux != 0) G4B_CUDA_TRY(cudaStreamWaitEvent(c->stream, b->ev_adi[k], 0));
     ev(3 + pass);
   }
-  if (fork) G4B_CUDA_TRY(cudaStreamWaitEvent(c->stream, b->ev_diag, 0));
+  if (fork && sp.parts == 0) G4B_CUDA_TRY(cudaStreamWaitEvent(c->stream, b->ev_diag, 0));
   {
     LaunchScope ls(c, "batch_diag_finalize");
     finalize_batch_kernel<<<b->grid[3], 256, 0, c->stream>>>(
@@ -2350,7 +2694,13 @@ int g4b_batch_create(g4b_ctx* c, int max_runs, g4b_batch** out) {
   b->last.assign(max_runs, 0);
   batch_default_grids(b);
   cudaFuncSetAttribute(deposit_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)kDepSmem);
+                       (int)dep_smem(kDepCells2));
+  for (int k = 0; k < 4; ++k)
+    dep_dispatch(k & 1, k & 2 ? 512 : 256, [&](auto nb, auto t) {
+      cudaFuncSetAttribute(deposit_diag_batch_kernel<decltype(nb)::value, decltype(t)::value>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)DepSplit{2, decltype(t)::value}.smem());
+    });
   if (int rc = batch_layout(b)) {
     g4b_batch_destroy(b);
     return rc;

@@ -198,3 +198,49 @@ def test_both_row_layouts_solve_the_same_system(ctx):
         b.set_layouts([9])
     a.close()
     b.close()
+
+
+# the deposition and the beam diagnostics of a slice are split by the number of
+# slices in the launch (dep_split: shared tile up to 21 slices, two CTAs of 512
+# or 256 threads per slice up to 147, one CTA above); widths 1 and 6 make tiles
+# of one band and of several, the slices start at odd offsets
+@pytest.mark.parametrize("width", [1.0, 6.0])
+@pytest.mark.parametrize("fill", [18, 19, 71, 72, 144, 145])
+def test_results_do_not_depend_on_how_the_slices_are_split(ctx, width, fill):
+    ns, ngrid, gm, n = 3, 151, 160e-6, 5
+    off, parts = synth.beam(ns, 1500, seed=11, ragged=True)
+    for k in ("x", "y"):
+        parts[k] = np.clip(parts[k] * width, -0.99 * gm, 0.99 * gm)
+    cells = synth.field(ns, ngrid, gm, seed=12, amplitude=2e12)
+    steps = [synth.und_step() for _ in range(n)]
+    fc = [[synth.coupling()]] * n
+    slip = [0.4] * n
+
+    def make(offsets, p, c, grid):
+        run = dev.Run(ctx, offsets, fields=[(1, grid, gm)], lambda0=synth.LAMBDA0,
+                      gamma_ref=synth.GAMMA0, time_run=True)
+        run.upload_beam(p)
+        run.upload_field(0, c, 0)
+        run.set_current(synth.CURRENT)
+        run.set_lattice(steps, fc, slip)
+        return run
+
+    alone = make(off, parts, cells, ngrid)
+    alone.advance(0, n, graph=True)
+    want = _result(alone, n)
+    foff, fparts = synth.beam(fill, 64, seed=13)
+    filler = make(foff, fparts, None, 33)
+    run = make(off, parts, cells, ngrid)
+    batch = dev.Batch(ctx, 2)
+    batch.attach(run, 0, n)
+    batch.attach(filler, 0, n)
+    batch.step(n)
+    got = _result(run, n)
+    assert np.any(want[1] != cells)
+    for k in want[0]:
+        assert np.array_equal(got[0][k], want[0][k])
+    assert np.array_equal(got[1], want[1]) and got[2] == want[2]
+    for a, b in zip(got[3], want[3]):
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    for o in (batch, run, filler, alone):
+        o.close()
