@@ -13,20 +13,35 @@
 //            solves (1 - i r d2y) u'' = R' and writes u'' transposed back into
 //            the natural layout.
 //
-// The tridiagonal solve is the reference's Thomas algorithm
-// (src/Core/FieldSolverADICUDA.cpp:222-277) written as two first-order linear
-// recurrences, y_k = cbet_k R_k + q_k y_{k-1} and u_k = y_k + s_k u_{k+1}
-// with q_k = s_k = i r cbet_k, evaluated by a warp: every lane runs the
-// recurrence over its own M consecutive elements, the lane carries are
-// combined by a 5-step Kogge-Stone scan of affine maps, and each lane adds
-// its carry times a precomputed product of coefficients.  All coefficients
-// (cbet, prefix/suffix products, scan multipliers) depend only on ngrid and r
-// and are computed once on the host in FP64 (FieldSolverADICUDA::init,
-// :821-902).
+// The tridiagonal system (1 - i r d2) u = R has constant coefficients, 1 + 2 i r
+// on the diagonal and - i r beside it, and zero walls at k = -1 and k = n.
+// With beta = (1 + 2 i r + sqrt(1 + 4 i r)) / 2 and q = i r / beta (|q| < 1) the
+// matrix of the unbounded line factors into the two recurrences
+//   y_k = (R_k + i r y_{k-1}) / beta,   u_k = y_k + q u_{k+1},
+// the constant limit of the pivots of the reference's Thomas algorithm
+// (src/Core/FieldSolverADICUDA.cpp:222-277).  Started with y_{-1} = 0 and
+// u_n = 0 they satisfy every row but the wall at k = -1, which the homogeneous
+// solution that vanishes at n mends:
+//   u_k - u_0 (q^{k+2} - q^{2n+2-k}) / (1 - q^{2n+2}).
+// A warp evaluates them: every lane runs the recurrences over its own M
+// consecutive elements, the lane carries are combined by a Kogge-Stone scan of
+// affine maps with multipliers q^(M 2^t) (only the steps whose multiplier
+// matters at this precision: |q| is 0.02 at the configurations' r, so one step
+// in place of five), and each lane adds its carry times a power of q.  All
+// coefficients but the lanes' wall terms are the same in every lane: the
+// single-run kernels read them from the constant bank.  With the Thomas pivots
+// and the products of their factors in per-lane tables the passes spent as much
+// of the load path on coefficients (four loads per element) as on the field:
+// per pass X / Y of 1024 slices of 201^2 in FP32 152 / 136 -> 138 / 124 us (4.8
+// and 5.3 TB/s of the field read and written), of 256 slices in FP64 96 / 83 ->
+// 80 / 66 us, of 40 slices of 401^2 98 / 77 -> 86 / 65 us.
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <cstring>
 #include <new>
+#include <utility>
+#include <vector>
 
 #include <atomic>
 
@@ -78,17 +93,6 @@ __device__ __forceinline__ C shfl_down_c(C v, int d) {
 // ------------------------------------------------------ row arithmetic ---
 // Forced inline into the single-run and the batched pass kernels: the same
 // operations in the same order, hence the same bits, in every kernel.
-// Tables of a row layout (L lanes of M elements), lane-minor:
-//   cbet [M][L], G prefix products [M][L], H suffix products [M][L],
-//   forward scan multipliers [5][L], backward scan multipliers [5][L],
-//   S: s_k = i r cbet_k (0 at the last row) [M][L].
-template <int M, int L, typename C> struct RowTabs {
-  const C *cb, *G, *H, *F, *B, *S;
-  __device__ __forceinline__ explicit RowTabs(const C* tab)
-      : cb(tab), G(tab + M * L), H(tab + 2 * M * L), F(tab + 3 * M * L),
-        B(tab + 3 * M * L + 5 * L), S(tab + 3 * M * L + 10 * L) {}
-};
-
 // Pass X right-hand side of the band row at tile slot row + 1 (neighbours at
 // slots row and row + 2): R = u + i r d2y(u) + S
 // (src/Core/FieldSolverADICUDA.cpp:197-220); elements j >= jn are zero.
@@ -113,65 +117,59 @@ __device__ __forceinline__ void px_rhs(C (&v)[M], const C* tile, int ld, int row
   }
 }
 
-// Local part of the forward recurrence y_k = cbet_k (R_k + i r y_{k-1}) over
-// lane gl's elements, with a zero carry in.
+// The tridiagonal solve (1 - i r d2) u = R of one row held by a group of L
+// lanes, M consecutive elements each (lane gl: elements gl*M .. gl*M+M-1, of
+// which the first jn lie in the row; R is zero in the others).  wall: the
+// lanes' q^(gl M) / (1 - q^(2n+2)), then their q^(2n+2-(gl+1)M) / (1 - q^(2n+2)).
 template <typename T, int M, int L, typename C>
-__device__ __forceinline__ void fwd_local(C (&v)[M], const RowTabs<M, L, C>& tb, int gl, T r) {
-  v[0] = cmul(__ldg(&tb.cb[gl]), v[0]);
+__device__ __forceinline__ void row_solve(C (&v)[M], const RowConst<C>& K, const C* wall, int gl,
+                                          int jn, T r) {
+  constexpr int kScan = L == 32 ? 5 : 4;  // log2 L
+  const C we = wall[gl], wd = wall[L + gl];
+  v[0] = cmul(K.cb, v[0]);
 #pragma unroll
   for (int j = 1; j < M; ++j) {
-    const C cb = __ldg(&tb.cb[j * L + gl]);
     C t;
     t.x = fma(-r, v[j - 1].y, v[j].x);
     t.y = fma(r, v[j - 1].x, v[j].y);
-    v[j] = cmul(cb, t);
+    v[j] = cmul(K.cb, t);
   }
-}
-
-// Local part of the backward recurrence u_k = y_k + s_k u_{k+1}.
-template <int M, int L, typename C>
-__device__ __forceinline__ void bwd_local(C (&v)[M], const RowTabs<M, L, C>& tb, int gl) {
-#pragma unroll
-  for (int j = M - 2; j >= 0; --j) v[j] = cfma(__ldg(&tb.S[j * L + gl]), v[j + 1], v[j]);
-}
-
-// v_j += P_j carry (P: the prefix or suffix products of lane gl).
-template <int M, int L, typename C>
-__device__ __forceinline__ void add_carry(C (&v)[M], const C* P, int gl, C carry) {
-#pragma unroll
-  for (int j = 0; j < M; ++j) v[j] = cfma(__ldg(&P[j * L + gl]), carry, v[j]);
-}
-
-// The tridiagonal solve (1 - i r d2) u = R of one row held by a group of L
-// lanes, M consecutive elements each (lane gl: elements gl*M .. gl*M+M-1):
-// local recurrences, the lane carries combined by a Kogge-Stone scan of
-// affine maps, each lane's carry times the products of its coefficients.
-template <typename T, int M, int L, typename C>
-__device__ __forceinline__ void row_solve(C (&v)[M], const C* tab, int gl, T r) {
-  constexpr int kScan = L == 32 ? 5 : 4;  // log2 L
-  const RowTabs<M, L, C> tb(tab);
-  fwd_local<T, M, L>(v, tb, gl, r);
   C b = v[M - 1];
 #pragma unroll
   for (int t = 0; t < kScan; ++t) {
-    const int d = 1 << t;
-    const C o = shfl_up_c<L>(b, d);
-    if (gl >= d) b = cfma(__ldg(&tb.F[t * L + gl]), o, b);
+    if (t >= K.nscan) break;
+    const C o = shfl_up_c<L>(b, 1 << t);
+    if (gl >= 1 << t) b = cfma(K.A[t], o, b);
   }
   C yin = shfl_up_c<L>(b, 1);
   if (gl == 0) yin = C{0, 0};
-  add_carry<M, L>(v, tb.G, gl, yin);
-  bwd_local<M, L>(v, tb, gl);
+#pragma unroll
+  for (int j = 0; j < M; ++j) v[j] = cfma(K.P[j + 1], yin, v[j]);
+  if (jn < M) {  // u is zero from n on
+#pragma unroll
+    for (int j = 0; j < M; ++j)
+      if (j >= jn) v[j] = C{0, 0};
+  }
+#pragma unroll
+  for (int j = M - 2; j >= 0; --j) v[j] = cfma(K.P[1], v[j + 1], v[j]);
   b = v[0];
 #pragma unroll
   for (int t = 0; t < kScan; ++t) {
-    const int d = 1 << t;
-    const C o = shfl_down_c<L>(b, d);
-    if (gl + d < L) b = cfma(__ldg(&tb.B[t * L + gl]), o, b);
+    if (t >= K.nscan) break;
+    const C o = shfl_down_c<L>(b, 1 << t);
+    if (gl + (1 << t) < L) b = cfma(K.A[t], o, b);
   }
   C uin = shfl_down_c<L>(b, 1);
   if (gl == L - 1) uin = C{0, 0};
-  add_carry<M, L>(v, tb.H, gl, uin);
+  // the wall at k = -1, from lane 0's first element
+  C u0 = cfma(K.P[M], uin, v[0]);
+  u0.x = -__shfl_sync(0xffffffffu, u0.x, 0, L);
+  u0.y = -__shfl_sync(0xffffffffu, u0.y, 0, L);
+  const C c = cmul(we, u0);
+  uin.x -= fma(wd.x, u0.x, -(wd.y * u0.y));
+  uin.y -= fma(wd.x, u0.y, wd.y * u0.x);
+#pragma unroll
+  for (int j = 0; j < M; ++j) v[j] = cfma(K.P[j + 2], c, cfma(K.P[M - j], uin, v[j]));
 }
 
 // R' = u' + i r d2x(u') + S (src/Core/FieldSolverADICUDA.cpp:279-323) of a
@@ -201,8 +199,7 @@ __device__ __forceinline__ void px_rprime(C (&v)[M], int gl, T r, unsigned long 
 
 // Warps per CTA and CTAs per SM (launch bounds) of the ADI kernels: FP64 9
 // warps of 32-lane rows, three CTAs per SM up to M = 7 (ngrid 224: pass X's
-// three tiles still fit the SM's shared memory; 416 -> 338 us per pass X of
-// 1024 x 201^2 against two); FP32 10 warps of 32-lane rows or 5 warps of two
+// three tiles still fit the SM's shared memory); FP32 10 warps of 32-lane rows or 5 warps of two
 // 16-lane rows each (10 rows per band either way; smaller CTAs of 16-lane
 // rows keep six on an SM so that one CTA's loads and stores overlap the
 // others' solves).
@@ -222,11 +219,10 @@ template <typename T, int M, int L> struct AdiBlocks {
 // phase this band waits on.  Returns false, with nothing solved or stored, if
 // the band's rows did not arrive within the bounded wait (the device error
 // flag then says so); the result is the same in every thread of the CTA.
-template <typename T, int M, bool PX, int L>
-__device__ __forceinline__ bool adi_band(const AdiPassArgs& a, const CUtensorMap* tm_out, int s,
-                                         int band, unsigned char* smem, uint64_t* bar,
-                                         uint32_t parity) {
-  using C = typename CT<T>::type;
+template <typename T, int M, bool PX, int L, typename C = typename CT<T>::type>
+__device__ __forceinline__ bool adi_band(const AdiPassArgs& a, const RowConst<C>& K,
+                                         const CUtensorMap* tm_out, int s, int band,
+                                         unsigned char* smem, uint64_t* bar, uint32_t parity) {
   constexpr int R = 32 / L;                     // rows per warp
   constexpr int W = BandW<T, L>::value * R;     // rows per band
   const int n = a.n, ld = a.ld;
@@ -304,7 +300,8 @@ __device__ __forceinline__ bool adi_band(const AdiPassArgs& a, const CUtensorMap
 #pragma unroll
       for (int j = 0; j < M; ++j) v[j] = j < jn ? tile[row * ld + gl * M + j] : C{0, 0};
     }
-    row_solve<T, M, L>(v, reinterpret_cast<const C*>(a.tab), gl, r);
+    row_solve<T, M, L>(v, K, reinterpret_cast<const C*>(static_cast<const RowConst<C>*>(a.tab) + 1),
+                       gl, jn, r);
     if (PX) px_rprime<T, M, L>(v, gl, r, smask, srow);
   } else {
 #pragma unroll
@@ -334,7 +331,11 @@ __device__ __forceinline__ bool adi_band(const AdiPassArgs& a, const CUtensorMap
     const int ic = (n * n - 1) / 2;
     const int icy = ic / n, icx = ic - icy * n;
     if (active) {
-      // cells past the row end hold exact zeros (their coefficients are 0)
+      if (jn < M) {  // cells past the row end
+#pragma unroll
+        for (int j = 0; j < M; ++j)
+          if (j >= jn) v[j] = C{0, 0};
+      }
       const T dy0 = (T)(gl * M) + shift;  // exact: small integers and halves
 #pragma unroll
       for (int j = 0; j < M; ++j) {
@@ -412,6 +413,7 @@ __device__ __forceinline__ bool adi_band(const AdiPassArgs& a, const CUtensorMap
 template <typename T, int M, bool PX, int L>
 __global__ void __launch_bounds__(BandW<T, L>::value * 32, AdiBlocks<T, M, L>::value)
     adi_pass_kernel(const __grid_constant__ AdiPassArgs a,
+                    const __grid_constant__ RowConst<typename CT<T>::type> K,
                     const __grid_constant__ CUtensorMap tm_out) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t bar;
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(BandW<T, L>::value * 32, AdiBlocks<T, M, L>::v
   }
   __syncthreads();
   ptx::pdl_wait();
-  adi_band<T, M, PX, L>(a, &tm_out, blockIdx.x / a.nband, blockIdx.x % a.nband, smem, &bar, 0u);
+  adi_band<T, M, PX, L>(a, K, &tm_out, blockIdx.x / a.nband, blockIdx.x % a.nband, smem, &bar, 0u);
 }
 
 // Persistent form over a work list of (run, slice, band) items of many runs
@@ -444,7 +446,10 @@ __global__ void __launch_bounds__(BandW<T, L>::value * 32, AdiBlocks<T, M, L>::v
     if (threadIdx.x == 0) ptx::fence_tensormap_acquire(tm);
     // a band whose rows never arrived leaves the barrier's phase open: stop
     // (the error flag reports it) rather than wait on it again
-    if (!adi_band<T, M, PX, L>(b.args[w.x], tm, w.y, w.z, smem, &bar, parity)) return;
+    const AdiPassArgs& a = b.args[w.x];
+    if (!adi_band<T, M, PX, L>(a, *static_cast<const RowConst<typename CT<T>::type>*>(a.tab), tm,
+                               w.y, w.z, smem, &bar, parity))
+      return;
     parity ^= 1u;
     __syncthreads();
   }
@@ -698,15 +703,16 @@ static int configure_pass_t(int device) {
 }
 
 template <typename T, int M, bool PX, int L>
-static int launch_pass_t(g4b_field* f, const AdiPassArgs& args, const CUtensorMap& tm,
-                         size_t smem) {
+static int launch_pass_t(g4b_field* f, const AdiPassArgs& args, const void* row,
+                         const CUtensorMap& tm, size_t smem) {
   constexpr int W = BandW<T, L>::value;  // warps per CTA
   auto kern = adi_pass_kernel<T, M, PX, L>;
   if (int rc = configure_pass_t<T, M, PX, L>(f->ctx->device)) return rc;
   const unsigned grid = (unsigned)(f->nslice * args.nband);
   {
     LaunchScope ls(f->ctx, PX ? "adi_pass_x" : "adi_pass_y");
-    G4B_CUDA_TRY(launch_pdl(kern, grid, W * 32, smem, f->ctx->stream, args, tm));
+    G4B_CUDA_TRY(launch_pdl(kern, grid, W * 32, smem, f->ctx->stream, args,
+                            *static_cast<const RowConst<typename CT<T>::type>*>(row), tm));
   }
   return check_launch(f->ctx, "adi_pass_kernel");
 }
@@ -743,10 +749,10 @@ int adi_configure(g4b_field* f) {
 }
 
 template <typename T, bool PX>
-static int launch_pass_m(int mode, g4b_field* f, const AdiPassArgs& args,
+static int launch_pass_m(int mode, g4b_field* f, const AdiPassArgs& args, const void* row,
                          const CUtensorMap& tm, size_t smem) {
 #define G4B_LAUNCH(m, l) \
-  case (l == 16 ? 100 : 0) + m: return launch_pass_t<T, m, PX, l>(f, args, tm, smem);
+  case (l == 16 ? 100 : 0) + m: return launch_pass_t<T, m, PX, l>(f, args, row, tm, smem);
   if constexpr (sizeof(T) == 8) {
     switch (mode) { G4B_MODES32(G4B_LAUNCH) }
   } else {
@@ -767,13 +773,16 @@ int adi_plan(g4b_adi* adi, g4b_field* f, const void* src, const int4* desc,
   args.err = f->ctx->d_error;
   args.box_rows = f->store_box_rows;
   args.nbox = f->store_nbox;
-  if (f->precision == G4B_FP64)
+  if (f->precision == G4B_FP64) {
     args.tab = adi->d_tab64;
-  else if (f->mode == adi->mode32)
+    P.row = &adi->k64;
+  } else if (f->mode == adi->mode32) {
     args.tab = adi->d_tab32;
-  else if (f->mode == adi->mode32_alt && adi->d_tab32_alt)
+    P.row = &adi->k32;
+  } else if (f->mode == adi->mode32_alt && adi->d_tab32_alt) {
     args.tab = adi->d_tab32_alt;
-  else
+    P.row = &adi->k32_alt;
+  } else
     return fail(G4B_ERR_STATE, "adi: solver and field row layouts differ");
   const size_t cb = f->cell_bytes;
   const size_t out_bytes = (size_t)f->store_nbox * f->store_box_rows * W * cb;
@@ -823,12 +832,12 @@ int adi_plan(g4b_adi* adi, g4b_field* f, const void* src, const int4* desc,
 
 int adi_launch(g4b_field* f, const AdiPlan& P) {
   int rc = P.precision == G4B_FP64
-               ? launch_pass_m<double, true>(P.M, f, P.x, *P.tm_x, P.smem_x)
-               : launch_pass_m<float, true>(P.M, f, P.x, *P.tm_x, P.smem_x);
+               ? launch_pass_m<double, true>(P.M, f, P.x, P.row, *P.tm_x, P.smem_x)
+               : launch_pass_m<float, true>(P.M, f, P.x, P.row, *P.tm_x, P.smem_x);
   if (rc) return rc;
   return P.precision == G4B_FP64
-             ? launch_pass_m<double, false>(P.M, f, P.y, *P.tm_y, P.smem_y)
-             : launch_pass_m<float, false>(P.M, f, P.y, *P.tm_y, P.smem_y);
+             ? launch_pass_m<double, false>(P.M, f, P.y, P.row, *P.tm_y, P.smem_y)
+             : launch_pass_m<float, false>(P.M, f, P.y, P.row, *P.tm_y, P.smem_y);
 }
 
 int adi_run(g4b_adi* adi, g4b_field* f, const void* src, const int4* desc,
@@ -924,8 +933,54 @@ int fp64_deposit(g4b_field* f, g4b_beam* b, const g4b_step* st, double fc) {
 
 using namespace g4b;
 
-extern "C" {
+namespace {
 
+using cld = std::complex<long double>;
+
+// Coefficients of rows of n elements held by L lanes of M, rounded to C, and
+// their device image: K, then the lanes' wall coefficients.
+template <typename C>
+void row_tables(double r, int n, int M, int L, RowConst<C>& K, std::vector<unsigned char>& image) {
+  using T = decltype(C{}.x);
+  const cld ir(0.0L, r), beta = (cld(1.0L, 2.0L * r) + std::sqrt(cld(1.0L, 4.0L * r))) / 2.0L;
+  const cld q = ir / beta;
+  auto power = [&](long long m) {  // q^m by squaring
+    cld p = 1.0L, s = q;
+    for (; m > 0; m >>= 1, s *= s)
+      if (m & 1) p *= s;
+    return p;
+  };
+  auto round = [](cld z) {
+    C c;
+    c.x = (T)z.real();
+    c.y = (T)z.imag();
+    return c;
+  };
+  K = RowConst<C>{};
+  for (int m = 0; m < kRowMaxM + 2; ++m) K.P[m] = round(power(m));
+  K.cb = round(1.0L / beta);
+  // a dropped scan step changes a carry by less than 2^-75 (FP32: 2^-45) of
+  // the largest, far below its rounding
+  const long double drop = sizeof(T) == 8 ? 0x1p-75L : 0x1p-45L;
+  for (int t = 0; (1 << t) < L; ++t) {
+    const cld A = power((long long)M << t);
+    K.A[t] = round(A);
+    if (std::abs(A) >= drop) K.nscan = t + 1;
+  }
+  std::vector<C> wall(2 * L, C{0, 0});
+  const cld den = 1.0L - power(2LL * n + 2);
+  for (int l = 0; l < L && l * M < n; ++l) {
+    wall[l] = round(power((long long)l * M) / den);
+    wall[L + l] = round(power(2LL * n + 2 - (long long)(l + 1) * M) / den);
+  }
+  image.resize(sizeof K + wall.size() * sizeof(C));
+  std::memcpy(image.data(), &K, sizeof K);
+  std::memcpy(image.data() + sizeof K, wall.data(), wall.size() * sizeof(C));
+}
+
+}  // namespace
+
+extern "C" {
 
 int g4b_adi_create(g4b_ctx* c, g4b_adi** out) {
   if (!c || !out) return fail(G4B_ERR_ARG, "g4b_adi_create: null arg");
@@ -949,8 +1004,8 @@ int g4b_adi_destroy(g4b_adi* a) {
 }
 
 // FieldSolverADICUDA::init (src/Core/FieldSolverADICUDA.cpp:821-866): the
-// Thomas factors of the constant matrix, then the scan tables derived from
-// them, all in FP64.
+// coefficients of the row solve, in long double, for every row layout a field
+// of this grid may take.
 int g4b_adi_init(g4b_adi* a, double delz, double dgrid, double xks, int ngrid) {
   if (!a) return fail(G4B_ERR_ARG, "g4b_adi_init: null adi");
   if (ngrid < 2 || !(dgrid > 0) || !(xks > 0))
@@ -960,116 +1015,33 @@ int g4b_adi_init(g4b_adi* a, double delz, double dgrid, double xks, int ngrid) {
     return G4B_OK;
   const int M = pick_M(ngrid);
   if (!M) return fail(G4B_ERR_RANGE, "g4b_adi_init: ngrid above 1056 is not supported");
-  using cd = std::complex<double>;
   const int n = ngrid;
   const double r = 0.25 * delz / (xks * dgrid * dgrid);
-  std::vector<double> mupp(n), mmid(n), mlow(n);
-  mupp[0] = r;
-  mmid[0] = -2 * r;
-  mlow[0] = 0;
-  for (int i = 1; i < n - 1; ++i) {
-    mupp[i] = r;
-    mmid[i] = -2 * r;
-    mlow[i] = r;
-  }
-  mupp[n - 1] = 0;
-  mmid[n - 1] = -2 * r;
-  mlow[n - 1] = r;
-  std::vector<cd> c(n), cbet(n), cwet(n);
-  for (int i = 0; i < n; ++i) c[i] = cd(0.0, -mlow[i]);
-  cbet[0] = cd(1.0, 0.0) / cd(1.0, -mmid[0]);
-  cwet[0] = cd(0.0, 0.0);
-  for (int i = 1; i < n; ++i) {
-    cwet[i] = cd(0.0, -mupp[i - 1]) * cbet[i - 1];
-    cbet[i] = cd(1.0, 0.0) / (cd(1.0, -mmid[i]) - c[i] * cwet[i]);
-  }
-  // Tables of one row layout: L lanes of M elements, recurrence
-  // coefficients on the padded index range [0, L M).
-  auto tables = [&](const int M, const int L) {
-    const int P = L * M;
-    std::vector<cd> cb(P, 0.0), q(P, 0.0), sv(P, 0.0), G(P), H(P);
-    for (int k = 0; k < n; ++k) cb[k] = cbet[k];
-    for (int k = 1; k < n; ++k) q[k] = -c[k] * cbet[k];         // y_k += q_k y_{k-1}
-    for (int k = 0; k + 1 < n; ++k) sv[k] = -cwet[k + 1];       // u_k += s_k u_{k+1}
-    std::vector<cd> A(L), B(L);
-    for (int lane = 0; lane < L; ++lane) {
-      const int k0 = lane * M, k1 = k0 + M - 1;
-      cd g = 1.0;
-      for (int k = k0; k <= k1; ++k) {
-        g *= q[k];
-        G[k] = g;
-      }
-      cd h = 1.0;
-      for (int k = k1; k >= k0; --k) {
-        h *= sv[k];
-        H[k] = h;
-      }
-      A[lane] = G[k1];
-      B[lane] = H[k0];
-    }
-    std::vector<cd> t(tab_total(M, L), 0.0);
-    for (int j = 0; j < M; ++j)
-      for (int lane = 0; lane < L; ++lane) {
-        const int k = lane * M + j;
-        t[tab_cbet(M, L) + j * L + lane] = cb[k];
-        t[tab_G(M, L) + j * L + lane] = G[k];
-        t[tab_H(M, L) + j * L + lane] = H[k];
-        t[tab_S(M, L) + j * L + lane] = sv[k];
-      }
-    std::vector<cd> af = A, ab = B;
-    for (int st = 0; (1 << st) < L; ++st) {
-      const int d = 1 << st;
-      for (int lane = 0; lane < L; ++lane) {
-        t[tab_scanF(M, L) + st * L + lane] = af[lane];
-        t[tab_scanB(M, L) + st * L + lane] = ab[lane];
-      }
-      std::vector<cd> nf = af, nb = ab;
-      for (int lane = 0; lane < L; ++lane) {
-        if (lane >= d) nf[lane] = af[lane] * af[lane - d];
-        if (lane + d < L) nb[lane] = ab[lane] * ab[lane + d];
-      }
-      af.swap(nf);
-      ab.swap(nb);
-    }
-    return t;
-  };
-  // FP64 fields solve rows with 32 lanes; FP32 fields with the layout of
-  // their mode (16-lane rows where those fit the row more closely)
-  // (and the tables of the other FP32 layout, which the batch tuner may pick)
-  const int mode32 = pick_mode(n, G4B_MIXED), mode32_alt = alt_mode(n);
-  const std::vector<cd> c64 = tables(M, 32);
-  auto to32 = [&](int mode) {
-    const std::vector<cd> c = tables(mode_M(mode), mode_L(mode));
-    std::vector<float2> t(c.size());
-    for (size_t k = 0; k < c.size(); ++k) t[k] = make_float2((float)c[k].real(), (float)c[k].imag());
-    return t;
-  };
-  std::vector<double2> t64(c64.size());
-  for (size_t k = 0; k < c64.size(); ++k) t64[k] = make_double2(c64[k].real(), c64[k].imag());
-  const std::vector<float2> t32 = to32(mode32);
-  const std::vector<float2> t32a = mode32_alt ? to32(mode32_alt) : std::vector<float2>();
   g4b_ctx* ctx = a->ctx;
   G4B_CUDA_TRY(cudaSetDevice(ctx->device));
   if (a->d_tab64) {
     cudaStreamSynchronize(ctx->stream);
-    dev_free(a->ctx, a->d_tab64);
-    dev_free(a->ctx, a->d_tab32);
-    dev_free(a->ctx, a->d_tab32_alt);
-    a->d_tab64 = nullptr;
-    a->d_tab32 = nullptr;
-    a->d_tab32_alt = nullptr;
+    for (void** d : {&a->d_tab64, &a->d_tab32, &a->d_tab32_alt}) {
+      dev_free(a->ctx, *d);
+      *d = nullptr;
+    }
+    a->ready = false;
   }
-  G4B_CUDA_TRY(dev_alloc(a->ctx, (void**)&a->d_tab64, t64.size() * sizeof(double2)));
-  G4B_CUDA_TRY(dev_alloc(a->ctx, (void**)&a->d_tab32, t32.size() * sizeof(float2)));
-  if (!t32a.empty())
-    G4B_CUDA_TRY(dev_alloc(a->ctx, (void**)&a->d_tab32_alt, t32a.size() * sizeof(float2)));
-  G4B_CUDA_TRY(cudaMemcpyAsync(a->d_tab64, t64.data(), t64.size() * sizeof(double2),
-                               cudaMemcpyHostToDevice, ctx->stream));
-  G4B_CUDA_TRY(cudaMemcpyAsync(a->d_tab32, t32.data(), t32.size() * sizeof(float2),
-                               cudaMemcpyHostToDevice, ctx->stream));
-  if (!t32a.empty())
-    G4B_CUDA_TRY(cudaMemcpyAsync(a->d_tab32_alt, t32a.data(), t32a.size() * sizeof(float2),
-                                 cudaMemcpyHostToDevice, ctx->stream));
+  // FP64 fields solve rows with 32 lanes; FP32 fields with the layout of
+  // their mode (16-lane rows where those fit the row more closely), or the
+  // other FP32 layout, which the batch tuner may pick
+  const int mode32 = pick_mode(n, G4B_MIXED), mode32_alt = alt_mode(n);
+  std::vector<unsigned char> t64, t32, t32a;
+  row_tables(r, n, M, 32, a->k64, t64);
+  row_tables(r, n, mode_M(mode32), mode_L(mode32), a->k32, t32);
+  if (mode32_alt) row_tables(r, n, mode_M(mode32_alt), mode_L(mode32_alt), a->k32_alt, t32a);
+  const std::pair<void**, std::vector<unsigned char>*> up[] = {
+      {&a->d_tab64, &t64}, {&a->d_tab32, &t32}, {&a->d_tab32_alt, &t32a}};
+  for (auto& [d, t] : up) {
+    if (t->empty()) continue;
+    G4B_CUDA_TRY(dev_alloc(ctx, d, t->size()));
+    G4B_CUDA_TRY(cudaMemcpyAsync(*d, t->data(), t->size(), cudaMemcpyHostToDevice, ctx->stream));
+  }
   G4B_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   a->ngrid = ngrid;
   a->delz = delz;

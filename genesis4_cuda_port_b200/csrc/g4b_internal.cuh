@@ -120,6 +120,20 @@ struct g4b_beam {
   uint64_t bytes = 0;
 };
 
+namespace g4b {
+// Coefficients of the tridiagonal row solve (g4b_adi.cu) with M elements per
+// lane: P[m] = q^m, A[t] = q^(M 2^t), 1 / beta, and the scan steps whose A[t]
+// matters at the precision of C.
+constexpr int kRowMaxM = 33;
+template <typename C>
+struct RowConst {
+  C P[kRowMaxM + 2];
+  C A[5];
+  C cb;
+  int nscan, pad;
+};
+}  // namespace g4b
+
 struct g4b_adi {
   g4b_ctx* ctx = nullptr;
   int ngrid = 0;
@@ -127,10 +141,11 @@ struct g4b_adi {
   int M = 0;                 // elements per lane (odd), 32-lane rows (FP64 fields)
   int mode32 = 0;            // row layout of FP32 fields (pick_mode)
   int mode32_alt = 0;        // the other FP32 row layout (alt_mode), 0 if none
-  // Tables in lane-minor order, complex (double2) and their FP32 copies.
-  double2* d_tab64 = nullptr;   // [3][M][32]: cbet, G, H ; then [2][5][32] scans
-  float2* d_tab32 = nullptr;
-  float2* d_tab32_alt = nullptr;  // tables of mode32_alt
+  // Coefficients of the row solve (RowConst), for the kernels' parameters, and
+  // on the device: RowConst, then the wall coefficients of the lanes [2][L].
+  g4b::RowConst<double2> k64;
+  g4b::RowConst<float2> k32, k32_alt;   // mode32, mode32_alt
+  void *d_tab64 = nullptr, *d_tab32 = nullptr, *d_tab32_alt = nullptr;
   bool ready = false;
 };
 
@@ -199,7 +214,7 @@ struct AdiPassArgs {
   const void* src;     // pass X only: compact per-slice source tiles; nullptr = none
   const int4* desc;    // per-slice source tile (x0, y0, width, height); width 0 = none
   size_t src_cap;      // cells reserved per slice in `src`
-  const void* tab;     // lane-minor tables of this precision
+  const void* tab;     // RowConst and wall coefficients of this precision and row layout
   int n, ld, nband;
   int out_off;         // byte offset of the output staging tile (pass X: 0, over the input)
   int box_rows, nbox;  // TMA store boxes per band
@@ -226,6 +241,7 @@ int adi_run(g4b_adi* adi, g4b_field* f, const void* src, const int4* desc,
 // The two passes of one field step, resolved but not launched.
 struct AdiPlan {
   AdiPassArgs x, y;
+  const void* row;          // RowConst of this precision and row layout (host)
   const CUtensorMap* tm_x;  // host copies of the field's store maps
   const CUtensorMap* tm_y;
   size_t smem_x, smem_y;
@@ -249,16 +265,6 @@ int adi_batch_launch(g4b_ctx* c, cudaStream_t st, int M, bool px, const AdiBatch
 // Sets the launch attributes of the ADI kernels for this field's grid (done
 // before any stream capture).
 int adi_configure(g4b_field* f);
-
-// Lane-minor table offsets (in complex elements) for rows of L lanes with M
-// elements each.
-inline size_t tab_cbet(int M, int L) { (void)M; (void)L; return 0; }
-inline size_t tab_G(int M, int L) { return (size_t)M * L; }
-inline size_t tab_H(int M, int L) { return (size_t)2 * M * L; }
-inline size_t tab_scanF(int M, int L) { return (size_t)3 * M * L; }
-inline size_t tab_scanB(int M, int L) { return (size_t)3 * M * L + 5 * L; }
-inline size_t tab_S(int M, int L) { return (size_t)3 * M * L + 10 * L; }
-inline size_t tab_total(int M, int L) { return (size_t)4 * M * L + 10 * L; }
 
 // Elements per lane for 32-lane rows (0 if n > 1056).
 int pick_M(int n);

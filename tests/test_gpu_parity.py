@@ -51,6 +51,45 @@ def test_adi_without_source(ctx, ngrid, nslice):
     assert synth.rel_err(got, ref) < TOL
 
 
+# the row solve at the edges of its lanes (one element, a last lane of one or of
+# all its elements) and of its coefficients: r = delz / (4 ks dgrid^2) from the
+# configurations' 0.02 (one scan step) to 40 (all of them, |q| near 1), backwards
+# and zero.  The recurrences are stable and the matrix's condition number is
+# below 1 + 4 |r|, so a step errs by at most some n (1 + 4 |r|) roundings.
+@pytest.mark.parametrize("r", [0.02, 1.0, 40.0, -0.5, 0.0])
+@pytest.mark.parametrize("ngrid", [2, 3, 16, 32, 33, 80, 81, 160, 161, 257])
+def test_adi_row_solve_at_its_edges(ctx, ngrid, r):
+    nslice, gridmax = 2, 200e-6
+    f0 = synth.field(nslice, ngrid, gridmax, seed=ngrid)
+    xks, dgrid = 2 * np.pi / synth.LAMBDA0, 2 * gridmax / (ngrid - 1)
+    step = synth.drift_step(delz=4 * r * xks * dgrid ** 2)
+    off = np.zeros(nslice + 1, np.int64)
+    parts = {k: np.zeros(0) for k in dev.BeamState.NAMES}
+    ref = f0.copy()
+    for _ in range(2):
+        orc.adi_advance(ref, harm=1, gridmax=gridmax, xks=xks, delz=step.delz, fc=0.0,
+                        enabled=True, step=step, off=off, current=np.zeros(nslice), parts=parts)
+    bound = 4 * ngrid * (1 + 4 * abs(r))
+    fld = dev.FieldState(ctx, nslice, ngrid, gridmax, synth.LAMBDA0)
+    fld.upload(f0)
+    adi = dev.FieldSolverADICUDA(ctx)
+    adi.init(step.delz, fld.dgrid, fld.xks, ngrid)
+    beam = _beam(ctx, off, parts)
+    for _ in range(2):
+        adi.advance(fld, beam, step, fc=0.0)
+    assert synth.rel_err(fld.download(), ref) < bound * 2.0 ** -53
+    run = dev.Run(ctx, off, fields=[(1, ngrid, gridmax)], lambda0=synth.LAMBDA0,
+                  gamma_ref=synth.GAMMA0, time_run=False)
+    run.upload_field(0, f0)
+    run.set_lattice([step] * 2, [[0.0]] * 2, [0.0] * 2)
+    for layout in {run.layouts()[0], 107 if ngrid == 81 else run.layouts()[0]}:
+        run.upload_field(0, f0)
+        run.set_layouts([layout])
+        run.advance(0, 2, graph=False)
+        assert synth.rel_err(run.download_field(0)[0], ref) < bound * 2.0 ** -24
+    run.close()
+
+
 @pytest.mark.parametrize("ngrid,nslice,first", [(33, 3, 1), (151, 2, 0), (201, 3, 2)])
 def test_adi_with_deposited_source(ctx, ngrid, nslice, first):
     gridmax = 200e-6
