@@ -458,10 +458,10 @@ __global__ void __launch_bounds__(BandW<T, L>::value * 32, AdiBlocks<T, M, L>::v
 // ------------------------------------------------------------ deposition ---
 // Deterministic replacement of adi_zero_source_grid + adi_deposit_source_atomic
 // (src/Core/FieldSolverADICUDA.cpp:98-174).  One CTA per beam slice:
-//  1. a pass over the slice's particles finds the largest per-particle weight
-//     q = sqrt(faw2)/gamma and the bounding box of the touched cells;
+//  1. a pass over the slice's particles finds a bound q of the per-particle
+//     weights sqrt(faw2)/gamma and the bounding box of the touched cells;
 //  2. the box is accumulated in shared memory as int64 fixed point with the
-//     exponent 2^E chosen so that count * max q * 2^E < 2^62 (integer adds are
+//     exponent 2^E chosen so that count * q * 2^E < 2^62 (integer adds are
 //     associative, so the result does not depend on the order of the atomics);
 //  3. the CTA writes only the box, scl * sum * 2^-E, as a compact tile of the
 //     target slice, and the tile's (x0, y0, width, height) descriptor; the
@@ -475,16 +475,22 @@ struct DepositArgs {
   int4* desc;          // per target slice
   size_t src_cap;
   int nslice, n, ld, first, harm, acc_cells;
-  double gridmax, dgrid, ax, ay, kx, ky, gradx, grady;
+  double gridmax, dgrid, inv_dgrid, ax, ay, kx, ky, gradx, grady;
   int* err;
 };
+
+// x / dgrid by the reciprocal and one Newton correction of the quotient.
+__device__ __forceinline__ double dep_over_dgrid(const DepositArgs& a, double x) {
+  const double t = x * a.inv_dgrid;
+  return fma(fma(-t, a.dgrid, x), a.inv_dgrid, t);
+}
 
 __device__ __forceinline__ bool dep_cell(const DepositArgs& a, double xp, double yp,
                                          int& ix, int& iy, double& wx, double& wy) {
   if (!(xp > -a.gridmax && xp < a.gridmax && yp > -a.gridmax && yp < a.gridmax))
     return false;
-  const double wx_raw = (xp + a.gridmax) / a.dgrid;
-  const double wy_raw = (yp + a.gridmax) / a.dgrid;
+  const double wx_raw = dep_over_dgrid(a, xp + a.gridmax);
+  const double wy_raw = dep_over_dgrid(a, yp + a.gridmax);
   ix = (int)floor(wx_raw);
   iy = (int)floor(wy_raw);
   if (ix < 0 || ix >= a.n - 1 || iy < 0 || iy >= a.n - 1) return false;
@@ -493,12 +499,10 @@ __device__ __forceinline__ bool dep_cell(const DepositArgs& a, double xp, double
   return true;
 }
 
-__device__ __forceinline__ double dep_weight(const DepositArgs& a, double xp,
-                                             double yp, double g) {
+// The particle's charge weight is sqrt(faw2) / gamma.
+__device__ __forceinline__ double dep_faw2(const DepositArgs& a, double xp, double yp) {
   const double dx = xp - a.ax, dy = yp - a.ay;
-  const double faw2 = 1.0 + a.kx * dx * dx + a.ky * dy * dy +
-                      2.0 * (a.gradx * dx + a.grady * dy);
-  return sqrt(faw2) / g;
+  return 1.0 + a.kx * dx * dx + a.ky * dy * dy + 2.0 * (a.gradx * dx + a.grady * dy);
 }
 
 template <typename V>
@@ -518,12 +522,21 @@ __device__ __forceinline__ V block_reduce(V v, V* sh, bool is_max) {
   return r;
 }
 
-constexpr int kDepFp64U = 2;  // particles in flight per thread (FP64 deposition)
+constexpr int kDepFp64U = 2;  // particles in flight per thread (the first pass)
+// One CTA of 1024 threads per SM with a band of 12800 cells: tiles of 80-110
+// cells a side are one band, so a particle's cell, weight and phase are worked
+// out once (two 512-thread CTAs with bands of 6144 cells: twice the cells and
+// the first pass's divisions; us per launch with 256 slices of 8192 at 201^2:
+// 89 -> 64, 64 slices of 4096 at 255^2 43 -> 27, 40 slices of 4096 at 401^2 72 ->
+// 46, 1 slice of 8192 42 -> 31).  Bound by the FP64 chain of a particle: sincos,
+// square root, division.
+constexpr int kDepFp64Threads = 1024;
+constexpr size_t kDepFp64Acc = 200 * 1024;  // accumulators: 12800 cells, one band in most runs
 
-__global__ void __launch_bounds__(512, 2) deposit_slice_kernel(const DepositArgs a) {
+__global__ void __launch_bounds__(kDepFp64Threads, 1) deposit_slice_kernel(const DepositArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ double shd[16];
-  __shared__ int shi[16];
+  __shared__ double shd[32];
+  __shared__ int shi[32];
   ptx::pdl_wait();
   unsigned long long* acc = reinterpret_cast<unsigned long long*>(smem);
   const int bs = blockIdx.x;
@@ -533,7 +546,9 @@ __global__ void __launch_bounds__(512, 2) deposit_slice_kernel(const DepositArgs
   const int64_t p0 = a.off[bs], p1 = a.off[bs + 1];
   const double scl = a.scl[bs];
 
-  double qmax = 0.0;
+  // largest faw2 and smallest |gamma| of the particles in the grid: their
+  // weights are at most sqrt(fmx) / gmn
+  double fmx = 0.0, gmn = INFINITY;
   int ixmin = 1 << 30, iymin = 1 << 30, ixmax = -1, iymax = -1, cnt = 0;
   const int nt = blockDim.x;
   if (scl != 0.0) {
@@ -556,9 +571,10 @@ __global__ void __launch_bounds__(512, 2) deposit_slice_kernel(const DepositArgs
         int ix, iy;
         double wx, wy;
         if (!dep_cell(a, lx[u], ly[u], ix, iy, wx, wy)) continue;
-        const double q = fabs(dep_weight(a, lx[u], ly[u], lg[u]));
-        qmax = q > qmax ? q : qmax;
-        if (!(q <= 1e300)) qmax = INFINITY;  // NaN or inf
+        const double f = dep_faw2(a, lx[u], ly[u]), g = fabs(lg[u]);
+        fmx = f > fmx ? f : fmx;
+        gmn = g < gmn ? g : gmn;
+        if (!(f >= 0.0 && f < 1e300 && g > 1e-290)) fmx = INFINITY;  // no finite weight
         ixmin = min(ixmin, ix);
         ixmax = max(ixmax, ix);
         iymin = min(iymin, iy);
@@ -567,7 +583,9 @@ __global__ void __launch_bounds__(512, 2) deposit_slice_kernel(const DepositArgs
       }
     }
   }
-  qmax = block_reduce<double>(qmax, shd, true);
+  fmx = block_reduce<double>(fmx, shd, true);
+  gmn = block_reduce<double>(gmn, shd, false);
+  const double qmax = fmx < INFINITY ? sqrt(fmx) / gmn : INFINITY;
   ixmin = block_reduce<int>(ixmin, shi, false);
   ixmax = block_reduce<int>(ixmax, shi, true);
   iymin = block_reduce<int>(iymin, shi, false);
@@ -613,46 +631,72 @@ __global__ void __launch_bounds__(512, 2) deposit_slice_kernel(const DepositArgs
     int* him = hre + ncell;
     for (int i = tid; i < 2 * ncell; i += blockDim.x) acc[i] = 0ull;
     __syncthreads();
-    for (int64_t pb = p0 + tid; pb < p1; pb += (int64_t)kDepFp64U * nt) {
-      double lx[kDepFp64U], ly[kDepFp64U], lg[kDepFp64U], lt[kDepFp64U];
+    auto add = [&](int cell, long long cr, long long ci) {
+      const unsigned int rlo = (unsigned int)cr, ilo = (unsigned int)ci;
+      const unsigned int rold = atomicAdd(&lre[cell], rlo);
+      const unsigned int iold = atomicAdd(&lim[cell], ilo);
+      atomicAdd(&hre[cell], (int)(cr >> 32) + (rold + rlo < rold ? 1 : 0));
+      atomicAdd(&him[cell], (int)(ci >> 32) + (iold + ilo < iold ? 1 : 0));
+    };
+    // One particle per lane, the next one's loads in flight.  Four consecutive
+    // particles of one base cell (a quiet-start beamlet: nbins = 4 particles at
+    // one transverse position) are summed over their lanes, each of which adds
+    // one corner (the same integer sums by a quarter of the atomics).
+    const int l = tid & 31;
+    const int64_t np = p1 - p0;
+    double nx = 0, ny = 0, ng = 1, nt_ = 0;
+    auto load = [&](int64_t p) {
+      if (p < np) {
+        nx = a.x[p0 + p];
+        ny = a.y[p0 + p];
+        ng = a.gamma[p0 + p];
+        nt_ = a.theta[p0 + p];
+      }
+    };
+    load(tid);
+    for (int64_t p = tid; p - l < np; p += nt) {  // whole warps
+      const double xp = nx, yp = ny, gp = ng, tp = nt_;
+      load(p + nt);
+      int cid = -1, ix, iy;  // (ext row iy - yb + 1, column) of the base cell
+      double wx, wy;
+      if (p < np && dep_cell(a, xp, yp, ix, iy, wx, wy) && iy + 1 >= yb && iy < yb + hb)
+        cid = (iy - yb + 1) * bw + (ix - bx0);
+      const int lead = __shfl_sync(0xffffffffu, cid, l & ~3);
+      const unsigned match = __ballot_sync(0xffffffffu, cid >= 0 && cid == lead);
+      const bool same = ((match >> (l & ~3)) & 15u) == 15u;
+      // (re, im) of the corners (ix, iy), (ix + 1, iy), (ix, iy + 1), (ix + 1, iy + 1)
+      long long c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (cid >= 0) {
+        const double q = sqrt(dep_faw2(a, xp, yp)) / gp;
+        double sn, cs;
+        sincos(hphase * tp, &sn, &cs);
+        const double vre = sn * q * scale, vim = cs * q * scale;
+        const double w[4] = {wx * wy, (1.0 - wx) * wy, wx * (1.0 - wy), (1.0 - wx) * (1.0 - wy)};
 #pragma unroll
-      for (int u = 0; u < kDepFp64U; ++u) {
-        const int64_t p = pb + (int64_t)u * nt;
-        if (p < p1) {
-          lx[u] = a.x[p];
-          ly[u] = a.y[p];
-          lg[u] = a.gamma[p];
-          lt[u] = a.theta[p];
+        for (int k = 0; k < 4; ++k) {
+          c[2 * k] = __double2ll_rn(vre * w[k]);
+          c[2 * k + 1] = __double2ll_rn(vim * w[k]);
         }
       }
+      // a beamlet's sums: lane l ends with the corner of row (l & 2), column (l & 1)
+      const bool up = (l & 2) != 0, right = (l & 1) != 0;
+      long long k[4];
 #pragma unroll
-      for (int u = 0; u < kDepFp64U; ++u) {
-      if (pb + (int64_t)u * nt >= p1) break;
-      int ix, iy;
-      double wx, wy;
-      const double xp = lx[u], yp = ly[u];
-      if (!dep_cell(a, xp, yp, ix, iy, wx, wy)) continue;
-      if (iy + 1 < yb || iy >= yb + hb) continue;
-      const double q = dep_weight(a, xp, yp, lg[u]);
-      double sn, cs;
-      sincos(hphase * lt[u], &sn, &cs);
-      const double vre = sn * q * scale, vim = cs * q * scale;
-      const double w[4] = {wx * wy, (1.0 - wx) * wy, wx * (1.0 - wy),
-                           (1.0 - wx) * (1.0 - wy)};
-      const int cx[4] = {ix, ix + 1, ix, ix + 1};
-      const int cy[4] = {iy, iy, iy + 1, iy + 1};
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int ry = cy[c] - yb;
-        if (ry < 0 || ry >= hb) continue;
-        const int cell = ry * bw + (cx[c] - bx0);
-        const long long cr = __double2ll_rn(vre * w[c]), ci = __double2ll_rn(vim * w[c]);
-        const unsigned int rlo = (unsigned int)cr, ilo = (unsigned int)ci;
-        const unsigned int rold = atomicAdd(&lre[cell], rlo);
-        const unsigned int iold = atomicAdd(&lim[cell], ilo);
-        atomicAdd(&hre[cell], (int)(cr >> 32) + (rold + rlo < rold ? 1 : 0));
-        atomicAdd(&him[cell], (int)(ci >> 32) + (iold + ilo < iold ? 1 : 0));
-      }
+      for (int i = 0; i < 4; ++i)
+        k[i] = (up ? c[4 + i] : c[i]) + __shfl_xor_sync(0xffffffffu, up ? c[i] : c[4 + i], 2);
+      const long long cr = (right ? k[2] : k[0]) + __shfl_xor_sync(0xffffffffu, right ? k[0] : k[2], 1);
+      const long long ci = (right ? k[3] : k[1]) + __shfl_xor_sync(0xffffffffu, right ? k[1] : k[3], 1);
+      if (same) {
+        if (up ? cid < ncell : cid >= bw) add((up ? cid : cid - bw) + (right ? 1 : 0), cr, ci);
+      } else if (cid >= 0) {
+        if (cid >= bw) {
+          add(cid - bw, c[0], c[1]);
+          add(cid - bw + 1, c[2], c[3]);
+        }
+        if (cid < ncell) {
+          add(cid, c[4], c[5]);
+          add(cid + 1, c[6], c[7]);
+        }
       }
     }
     __syncthreads();
@@ -916,14 +960,16 @@ int fp64_deposit(g4b_field* f, g4b_beam* b, const g4b_step* st, double fc) {
   da.gradx = st->gradx;
   da.grady = st->grady;
   da.err = c->d_error;
-  const size_t acc_bytes = 96 * 1024;
+  const size_t acc_bytes = kDepFp64Acc;
   da.acc_cells = (int)(acc_bytes / 16);
+  da.inv_dgrid = 1.0 / f->dgrid;
   G4B_CUDA_TRY(cudaFuncSetAttribute(deposit_slice_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)acc_bytes));  // per device, cheap
   {
     LaunchScope ls(c, "deposit");
-    G4B_CUDA_TRY(launch_pdl(deposit_slice_kernel, (unsigned)f->nslice, 512, acc_bytes, c->stream, da));
+    G4B_CUDA_TRY(launch_pdl(deposit_slice_kernel, (unsigned)f->nslice, kDepFp64Threads,
+                            acc_bytes, c->stream, da));
   }
   if (int rc = check_launch(c, "deposit_slice_kernel")) return rc;
   return G4B_OK;
