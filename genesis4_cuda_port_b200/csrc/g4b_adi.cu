@@ -25,16 +25,17 @@
 //   u_k - u_0 (q^{k+2} - q^{2n+2-k}) / (1 - q^{2n+2}).
 // A warp evaluates them: every lane runs the recurrences over its own M
 // consecutive elements, the lane carries are combined by a Kogge-Stone scan of
-// affine maps with multipliers q^(M 2^t) (only the steps whose multiplier
-// matters at this precision: |q| is 0.02 at the configurations' r, so one step
-// in place of five), and each lane adds its carry times a power of q.  All
+// affine maps with multipliers q^(M 2^t) (only the steps whose multiplier is
+// not zero at this precision: |q| is 0.02 at the configurations' r, so one step
+// in place of four for FP32 rows of 201), and each lane adds its carry times a
+// power of q.  All
 // coefficients but the lanes' wall terms are the same in every lane: the
 // single-run kernels read them from the constant bank.  With the Thomas pivots
 // and the products of their factors in per-lane tables the passes spent as much
 // of the load path on coefficients (four loads per element) as on the field:
-// per pass X / Y of 1024 slices of 201^2 in FP32 152 / 136 -> 138 / 124 us (4.8
+// per pass X / Y of 1024 slices of 201^2 in FP32 152 / 136 -> 140 / 125 us (4.7
 // and 5.3 TB/s of the field read and written), of 256 slices in FP64 96 / 83 ->
-// 80 / 66 us, of 40 slices of 401^2 98 / 77 -> 86 / 65 us.
+// 84 / 68 us, of 40 slices of 401^2 98 / 77 -> 90 / 70 us.
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -1005,13 +1006,11 @@ void row_tables(double r, int n, int M, int L, RowConst<C>& K, std::vector<unsig
   K = RowConst<C>{};
   for (int m = 0; m < kRowMaxM + 2; ++m) K.P[m] = round(power(m));
   K.cb = round(1.0L / beta);
-  // a dropped scan step changes a carry by less than 2^-75 (FP32: 2^-45) of
-  // the largest, far below its rounding
-  const long double drop = sizeof(T) == 8 ? 0x1p-75L : 0x1p-45L;
+  // scan steps whose multiplier rounds to zero are left out (no more than that:
+  // the field far outside the beam is a power of q, small but exact)
   for (int t = 0; (1 << t) < L; ++t) {
-    const cld A = power((long long)M << t);
-    K.A[t] = round(A);
-    if (std::abs(A) >= drop) K.nscan = t + 1;
+    K.A[t] = round(power((long long)M << t));
+    if (K.A[t].x != 0 || K.A[t].y != 0) K.nscan = t + 1;
   }
   std::vector<C> wall(2 * L, C{0, 0});
   const cld den = 1.0L - power(2LL * n + 2);

@@ -123,7 +123,7 @@ struct g4b_beam {
 namespace g4b {
 // Coefficients of the tridiagonal row solve (g4b_adi.cu) with M elements per
 // lane: P[m] = q^m, A[t] = q^(M 2^t), 1 / beta, and the scan steps whose A[t]
-// matters at the precision of C.
+// is not zero at the precision of C.
 constexpr int kRowMaxM = 33;
 template <typename C>
 struct RowConst {

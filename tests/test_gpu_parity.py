@@ -53,7 +53,7 @@ def test_adi_without_source(ctx, ngrid, nslice):
 
 # the row solve at the edges of its lanes (one element, a last lane of one or of
 # all its elements) and of its coefficients: r = delz / (4 ks dgrid^2) from the
-# configurations' 0.02 (one scan step) to 40 (all of them, |q| near 1), backwards
+# configurations' 0.02 to 40 (|q| near 1), backwards
 # and zero.  The recurrences are stable and the matrix's condition number is
 # below 1 + 4 |r|, so a step errs by at most some n (1 + 4 |r|) roundings.
 @pytest.mark.parametrize("r", [0.02, 1.0, 40.0, -0.5, 0.0])
@@ -88,6 +88,30 @@ def test_adi_row_solve_at_its_edges(ctx, ngrid, r):
         run.advance(0, 2, graph=False)
         assert synth.rel_err(run.download_field(0)[0], ref) < bound * 2.0 ** -24
     run.close()
+
+
+# Far from a localised field the solution falls by |q| per cell, over hundreds of
+# orders of magnitude, and stays relatively accurate: each cell is a product of
+# up to 2 n powers, so some 4 n roundings.
+@pytest.mark.parametrize("ngrid", [64, 151, 182, 201])
+def test_adi_far_field_is_relatively_accurate(ctx, ngrid):
+    gridmax = 200e-6
+    f0 = np.zeros((1, ngrid, ngrid), np.complex128)
+    f0[0, ngrid // 2, ngrid // 2] = 1e12
+    fld = dev.FieldState(ctx, 1, ngrid, gridmax, synth.LAMBDA0)
+    fld.upload(f0)
+    step = synth.drift_step(delz=0.015)
+    off = np.zeros(2, np.int64)
+    parts = {k: np.zeros(0) for k in dev.BeamState.NAMES}
+    adi = dev.FieldSolverADICUDA(ctx)
+    adi.init(step.delz, fld.dgrid, fld.xks, ngrid)
+    adi.advance(fld, _beam(ctx, off, parts), step, fc=0.0)
+    orc.adi_advance(f0, harm=1, gridmax=gridmax, xks=fld.xks, delz=step.delz, fc=0.0,
+                    enabled=True, step=step, off=off, current=np.zeros(1), parts=parts)
+    got = fld.download()
+    ok = np.abs(f0) > 1e-280
+    assert ok.sum() > 0.5 * ok.size
+    assert np.max(np.abs(got[ok] - f0[ok]) / np.abs(f0[ok])) < 4 * ngrid * 2.0 ** -53
 
 
 @pytest.mark.parametrize("ngrid,nslice,first", [(33, 3, 1), (151, 2, 0), (201, 3, 2)])
