@@ -1,10 +1,21 @@
 // g4b_diag.cu -- per-slice beam and field diagnostics (DiagnosticCUDA) for sm_100a.
 //
-// One CTA per slice reads its particles (or its field plane) once and keeps
-// every moment in registers; reductions run in a fixed order (warp xor tree,
-// then warps in index order), so results are reproducible run to run.
+// A CTA reads its share of a slice's particles (or of the rows of its field
+// plane) once and keeps every moment in registers; reductions run in a fixed
+// order (warp xor tree, then warps in index order).  A slice is split over
+// `parts` CTAs where there are fewer slices than the GPU holds CTAs; every CTA
+// writes one record, and the host, which is what the results are for, adds the
+// parts in order.  The entry points' records go straight to pinned host memory,
+// so a call is one launch and one synchronisation (before: one CTA per slice, a
+// device buffer and two or three copies to pageable memory; 60 FP64 steps of one
+// slice with both diagnostics every step 11.4 -> 6.3 ms).  Per launch, beam /
+// field: 1 slice of 8192 and 151^2 24 / 24 -> 13 / 11 us, 256 slices of 8192 and
+// 201^2 45 / 60 -> 39 / 44 us, 300 slices of 5000 with four harmonics 61 -> 43 us.
+// Bound by the latency of the loads and, with several harmonics, by the FP64
+// pipe.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -15,7 +26,6 @@ namespace g4b {
 
 constexpr int kDiagThreads = 256;
 constexpr int kDiagWarps = kDiagThreads / 32;
-constexpr int kMaxHarmPass = 8;  // harmonics accumulated per pass
 
 enum class Red { Sum, Min, Max };
 
@@ -27,22 +37,27 @@ __device__ __forceinline__ double warp_red(double v, Red op) {
   return v;
 }
 
+struct BeamRecArgs {
+  const int64_t* off;
+  const double *x, *y, *px, *py, *gamma, *theta;
+  double* rec;  // [nslice][parts][23 + 2 nharm]
+  int nharm, need_aux, parts;
+};
+
 // g4_beam_slice_reduce_kernel (src/Core/DiagnosticCUDA.cpp:188-303); HP
-// harmonics accumulated per pass over the particles.  For the fundamental
-// alone (HP = 1) three CTAs per SM at 80 registers: 157 -> 119 us per
-// 1024 x 8192 particles against one CTA size for all (the same arithmetic).
+// harmonics accumulated per pass over the particles, the higher ones from one
+// sincos by multiplication with e^{i theta}.  U particles in flight per thread.
 template <int HP>
-__global__ void __launch_bounds__(kDiagThreads, HP == 1 ? 3 : 1)
-    beam_diag_kernel(int nslice, int nharm, int need_aux, const int64_t* off,
-                     const double* x, const double* y, const double* px, const double* py,
-                     const double* gamma, const double* theta, double* stats, double* bre,
-                     double* bim) {
+__global__ void __launch_bounds__(kDiagThreads, HP <= 4 ? 2 : 1)
+    beam_diag_kernel(const __grid_constant__ BeamRecArgs a) {
+  constexpr int U = HP == 1 ? 4 : 2;
   __shared__ double part[kDiagWarps][23 + 2 * HP];
   ptx::pdl_wait();
-  const int is = blockIdx.x;
-  if (is >= nslice) return;
+  const int is = blockIdx.x / a.parts, ip = blockIdx.x % a.parts;
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
-  const int64_t p0 = off[is], p1 = off[is + 1];
+  const int64_t q0 = a.off[is], all = a.off[is + 1] - q0, per = (all + a.parts - 1) / a.parts;
+  const int64_t p0 = q0 + min(all, ip * per), p1 = q0 + min(all, (ip + 1) * per);
+  double* rec = a.rec + (size_t)blockIdx.x * (23 + 2 * a.nharm);
   double v[23];
 #pragma unroll
   for (int k = 0; k < 13; ++k) v[k] = 0.0;
@@ -51,140 +66,124 @@ __global__ void __launch_bounds__(kDiagThreads, HP == 1 ? 3 : 1)
   v[17] = 1.0e5; v[18] = -1.0e5;  // ymin ymax
   v[19] = 1.0e5; v[20] = -1.0e5;  // pymin pymax
   v[21] = 1.0e7; v[22] = 1.0;     // gmin gmax
-  const int h0n = min(nharm, HP);
-  double br[HP], bi[HP];
+  for (int hb = 0; hb < a.nharm; hb += HP) {
+    const int hn = min(a.nharm - hb, HP);
+    double br[HP], bi[HP];
 #pragma unroll
-  for (int h = 0; h < HP; ++h) br[h] = bi[h] = 0.0;
-  for (int64_t p = p0 + tid; p < p1; p += kDiagThreads) {
-    const double xv = x[p], yv = y[p], pxv = px[p], pyv = py[p], gv = gamma[p];
-    v[0] += gv;
-    v[1] += gv * gv;
-    v[2] += xv;
-    v[3] += xv * xv;
-    v[4] += yv;
-    v[5] += yv * yv;
-    v[6] += pxv;
-    v[7] += pxv * pxv;
-    v[8] += pyv;
-    v[9] += pyv * pyv;
-    v[10] += xv * pxv;
-    v[11] += yv * pyv;
-    v[12] += 1.0;
-    if (need_aux) {
-      v[13] = fmin(v[13], xv); v[14] = fmax(v[14], xv);
-      v[15] = fmin(v[15], pxv); v[16] = fmax(v[16], pxv);
-      v[17] = fmin(v[17], yv); v[18] = fmax(v[18], yv);
-      v[19] = fmin(v[19], pyv); v[20] = fmax(v[20], pyv);
-      v[21] = fmin(v[21], gv); v[22] = fmax(v[22], gv);
-    }
-    const double th = theta[p];
+    for (int h = 0; h < HP; ++h) br[h] = bi[h] = 0.0;
+    for (int64_t pb = p0 + tid; pb < p1; pb += U * kDiagThreads) {
+      double lx[U], ly[U], lpx[U], lpy[U], lg[U], lt[U];
 #pragma unroll
-    for (int h = 0; h < HP; ++h) {
-      if (h < h0n) {
-        double s, c;
-        sincos((double)(h + 1) * th, &s, &c);
-        br[h] += c;
-        bi[h] += s;
+      for (int u = 0; u < U; ++u) {
+        const int64_t p = pb + u * kDiagThreads;
+        if (p < p1) {
+          lt[u] = a.theta[p];
+          if (hb == 0) {
+            lx[u] = a.x[p];
+            ly[u] = a.y[p];
+            lpx[u] = a.px[p];
+            lpy[u] = a.py[p];
+            lg[u] = a.gamma[p];
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (pb + u * kDiagThreads >= p1) break;
+        if (hb == 0) {
+          const double xv = lx[u], yv = ly[u], pxv = lpx[u], pyv = lpy[u], gv = lg[u];
+          v[0] += gv;
+          v[1] += gv * gv;
+          v[2] += xv;
+          v[3] += xv * xv;
+          v[4] += yv;
+          v[5] += yv * yv;
+          v[6] += pxv;
+          v[7] += pxv * pxv;
+          v[8] += pyv;
+          v[9] += pyv * pyv;
+          v[10] += xv * pxv;
+          v[11] += yv * pyv;
+          v[12] += 1.0;
+          if (a.need_aux) {
+            v[13] = fmin(v[13], xv); v[14] = fmax(v[14], xv);
+            v[15] = fmin(v[15], pxv); v[16] = fmax(v[16], pxv);
+            v[17] = fmin(v[17], yv); v[18] = fmax(v[18], yv);
+            v[19] = fmin(v[19], pyv); v[20] = fmax(v[20], pyv);
+            v[21] = fmin(v[21], gv); v[22] = fmax(v[22], gv);
+          }
+        }
+        double s1, c1;
+        sincos(lt[u], &s1, &c1);
+        double s = s1, c = c1;
+        if (hb > 0) sincos((double)(hb + 1) * lt[u], &s, &c);
+#pragma unroll
+        for (int h = 0; h < HP; ++h) {
+          if (h >= hn) break;
+          br[h] += c;
+          bi[h] += s;
+          if (h + 1 < HP) {
+            const double t = fma(c, c1, -s * s1);
+            s = fma(s, c1, c * s1);
+            c = t;
+          }
+        }
       }
     }
-  }
+    if (hb == 0) {
 #pragma unroll
-  for (int k = 0; k < 23; ++k) {
-    const Red op = k < 13 ? Red::Sum : ((k - 13) % 2 == 0 ? Red::Min : Red::Max);
-    const double r = warp_red(v[k], op);
-    if (l == 0) part[w][k] = r;
-  }
+      for (int k = 0; k < 23; ++k) {
+        const Red op = k < 13 ? Red::Sum : ((k - 13) % 2 == 0 ? Red::Min : Red::Max);
+        const double r = warp_red(v[k], op);
+        if (l == 0) part[w][k] = r;
+      }
+    }
 #pragma unroll
-  for (int h = 0; h < HP; ++h) {
-    if (h < h0n) {
+    for (int h = 0; h < HP; ++h) {
+      if (h >= hn) break;
       const double rr = warp_red(br[h], Red::Sum), ri = warp_red(bi[h], Red::Sum);
       if (l == 0) {
         part[w][23 + 2 * h] = rr;
         part[w][24 + 2 * h] = ri;
       }
     }
-  }
-  __syncthreads();
-  if (tid < 23) {
-    const int k = tid;
-    const Red op = k < 13 ? Red::Sum : ((k - 13) % 2 == 0 ? Red::Min : Red::Max);
-    double r = part[0][k];
-    for (int i = 1; i < kDiagWarps; ++i) {
-      const double t = part[i][k];
-      r = op == Red::Sum ? r + t : (op == Red::Min ? fmin(r, t) : fmax(r, t));
-    }
-    if (k >= 13 && !need_aux) r = 0.0;
-    stats[(size_t)is * 23 + k] = r;
-  } else if (tid >= 32 && tid < 32 + 2 * h0n) {
-    const int k = tid - 32;
-    double r = part[0][23 + k];
-    for (int i = 1; i < kDiagWarps; ++i) r += part[i][23 + k];
-    const int h = k >> 1;
-    if (k & 1)
-      bim[(size_t)is * nharm + h] = r;
-    else
-      bre[(size_t)is * nharm + h] = r;
-  }
-  // further harmonics, HP at a time
-  for (int hb = HP; hb < nharm; hb += HP) {
-    const int hn = min(nharm - hb, HP);
-#pragma unroll
-    for (int h = 0; h < HP; ++h) br[h] = bi[h] = 0.0;
-    for (int64_t p = p0 + tid; p < p1; p += kDiagThreads) {
-      const double th = theta[p];
-#pragma unroll
-      for (int h = 0; h < HP; ++h) {
-        if (h < hn) {
-          double s, c;
-          sincos((double)(hb + h + 1) * th, &s, &c);
-          br[h] += c;
-          bi[h] += s;
-        }
+    __syncthreads();
+    if (tid < 23 + 2 * hn && (hb == 0 || tid >= 23)) {
+      const int k = tid;
+      const Red op = k < 13 || k >= 23 ? Red::Sum : ((k - 13) % 2 == 0 ? Red::Min : Red::Max);
+      double r = part[0][k];
+      for (int i = 1; i < kDiagWarps; ++i) {
+        const double t = part[i][k];
+        r = op == Red::Sum ? r + t : (op == Red::Min ? fmin(r, t) : fmax(r, t));
       }
+      rec[k < 23 ? k : k + 2 * hb] = r;
     }
     __syncthreads();
-#pragma unroll
-    for (int h = 0; h < HP; ++h) {
-      if (h < hn) {
-        const double rr = warp_red(br[h], Red::Sum), ri = warp_red(bi[h], Red::Sum);
-        if (l == 0) {
-          part[w][2 * h] = rr;
-          part[w][2 * h + 1] = ri;
-        }
-      }
-    }
-    __syncthreads();
-    if (tid < 2 * hn) {
-      double r = part[0][tid];
-      for (int i = 1; i < kDiagWarps; ++i) r += part[i][tid];
-      const int h = hb + (tid >> 1);
-      if (tid & 1)
-        bim[(size_t)is * nharm + h] = r;
-      else
-        bre[(size_t)is * nharm + h] = r;
-    }
   }
 }
 
-// g4_field_slice_reduce_kernel (src/Core/DiagnosticCUDA.cpp:305-363)
+// g4_field_slice_reduce_kernel (src/Core/DiagnosticCUDA.cpp:305-363): records
+// [nslice][parts][9], seven sums and (in the first part) the centre cell; part
+// ip takes the rows of its warps, parts * 8 rows apart.
 template <typename C>
 __global__ void __launch_bounds__(kDiagThreads)
-    field_diag_kernel(int nslice, int n, int ld, int first, const C* cells, double* stats,
-                      double* center) {
+    field_diag_kernel(int nslice, int n, int ld, int first, int parts, const C* cells,
+                      double* rec) {
   __shared__ double part[kDiagWarps][7];
-  const int is0 = blockIdx.x;
-  if (is0 >= nslice) return;
+  ptx::pdl_wait();
+  const int is0 = blockIdx.x / parts, ip = blockIdx.x % parts;
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   const C* c = cells + (size_t)is0 * n * ld;
   const int is = (nslice + is0 - first) % nslice;
+  rec += ((size_t)is * parts + ip) * 9;
   const double shift = -0.5 * (double)(n - 1);
   double v[7] = {0, 0, 0, 0, 0, 0, 0};
-  const int plane = n * n;
   // a warp per row: coalesced row reads with no index division, the row's
   // sums first, then its y moments from the row's power
-  for (int iy = w; iy < n; iy += kDiagWarps) {
+  for (int iy = ip * kDiagWarps + w; iy < n; iy += parts * kDiagWarps) {
     const C* row = c + (size_t)iy * ld;
     double p = 0, px = 0, pxx = 0, sre = 0, sim = 0;
+#pragma unroll 4
     for (int ix = l; ix < n; ix += 32) {
       const C u = row[ix];
       const double re = u.x, im = u.y;
@@ -214,12 +213,12 @@ __global__ void __launch_bounds__(kDiagThreads)
   if (tid < 7) {
     double r = part[0][tid];
     for (int i = 1; i < kDiagWarps; ++i) r += part[i][tid];
-    stats[(size_t)is * 7 + tid] = r;
-  } else if (tid == 32) {
-    const int ic = (plane - 1) / 2;
+    rec[tid] = r;
+  } else if (tid == 32 && ip == 0) {
+    const int ic = (n * n - 1) / 2;
     const C u = c[(size_t)(ic / n) * ld + (ic % n)];
-    center[2 * is] = u.x;
-    center[2 * is + 1] = u.y;
+    rec[7] = u.x;
+    rec[8] = u.y;
   }
 }
 
@@ -228,30 +227,68 @@ __global__ void __launch_bounds__(kDiagThreads)
 using namespace g4b;
 
 namespace {
-struct DiagScratch {
-  double* d = nullptr;
+// Pinned host memory of the diagnostics entry points that kernels write to:
+// one buffer per calling host thread (every call ends with a synchronisation,
+// so it is free again for the thread's next one, on any device), as large as
+// the thread's largest call, freed with the thread.
+struct DiagHost {
+  double* p = nullptr;
   size_t cap = 0;
+  ~DiagHost() {
+    if (p) cudaFreeHost(p);
+  }
 };
-// Grow-on-demand scratch of the diagnostics entry points, one buffer per
-// calling host thread and device: a thread may drive contexts on several
-// devices, and a buffer is only ever used (and freed) with its own device
-// current.  Freed with the process (small).
-constexpr int kDiagScratchDevices = 64;
-int diag_scratch(int device, DiagScratch** out) {
-  static thread_local DiagScratch per_device[kDiagScratchDevices];
-  if (device < 0 || device >= kDiagScratchDevices)
-    return fail(G4B_ERR_RANGE, "diagnostics: device index above 63");
-  *out = &per_device[device];
+int diag_host(size_t n, double** out) {
+  static thread_local DiagHost h;
+  if (h.cap < n) {
+    if (h.p) cudaFreeHost(h.p);
+    h.p = nullptr;
+    h.cap = 0;
+    size_t cap = 8192;
+    while (cap < n) cap *= 2;
+    G4B_CUDA_TRY(cudaHostAlloc((void**)&h.p, cap * sizeof(double), cudaHostAllocPortable));
+    h.cap = cap;
+  }
+  *out = h.p;
   return G4B_OK;
 }
-int ensure(DiagScratch& s, size_t n) {
-  if (s.cap >= n) return G4B_OK;
-  if (s.d) cudaFree(s.d);
-  s.d = nullptr;
-  s.cap = 0;
-  G4B_CUDA_TRY(cudaMalloc(&s.d, n * sizeof(double)));
-  s.cap = n;
-  return G4B_OK;
+
+// CTAs per slice: `per_sm` CTAs on every SM, but no more than `most` (a share
+// below which a CTA is not worth its launch).
+int diag_parts(g4b_ctx* c, int nslice, int per_sm, int64_t most) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(most, per_sm * c->sm_count / nslice));
+}
+int field_parts(g4b_field* f) { return diag_parts(f->ctx, f->nslice, 8, (f->ngrid + 15) / 16); }
+
+int launch_field_diag(g4b_field* f, int parts, double* rec) {
+  g4b_ctx* c = f->ctx;
+  {
+    LaunchScope ls(c, "diag_field");
+    const unsigned grid = (unsigned)(f->nslice * parts);
+    if (f->precision == G4B_FP64)
+      G4B_CUDA_TRY(launch_pdl(field_diag_kernel<double2>, grid, kDiagThreads, 0, c->stream,
+                              f->nslice, f->ngrid, f->ld, f->first, parts,
+                              static_cast<const double2*>(f->a), rec));
+    else
+      G4B_CUDA_TRY(launch_pdl(field_diag_kernel<float2>, grid, kDiagThreads, 0, c->stream,
+                              f->nslice, f->ngrid, f->ld, f->first, parts,
+                              static_cast<const float2*>(f->a), rec));
+  }
+  return check_launch(c, "field_diag_kernel");
+}
+
+// The parts' field records into the caller's arrays.
+void gather_field(const double* rec, int nslice, int parts, double* stats, double* center) {
+  for (int s = 0; s < nslice; ++s) {
+    const double* r = rec + (size_t)s * parts * 9;
+    for (int k = 0; k < 7; ++k) {
+      double t = r[k];
+      for (int p = 1; p < parts; ++p) t += r[9 * p + k];
+      stats[(size_t)s * 7 + k] = t;
+    }
+    center[2 * s] = r[7];
+    center[2 * s + 1] = r[8];
+  }
 }
 }  // namespace
 
@@ -261,9 +298,9 @@ namespace {
 // Some callers must not allocate device memory when they ask for the field
 // statistics: a host that hands the device's memory to its own pool and
 // forbids growth during a run, or a loop whose latency budget has no room for
-// cudaMalloc's implicit device-wide synchronisation.  For them the scratch of
-// field_diag_kernel lives in one fixed file-scope device array instead of the
-// grow-on-demand buffer above.  Its size bounds the slices per call.
+// an allocation's implicit device-wide synchronisation.  For them the records of
+// field_diag_kernel go to one fixed file-scope device array instead of the
+// pinned buffer above, which grows with its thread's largest call.  Its size bounds the slices per call.
 constexpr int kStaticDiagMaxSlices = 4096;               // 4096 x 9 doubles = 288 KiB
 static __device__ __align__(256) double g_field_diag_scratch[kStaticDiagMaxSlices * 9];
 
@@ -302,29 +339,36 @@ int g4b_diag_beam(g4b_beam* b, int nharm, int need_aux, double* stats, double* b
   if (b->precision != G4B_FP64) return fail(G4B_ERR_ARG, "g4b_diag_beam: FP64 beam expected");
   g4b_ctx* c = b->ctx;
   G4B_CUDA_TRY(cudaSetDevice(c->device));
-  DiagScratch* scratch = nullptr;
-  if (int rc = diag_scratch(c->device, &scratch)) return rc;
-  const size_t ns = b->nslice;
-  const size_t need = ns * 23 + 2 * ns * nharm;
-  if (int rc = ensure(*scratch, need)) return rc;
-  double* d_stats = scratch->d;
-  double* d_bre = d_stats + ns * 23;
-  double* d_bim = d_bre + ns * nharm;
+  const int ns = b->nslice, nrec = 23 + 2 * nharm;
+  const int parts = diag_parts(c, ns, 2, (b->max_slice_np + 511) / 512);
+  double* rec = nullptr;
+  if (int rc = diag_host((size_t)ns * parts * nrec, &rec)) return rc;
   {
     LaunchScope ls(c, "diag_beam");
-    auto kern = nharm == 1 ? beam_diag_kernel<1> : beam_diag_kernel<kMaxHarmPass>;
-    G4B_CUDA_TRY(launch_pdl(kern, (unsigned)b->nslice, kDiagThreads, 0, c->stream, b->nslice,
-                            nharm, need_aux, b->d_off, b->x, b->y, b->px, b->py, b->gamma,
-                            b->theta, d_stats, d_bre, d_bim));
+    const BeamRecArgs a{b->d_off, b->x,     b->y,  b->px, b->py, b->gamma,
+                        b->theta, rec, nharm, need_aux, parts};
+    auto kern = nharm == 1 ? beam_diag_kernel<1>
+                           : (nharm <= 4 ? beam_diag_kernel<4> : beam_diag_kernel<8>);
+    G4B_CUDA_TRY(launch_pdl(kern, (unsigned)(ns * parts), kDiagThreads, 0, c->stream, a));
   }
   if (int rc = check_launch(c, "beam_diag_kernel")) return rc;
-  G4B_CUDA_TRY(cudaMemcpyAsync(stats, d_stats, ns * 23 * sizeof(double),
-                               cudaMemcpyDeviceToHost, c->stream));
-  G4B_CUDA_TRY(cudaMemcpyAsync(bre, d_bre, ns * nharm * sizeof(double),
-                               cudaMemcpyDeviceToHost, c->stream));
-  G4B_CUDA_TRY(cudaMemcpyAsync(bim, d_bim, ns * nharm * sizeof(double),
-                               cudaMemcpyDeviceToHost, c->stream));
   G4B_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  for (int s = 0; s < ns; ++s) {
+    const double* r = rec + (size_t)s * parts * nrec;
+    double* st = stats + (size_t)s * 23;
+    for (int k = 0; k < nrec; ++k) {
+      const bool sum = k < 13 || k >= 23, lo = (k - 13) % 2 == 0;
+      double t = r[k];
+      for (int p = 1; p < parts; ++p) {
+        const double u = r[(size_t)p * nrec + k];
+        t = sum ? t + u : (lo ? std::fmin(t, u) : std::fmax(t, u));
+      }
+      if (k < 23)
+        st[k] = k >= 13 && !need_aux ? 0.0 : t;
+      else
+        (k % 2 ? bre : bim)[(size_t)s * nharm + (k - 23) / 2] = t;
+    }
+  }
   return G4B_OK;
 }
 
@@ -332,29 +376,12 @@ int g4b_diag_field(g4b_field* f, double* stats, double* center) {
   if (!f || !stats || !center) return fail(G4B_ERR_ARG, "g4b_diag_field: null arg");
   g4b_ctx* c = f->ctx;
   G4B_CUDA_TRY(cudaSetDevice(c->device));
-  DiagScratch* scratch = nullptr;
-  if (int rc = diag_scratch(c->device, &scratch)) return rc;
-  const size_t ns = f->nslice;
-  if (int rc = ensure(*scratch, ns * 9)) return rc;
-  double* d_stats = scratch->d;
-  double* d_center = d_stats + ns * 7;
-  {
-    LaunchScope ls(c, "diag_field");
-    if (f->precision == G4B_FP64)
-      field_diag_kernel<double2><<<f->nslice, kDiagThreads, 0, c->stream>>>(
-          f->nslice, f->ngrid, f->ld, f->first, static_cast<const double2*>(f->a), d_stats,
-          d_center);
-    else
-      field_diag_kernel<float2><<<f->nslice, kDiagThreads, 0, c->stream>>>(
-          f->nslice, f->ngrid, f->ld, f->first, static_cast<const float2*>(f->a), d_stats,
-          d_center);
-  }
-  if (int rc = check_launch(c, "field_diag_kernel")) return rc;
-  G4B_CUDA_TRY(cudaMemcpyAsync(stats, d_stats, ns * 7 * sizeof(double),
-                               cudaMemcpyDeviceToHost, c->stream));
-  G4B_CUDA_TRY(cudaMemcpyAsync(center, d_center, ns * 2 * sizeof(double),
-                               cudaMemcpyDeviceToHost, c->stream));
+  const int parts = field_parts(f);
+  double* rec = nullptr;
+  if (int rc = diag_host((size_t)f->nslice * parts * 9, &rec)) return rc;
+  if (int rc = launch_field_diag(f, parts, rec)) return rc;
   G4B_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  gather_field(rec, f->nslice, parts, stats, center);
   return G4B_OK;
 }
 
@@ -370,25 +397,16 @@ int g4b_diag_field_static(g4b_field* f, double* stats, double* center) {
                                    std::to_string(kStaticDiagMaxSlices));
   g4b_ctx* c = f->ctx;
   G4B_CUDA_TRY(cudaSetDevice(c->device));
-  double* d_stats = nullptr;
-  if (int rc = static_diag_scratch(c->device, &d_stats)) return rc;
-  const size_t ns = f->nslice;
-  double* d_center = d_stats + ns * 7;
-  if (f->precision == G4B_FP64)
-    field_diag_kernel<double2><<<f->nslice, kDiagThreads, 0, c->stream>>>(
-        f->nslice, f->ngrid, f->ld, f->first, static_cast<const double2*>(f->a), d_stats,
-        d_center);
-  else
-    field_diag_kernel<float2><<<f->nslice, kDiagThreads, 0, c->stream>>>(
-        f->nslice, f->ngrid, f->ld, f->first, static_cast<const float2*>(f->a), d_stats,
-        d_center);
-  count_launch(c);
-  if (int rc = check_launch(c, "field_diag_kernel")) return rc;
-  G4B_CUDA_TRY(cudaMemcpyAsync(stats, d_stats, ns * 7 * sizeof(double),
-                               cudaMemcpyDeviceToHost, c->stream));
-  G4B_CUDA_TRY(cudaMemcpyAsync(center, d_center, ns * 2 * sizeof(double),
+  double* rec = nullptr;
+  if (int rc = static_diag_scratch(c->device, &rec)) return rc;
+  // the records of every part fit: nslice * parts <= max(nslice, 8 CTAs per SM)
+  const int parts = std::min(field_parts(f), kStaticDiagMaxSlices / f->nslice);
+  if (int rc = launch_field_diag(f, parts, rec)) return rc;
+  std::vector<double> host((size_t)f->nslice * parts * 9);
+  G4B_CUDA_TRY(cudaMemcpyAsync(host.data(), rec, host.size() * sizeof(double),
                                cudaMemcpyDeviceToHost, c->stream));
   G4B_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  gather_field(host.data(), f->nslice, parts, stats, center);
   return G4B_OK;
 }
 

@@ -304,3 +304,25 @@ def test_full_steps_match_oracle(ctx):
         assert synth.rel_err(got[k], ref_parts[k]) < 1e-11, k
     assert fld.first == ref_field["first"]
     assert synth.rel_err(fld.download(), ref_field["cells"]) < 1e-11
+
+
+# slices split over several CTAs (down to 512 particles and 16 rows each) and
+# not, one harmonic pass and several, particle counts off every tile.  The sums
+# are FP64 additions of at most N terms: a few N roundings of the largest.
+@pytest.mark.parametrize("nslice,npart,ngrid,nharm", [(1, 1, 2, 1), (1, 513, 17, 2), (1, 9001, 151, 4),
+                                                      (3, 2047, 64, 5), (40, 700, 33, 9),
+                                                      (700, 300, 9, 1)])
+def test_diagnostics_split_over_ctas(ctx, nslice, npart, ngrid, nharm):
+    off, parts = synth.beam(nslice, npart, seed=nslice, ragged=nslice > 1)
+    beam = _beam(ctx, off, parts)
+    got, want = beam.diagnostics(nharm, True), orc.diag_beam(off, parts, nharm, True)
+    for g, w in zip(got, want):
+        assert np.max(np.abs(g - w) / np.maximum(np.max(np.abs(w), 0), 1.0)) < 8 * npart * 2.0 ** -53
+    f0 = synth.field(nslice, ngrid, 160e-6, seed=3, amplitude=2e12)
+    fld = dev.FieldState(ctx, nslice, ngrid, 160e-6, synth.LAMBDA0)
+    fld.upload(f0)
+    fld.first = nslice // 2
+    st, cen = fld.diagnostics()
+    rs, rc = orc.diag_field(f0, nslice // 2)
+    assert np.max(np.abs(st - rs) / np.max(np.abs(rs), 0)) < 8 * ngrid ** 2 * 2.0 ** -53
+    assert np.array_equal(cen, rc)
