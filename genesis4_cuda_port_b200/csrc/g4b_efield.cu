@@ -5,7 +5,7 @@
 // every slice on the host particle copies and uploads a per-particle field
 // (getEField(ip) + slice loss) that the push reads in place of the slice loss
 // (src/Core/BeamSolverCUDA.cpp:523-547, 184-195, 633-680).  Here the whole
-// step stays on the device: one CTA per slice builds the slice's azimuthal
+// step stays on the device: a cluster of CTAs per slice builds the slice's azimuthal
 // and longitudinal density modes on a radial grid, solves one tridiagonal
 // system per mode and writes every particle's field into the beam's
 // per-particle buffer, which the push then reads.
@@ -66,22 +66,82 @@ __device__ __forceinline__ double block_sum_max(double v, double* sh, bool is_ma
   return r;
 }
 
-__device__ __forceinline__ void fix_add(unsigned long long* acc, double re, double im) {
-  atomicAdd(acc, (unsigned long long)__double2ll_rn(re * kScFix));
-  atomicAdd(acc + 1, (unsigned long long)__double2ll_rn(im * kScFix));
+// Cluster helpers: rank and size of the CTA's cluster, its hardware barrier,
+// and loads of another CTA's shared memory.
+__device__ __forceinline__ uint32_t cl_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cl_size() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cl_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
+                   : "memory");
+}
+__device__ __forceinline__ uint32_t cl_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(ptx::smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ double cl_load(const double* p, uint32_t rank) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cl_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ double2 cl_load2(const double2* p, uint32_t rank) {
+  double2 v;
+  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];"
+               : "=d"(v.x), "=d"(v.y)
+               : "r"(cl_addr(p, rank))
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ longlong2 cl_load2(const longlong2* p, uint32_t rank) {
+  longlong2 v;
+  asm volatile("ld.shared::cluster.v2.s64 {%0, %1}, [%2];"
+               : "=l"(v.x), "=l"(v.y)
+               : "r"(cl_addr(p, rank))
+               : "memory");
+  return v;
 }
 
+// (c, s) = (c, s) times (a, b) as complex numbers
+__device__ __forceinline__ void turn(double& c, double& s, double a, double b) {
+  const double t = fma(c, a, -s * b);
+  s = fma(s, a, c * b);
+  c = t;
+}
+
+// A slice per cluster of C CTAs (C chosen so that the slices fill the GPU):
+// each takes 1/C of the particles and of the modes.  Bound by the FP64 work per
+// particle, done twice (radius and azimuth: a square root and two divisions; the
+// phase: one sincos for all modes), and by the chain of the radial solves (one
+// division per cell).  48 slices of 8192, nz = 2, |m| <= 1, 100 cells: 348 us
+// with one CTA per slice, a sincos per harmonic, three divisions per cell and
+// 64-bit shared atomics per particle; now 72 us, with the particles of a
+// quiet-start beamlet adding theirs together (one slice 319 -> 63 us, 150 slices
+// with one mode 160 -> 79, 250 slices with fifteen modes, one CTA each, 713 ->
+// 267).
 __global__ void __launch_bounds__(kScThreads) short_range_kernel(const ScArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double shd[kScThreads / 32];
+  __shared__ double part[3];  // this CTA's sums of x and y, largest radius squared
   const int n = a.ngrid, nmode = a.nmode, nm = 2 * a.nphi + 1;
-  unsigned long long* acc = reinterpret_cast<unsigned long long*>(smem);  // [mode][cell][2]
-  double2* u = reinterpret_cast<double2*>(acc + 2 * (size_t)nmode * n);   // [mode][cell]
+  longlong2* acc = reinterpret_cast<longlong2*>(smem);                    // [mode][cell]
+  double2* u = reinterpret_cast<double2*>(acc + (size_t)nmode * n);       // [mode][cell]
   double* cp = reinterpret_cast<double*>(u + (size_t)nmode * n);          // Thomas c'
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int s = blockIdx.x; s < a.nslice; s += gridDim.x) {
-    const int64_t p0 = a.off[s], p1 = a.off[s + 1], np = p1 - p0;
-    if (np <= 0) continue;  // uniform across the CTA
+  const int tid = threadIdx.x, nt = blockDim.x, l = tid & 31;
+  const int rank = (int)cl_rank(), C = (int)cl_size();
+  for (int s = blockIdx.x / C; s < a.nslice; s += gridDim.x / C) {
+    const int64_t q0 = a.off[s], np = a.off[s + 1] - q0;
+    if (np <= 0) continue;  // uniform across the cluster
+    // this CTA's particles, in whole groups of four
+    const int64_t share = ((np + 3) / 4 + C - 1) / C * 4;
+    const int64_t p0 = q0 + min(np, rank * share), p1 = q0 + min(np, (rank + 1) * share);
     const double eloss = a.eloss[s], cur = a.current[s];
     double sx = 0.0, sy = 0.0;
     for (int64_t p = p0 + tid; p < p1; p += nt) {
@@ -90,6 +150,16 @@ __global__ void __launch_bounds__(kScThreads) short_range_kernel(const ScArgs a)
     }
     sx = block_sum_max(sx, shd, false);
     sy = block_sum_max(sy, shd, false);
+    if (tid == 0) {
+      part[0] = sx;
+      part[1] = sy;
+    }
+    cl_sync();
+    sx = sy = 0.0;
+    for (int r = 0; r < C; ++r) {
+      sx += cl_load(&part[0], r);
+      sy += cl_load(&part[1], r);
+    }
     const double xc = sx / (double)np, yc = sy / (double)np;
     double r2 = 0.0;
     for (int64_t p = p0 + tid; p < p1; p += nt) {
@@ -97,62 +167,98 @@ __global__ void __launch_bounds__(kScThreads) short_range_kernel(const ScArgs a)
       r2 = fmax(r2, dx * dx + dy * dy);
     }
     r2 = block_sum_max(r2, shd, true);
+    if (tid == 0) part[2] = r2;
+    for (int i = tid; i < nmode * n; i += nt) acc[i] = make_longlong2(0, 0);
+    cl_sync();
+    for (int r = 0; r < C; ++r) r2 = fmax(r2, cl_load(&part[2], r));
     const double R = a.rmax * sqrt(r2);
     if (!(R > 0.0) || cur == 0.0) {
       for (int64_t p = p0 + tid; p < p1; p += nt) a.pez[p] = eloss;
+      cl_sync();  // the next slice reuses the shared arrays
       continue;
     }
     const double dr = R / (double)n;
-    for (int i = tid; i < 2 * nmode * n; i += nt) acc[i] = 0ull;
-    __syncthreads();
-    for (int64_t p = p0 + tid; p < p1; p += nt) {
+    // cell, e^{i phi} and e^{i theta} of a particle
+    auto particle = [&](int64_t p, int& j, double& cph, double& sph, double& cth, double& sth) {
       const double dx = a.x[p] - xc, dy = a.y[p] - yc;
       const double r = sqrt(dx * dx + dy * dy);
       const double q = r / dr;  // NaN or beyond the wall: the last cell
-      const int j = q >= 0.0 && q < (double)n ? (int)q : n - 1;
-      const double cph = r > 0.0 ? dx / r : 1.0, sph = r > 0.0 ? dy / r : 0.0;
-      const double th = a.theta[p];
-      for (int l = 1; l <= a.nz; ++l) {
-        double sl, cl;
-        sincos((double)l * th, &sl, &cl);
-        unsigned long long* base = acc + 2 * ((size_t)(l - 1) * nm + a.nphi) * n;
-        fix_add(base + 2 * j, cl, -sl);  // m = 0: e^{-i l theta}
+      j = q >= 0.0 && q < (double)n ? (int)q : n - 1;
+      const double ir = 1.0 / r;
+      cph = r > 0.0 ? dx * ir : 1.0;
+      sph = r > 0.0 ? dy * ir : 0.0;
+      sincos(a.theta[p], &sth, &cth);
+    };
+    for (int64_t p = p0 + tid; p - l < p1; p += nt) {  // whole warps
+      int j = -1;
+      double cph = 0, sph = 0, cth = 0, sth = 0;
+      if (p < p1) particle(p, j, cph, sph, cth, sth);
+      // four consecutive particles of one cell add their sums together
+      const int lead = __shfl_sync(0xffffffffu, j, l & ~3);
+      const unsigned match = __ballot_sync(0xffffffffu, j >= 0 && j == lead);
+      const bool same = ((match >> (l & ~3)) & 15u) == 15u;
+      auto add = [&](longlong2* cell, double re, double im) {
+        long long vr = __double2ll_rn(re * kScFix), vi = __double2ll_rn(im * kScFix);
+        // lanes 0 and 1 of a group end with the sums of re and im
+        const bool odd = (l & 1) != 0;
+        long long v = (odd ? vi : vr) + __shfl_xor_sync(0xffffffffu, odd ? vr : vi, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        unsigned long long* to = reinterpret_cast<unsigned long long*>(cell);
+        if (same) {
+          if ((l & 2) == 0) atomicAdd(to + (odd ? 1 : 0), (unsigned long long)v);
+        } else if (j >= 0) {
+          atomicAdd(to, (unsigned long long)vr);
+          atomicAdd(to + 1, (unsigned long long)vi);
+        }
+      };
+      double cl = cth, sl = sth;
+      for (int h = 1; h <= a.nz; ++h) {
+        longlong2* base = acc + ((size_t)(h - 1) * nm + a.nphi) * n + max(j, 0);
+        add(base, cl, -sl);  // m = 0: e^{-i h theta}
         double pr = cl, pi = -sl, qr = cl, qi = -sl;
         for (int m = 1; m <= a.nphi; ++m) {
-          // e^{-i(l theta + m phi)} and e^{-i(l theta - m phi)}
-          const double tr = pr * cph + pi * sph, ti = pi * cph - pr * sph;
-          const double ur = qr * cph - qi * sph, ui = qi * cph + qr * sph;
-          pr = tr;
-          pi = ti;
-          qr = ur;
-          qi = ui;
-          fix_add(base + 2 * ((size_t)m * n + j), pr, pi);
-          fix_add(base - 2 * ((size_t)m * n) + 2 * j, qr, qi);
+          // e^{-i(h theta + m phi)} and e^{-i(h theta - m phi)}
+          turn(pr, pi, cph, -sph);
+          turn(qr, qi, cph, sph);
+          add(base + (size_t)m * n, pr, pi);
+          add(base - (size_t)m * n, qr, qi);
         }
+        turn(cl, sl, cth, sth);
       }
+    }
+    cl_sync();
+    // this CTA's modes (t = rank, rank + C, ...): their sums over the cluster
+    const int mine = (nmode - rank + C - 1) / C;
+    const double rs = -kScUnfix / (6.283185307179586 * (double)np);
+    for (int i = tid; i < mine * n; i += nt) {
+      const int at = (rank + i / n * C) * n + i % n;
+      long long re = 0, im = 0;
+      for (int r = 0; r < C; ++r) {
+        const longlong2 v = cl_load2(acc + at, r);
+        re += v.x;
+        im += v.y;
+      }
+      u[at] = make_double2(rs * (double)re, rs * (double)im);
     }
     __syncthreads();
     // one tridiagonal solve per mode (Thomas, FP64), in cell units of dr
-    for (int t = tid; t < nmode; t += nt) {
-      const int l = t / nm + 1, m = t % nm - a.nphi;
-      const double kdr = (double)l * a.ks * dr;
+    for (int k = tid; k < mine; k += nt) {
+      const int t = rank + k * C, h = t / nm + 1, m = t % nm - a.nphi;
+      const double kdr = (double)h * a.ks * dr;
       const double k2 = kdr * kdr / a.gammaz2;
-      const double rs = -kScUnfix / (6.283185307179586 * (double)np);
       double2* ut = u + (size_t)t * n;
       double* ct = cp + (size_t)t * n;
-      const unsigned long long* at = acc + 2 * (size_t)t * n;
       double prev_c = 0.0, prev_dr = 0.0, prev_di = 0.0;
       for (int j = 0; j < n; ++j) {
         const double rc = (double)j + 0.5;
         const double lo = (double)j, up = (double)(j + 1);
         const double diag = -lo - (j == n - 1 ? 2.0 * up : up) -
                             ((double)(m * m) / (rc * rc) + k2) * rc;
-        const double bre = rs * (double)(long long)at[2 * j];
-        const double bim = rs * (double)(long long)at[2 * j + 1];
-        const double den = diag - lo * prev_c;
-        prev_c = j < n - 1 ? up / den : 0.0;
-        prev_dr = (bre - lo * prev_dr) / den;
-        prev_di = (bim - lo * prev_di) / den;
+        const double2 b = ut[j];
+        const double inv = 1.0 / (diag - lo * prev_c);
+        prev_c = j < n - 1 ? up * inv : 0.0;
+        prev_dr = (b.x - lo * prev_dr) * inv;
+        prev_di = (b.y - lo * prev_di) * inv;
         ct[j] = prev_c;
         ut[j] = make_double2(prev_dr, prev_di);
       }
@@ -162,41 +268,38 @@ __global__ void __launch_bounds__(kScThreads) short_range_kernel(const ScArgs a)
         ut[j].y -= ct[j] * nx.y;
       }
     }
+    cl_sync();
+    for (int i = tid; i < nmode * n; i += nt) {
+      const int owner = i / n % C;
+      if (owner != rank) u[i] = cl_load2(u + i, owner);
+    }
     __syncthreads();
     const double scale = a.coef * cur;
     for (int64_t p = p0 + tid; p < p1; p += nt) {
-      const double dx = a.x[p] - xc, dy = a.y[p] - yc;
-      const double r = sqrt(dx * dx + dy * dy);
-      const double q = r / dr;  // NaN or beyond the wall: the last cell
-      const int j = q >= 0.0 && q < (double)n ? (int)q : n - 1;
-      const double cph = r > 0.0 ? dx / r : 1.0, sph = r > 0.0 ? dy / r : 0.0;
-      const double th = a.theta[p];
-      double sum = 0.0;
-      for (int l = 1; l <= a.nz; ++l) {
-        double sl, cl;
-        sincos((double)l * th, &sl, &cl);
-        const double2* base = u + ((size_t)(l - 1) * nm + a.nphi) * n;
-        // Im[u_lm e^{i(l theta + m phi)}]
-        double2 c = base[j];
+      int j;
+      double cph, sph, cth, sth;
+      particle(p, j, cph, sph, cth, sth);
+      double sum = 0.0, cl = cth, sl = sth;
+      for (int h = 1; h <= a.nz; ++h) {
+        const double2* base = u + ((size_t)(h - 1) * nm + a.nphi) * n + j;
+        // Im[u_hm e^{i(h theta + m phi)}]
+        double2 c = base[0];
         double im = c.x * sl + c.y * cl;
         double pr = cl, pi = sl, qr = cl, qi = sl;
         for (int m = 1; m <= a.nphi; ++m) {
-          const double tr = pr * cph - pi * sph, ti = pi * cph + pr * sph;
-          const double ur = qr * cph + qi * sph, ui = qi * cph - qr * sph;
-          pr = tr;
-          pi = ti;
-          qr = ur;
-          qi = ui;
-          c = base[(size_t)m * n + j];
+          turn(pr, pi, cph, sph);
+          turn(qr, qi, cph, -sph);
+          c = base[(size_t)m * n];
           im += c.x * pi + c.y * pr;
-          c = base[j - (ptrdiff_t)m * n];
+          c = *(base - (size_t)m * n);
           im += c.x * qi + c.y * qr;
         }
-        sum += (double)l * im;
+        sum += (double)h * im;
+        turn(cl, sl, cth, sth);
       }
       a.pez[p] = eloss + scale * sum;
     }
-    __syncthreads();  // the next slice reuses the shared arrays
+    cl_sync();  // the next slice reuses the shared arrays
   }
 }
 
@@ -293,10 +396,15 @@ int g4b_efield_short_range(g4b_efield* e, g4b_beam* b, double gammaz2) {
   G4B_CUDA_TRY(cudaFuncSetAttribute(short_range_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)e->smem));
-  const unsigned grid = (unsigned)std::max(1, std::min(b->nslice, c->sm_count * 8));
+  // the largest cluster with which the slices still fit three CTAs per SM, of at
+  // least 512 particles each
+  int C = 8;
+  while (C > 1 && ((int64_t)b->nslice * C > 3 * c->sm_count || b->max_slice_np < 512 * C)) C >>= 1;
+  const unsigned grid = (unsigned)(C * std::max(1, std::min(b->nslice, c->sm_count * 8)));
   {
     LaunchScope ls(c, "short_range");
-    short_range_kernel<<<grid, kScThreads, e->smem, c->stream>>>(a);
+    G4B_CUDA_TRY(launch_cluster(short_range_kernel, grid, kScThreads, (unsigned)C, e->smem,
+                                c->stream, a));
   }
   return check_launch(c, "short_range_kernel");
 }

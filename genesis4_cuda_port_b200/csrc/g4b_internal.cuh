@@ -207,6 +207,24 @@ inline cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned block,
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<A&&>(args)...);
 }
+// Launches kern in clusters of `cluster` CTAs.
+template <typename... P, typename... A>
+inline cudaError_t launch_cluster(void (*kern)(P...), unsigned grid, unsigned block,
+                                  unsigned cluster, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<A&&>(args)...);
+}
 #endif
 
 struct AdiPassArgs {

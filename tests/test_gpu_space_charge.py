@@ -67,6 +67,28 @@ def test_short_range_matches_the_oracle(ctx, nz, nphi, ngrid, rmax):
         o.close()
 
 
+# clusters of 8, 4, 2 and 1 CTAs per slice (at least 512 particles each, three
+# CTAs per SM), shares off the groups of four, fewer modes than CTAs
+@pytest.mark.parametrize("nslice,npart,nz,nphi", [(1, 4099, 2, 1), (1, 4095, 1, 0), (1, 515, 1, 1),
+                                                  (1, 3, 1, 0), (60, 2050, 1, 1), (120, 1030, 1, 0),
+                                                  (450, 21, 1, 1)])
+def test_short_range_split_over_clusters(ctx, nslice, npart, nz, nphi):
+    off, p = _bunched(nslice, npart, seed=nslice + npart)
+    cur = np.linspace(2500.0, 800.0, nslice)
+    beam = dev.BeamState(ctx, off, synth.GAMMA0)
+    beam.upload(p)
+    beam.set_current(cur)
+    sc = dev.EFieldSolver(ctx, 2.3, 30, nz, nphi, synth.LAMBDA0)
+    sc.short_range(beam, GZ2)
+    got = beam.particle_ez()
+    want = orc.short_range(off, p, cur, GZ2, rmax=2.3, ngrid=30, nz=nz, nphi=nphi,
+                           lambda0=synth.LAMBDA0)
+    # the same fixed-point mode sums (quantum 2^-40 of a sum of npart terms)
+    assert np.max(np.abs(got - want)) < 1e-9 * np.max(np.abs(want))
+    for o in (sc, beam):
+        o.close()
+
+
 def test_short_range_off_and_limits(ctx):
     off, p = _bunched(2, 500, seed=3)
     beam = dev.BeamState(ctx, off, synth.GAMMA0)
