@@ -327,7 +327,7 @@ def kernel_alg_bytes(wl, mixed: bool):
                 "adi_pass_x": 16 * C, "adi_pass_y": 16 * C, "run_diag_finalize": 0}
     return {"track": 72 * N, "push": 64 * N, "r56": 24 * N, "deposit": 32 * N,
             "adi_pass_x": 32 * C, "adi_pass_y": 32 * C, "diag_beam": 48 * N,
-            "diag_field": 16 * C, "slice_scl": 24 * wl.nslice}
+            "diag_field": 16 * C}
 
 
 class MixedRun:

@@ -471,7 +471,8 @@ __global__ void __launch_bounds__(BandW<T, L>::value * 32, AdiBlocks<T, M, L>::v
 struct DepositArgs {
   const double *x, *y, *gamma, *theta;
   const int64_t* off;
-  const double* scl;
+  const double* current;
+  double fc, xks, delz, vacimp, eev;
   double2* src;        // compact tiles, src_cap cells per slice
   int4* desc;          // per target slice
   size_t src_cap;
@@ -506,38 +507,42 @@ __device__ __forceinline__ double dep_faw2(const DepositArgs& a, double xp, doub
   return 1.0 + a.kx * dx * dx + a.ky * dy * dy + 2.0 * (a.gradx * dx + a.grady * dy);
 }
 
-template <typename V>
-__device__ __forceinline__ V block_reduce(V v, V* sh, bool is_max) {
-  // fixed-order reduction: warp xor-tree, then warp 0 over the warp partials
-  for (int o = 16; o > 0; o >>= 1) {
-    V t = __shfl_xor_sync(0xffffffffu, v, o);
-    v = is_max ? (t > v ? t : v) : (t < v ? t : v);
+// What the first pass keeps of the particles in the grid: the largest faw2, the
+// smallest |gamma|, the box of their base cells and their number.
+struct DepBox {
+  double fmx = 0.0, gmn = INFINITY;
+  int ixmin = 1 << 30, iymin = 1 << 30, ixmax = -1, iymax = -1, cnt = 0;
+  __device__ __forceinline__ void warp_reduce() {
+    for (int o = 16; o > 0; o >>= 1) {
+      const double f = __shfl_xor_sync(0xffffffffu, fmx, o), g = __shfl_xor_sync(0xffffffffu, gmn, o);
+      fmx = f > fmx ? f : fmx;
+      gmn = g < gmn ? g : gmn;
+    }
+    ixmin = __reduce_min_sync(0xffffffffu, ixmin);
+    iymin = __reduce_min_sync(0xffffffffu, iymin);
+    ixmax = __reduce_max_sync(0xffffffffu, ixmax);
+    iymax = __reduce_max_sync(0xffffffffu, iymax);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
   }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  const int nw = blockDim.x >> 5;
-  V r = sh[0];
-  for (int i = 1; i < nw; ++i) r = is_max ? (sh[i] > r ? sh[i] : r) : (sh[i] < r ? sh[i] : r);
-  return r;
-}
+};
 
 constexpr int kDepFp64U = 2;  // particles in flight per thread (the first pass)
 // One CTA of 1024 threads per SM with a band of 12800 cells: tiles of 80-110
 // cells a side are one band, so a particle's cell, weight and phase are worked
 // out once (two 512-thread CTAs with bands of 6144 cells: twice the cells and
 // the first pass's divisions; us per launch with 256 slices of 8192 at 201^2:
-// 89 -> 64, 64 slices of 4096 at 255^2 43 -> 27, 40 slices of 4096 at 401^2 72 ->
-// 46, 1 slice of 8192 42 -> 31).  Bound by the FP64 chain of a particle: sincos,
-// square root, division.
+// 94 -> 66, 64 slices of 4096 at 255^2 48 -> 30, 40 slices of 4096 at 401^2 80 ->
+// 48, 1 slice of 8192 at 151^2 37 -> 29, 8 of 2048 at 101^2 17 -> 15).  Bound by
+// the FP64 chain of a particle: sincos, square root, division.  A few slices as
+// clusters of CTAs, their tiles added through distributed shared memory, gain a
+// tenth at 4 slices and lose as much at 16 and with small slices.
 constexpr int kDepFp64Threads = 1024;
 constexpr size_t kDepFp64Acc = 200 * 1024;  // accumulators: 12800 cells, one band in most runs
 
 __global__ void __launch_bounds__(kDepFp64Threads, 1) deposit_slice_kernel(const DepositArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ double shd[32];
-  __shared__ int shi[32];
+  __shared__ double shd[2][32];
+  __shared__ int shi[5][32];
   ptx::pdl_wait();
   unsigned long long* acc = reinterpret_cast<unsigned long long*>(smem);
   const int bs = blockIdx.x;
@@ -545,12 +550,16 @@ __global__ void __launch_bounds__(kDepFp64Threads, 1) deposit_slice_kernel(const
   const int target = (bs + a.first) % a.nslice;
   double2* S = a.src + (size_t)target * a.src_cap;
   const int64_t p0 = a.off[bs], p1 = a.off[bs + 1];
-  const double scl = a.scl[bs];
+  // adi_compute_slice_scl (src/Core/FieldSolverADICUDA.cpp:75-96); a kernel of
+  // its own was 2 us of a step's launches
+  double scl = 0.0;
+  if (p1 > p0) {
+    scl = a.fc * a.vacimp * a.current[bs] * a.xks * a.delz;
+    scl /= 4.0 * a.eev * (double)(p1 - p0) * a.dgrid * a.dgrid;
+  }
 
-  // largest faw2 and smallest |gamma| of the particles in the grid: their
-  // weights are at most sqrt(fmx) / gmn
-  double fmx = 0.0, gmn = INFINITY;
-  int ixmin = 1 << 30, iymin = 1 << 30, ixmax = -1, iymax = -1, cnt = 0;
+  // largest faw2 and smallest |gamma|: the weights are at most sqrt(fmx) / gmn
+  DepBox m;
   const int nt = blockDim.x;
   if (scl != 0.0) {
     // kDepFp64U particles in flight per thread: their loads are issued
@@ -573,44 +582,57 @@ __global__ void __launch_bounds__(kDepFp64Threads, 1) deposit_slice_kernel(const
         double wx, wy;
         if (!dep_cell(a, lx[u], ly[u], ix, iy, wx, wy)) continue;
         const double f = dep_faw2(a, lx[u], ly[u]), g = fabs(lg[u]);
-        fmx = f > fmx ? f : fmx;
-        gmn = g < gmn ? g : gmn;
-        if (!(f >= 0.0 && f < 1e300 && g > 1e-290)) fmx = INFINITY;  // no finite weight
-        ixmin = min(ixmin, ix);
-        ixmax = max(ixmax, ix);
-        iymin = min(iymin, iy);
-        iymax = max(iymax, iy);
-        ++cnt;
+        m.fmx = f > m.fmx ? f : m.fmx;
+        m.gmn = g < m.gmn ? g : m.gmn;
+        if (!(f >= 0.0 && f < 1e300 && g > 1e-290)) m.fmx = INFINITY;  // no finite weight
+        m.ixmin = min(m.ixmin, ix);
+        m.ixmax = max(m.ixmax, ix);
+        m.iymin = min(m.iymin, iy);
+        m.iymax = max(m.iymax, iy);
+        ++m.cnt;
       }
     }
   }
-  fmx = block_reduce<double>(fmx, shd, true);
-  gmn = block_reduce<double>(gmn, shd, false);
-  const double qmax = fmx < INFINITY ? sqrt(fmx) / gmn : INFINITY;
-  ixmin = block_reduce<int>(ixmin, shi, false);
-  ixmax = block_reduce<int>(ixmax, shi, true);
-  iymin = block_reduce<int>(iymin, shi, false);
-  iymax = block_reduce<int>(iymax, shi, true);
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+  // one exchange through shared memory, then the same tree in every warp (seven
+  // block reductions, each a serial loop over 32 warps: 6 us more of a launch)
+  const int w = tid >> 5, l = tid & 31;
+  m.warp_reduce();
+  if (l == 0) {
+    shd[0][w] = m.fmx;
+    shd[1][w] = m.gmn;
+    shi[0][w] = m.ixmin;
+    shi[1][w] = m.iymin;
+    shi[2][w] = m.ixmax;
+    shi[3][w] = m.iymax;
+    shi[4][w] = m.cnt;
+  }
   __syncthreads();
-  if ((tid & 31) == 0) shi[tid >> 5] = cnt;
-  __syncthreads();
-  int total = 0;
-  for (int i = 0; i < (int)(blockDim.x >> 5); ++i) total += shi[i];
-  __syncthreads();
+  if (l < (nt >> 5)) {
+    m.fmx = shd[0][l];
+    m.gmn = shd[1][l];
+    m.ixmin = shi[0][l];
+    m.iymin = shi[1][l];
+    m.ixmax = shi[2][l];
+    m.iymax = shi[3][l];
+    m.cnt = shi[4][l];
+  } else {
+    m.cnt = 0;  // lane 0's values are copies of this warp's: they add no extreme
+  }
+  m.warp_reduce();
+  const double qmax = m.fmx < INFINITY ? sqrt(m.fmx) / m.gmn : INFINITY;
 
-  const bool any = total > 0 && qmax > 0.0;
+  const bool any = m.cnt > 0 && qmax > 0.0;
   if (any && !(qmax < INFINITY) && tid == 0) atomicOr(a.err, kErrFixedRange);
   const bool ok = any && qmax < INFINITY;
   int bx0 = 0, by0 = 0, bw = 0, bh = 0;
   double scale = 0.0, unscale = 0.0;
   if (ok) {
-    bx0 = ixmin;
-    by0 = iymin;
-    bw = ixmax - ixmin + 2;  // corners ix..ix+1
-    bh = iymax - iymin + 2;
+    bx0 = m.ixmin;
+    by0 = m.iymin;
+    bw = m.ixmax - m.ixmin + 2;  // corners ix..ix+1
+    bh = m.iymax - m.iymin + 2;
     int e;
-    frexp(qmax * (double)total, &e);  // qmax*total < 2^e
+    frexp(qmax * (double)m.cnt, &e);  // qmax*m.cnt < 2^e
     scale = ldexp(1.0, 62 - e);
     unscale = scl * ldexp(1.0, e - 62);
   }
@@ -643,7 +665,6 @@ __global__ void __launch_bounds__(kDepFp64Threads, 1) deposit_slice_kernel(const
     // particles of one base cell (a quiet-start beamlet: nbins = 4 particles at
     // one transverse position) are summed over their lanes, each of which adds
     // one corner (the same integer sums by a quarter of the atomics).
-    const int l = tid & 31;
     const int64_t np = p1 - p0;
     double nx = 0, ny = 0, ng = 1, nt_ = 0;
     auto load = [&](int64_t p) {
@@ -709,22 +730,6 @@ __global__ void __launch_bounds__(kDepFp64Threads, 1) deposit_slice_kernel(const
     }
     __syncthreads();
   }
-}
-
-// adi_compute_slice_scl (src/Core/FieldSolverADICUDA.cpp:75-96)
-__global__ void slice_scl_kernel(int nslice, const int64_t* off, const double* current,
-                                 double fc, double xks, double dgrid, double delz,
-                                 double vacimp, double eev, double* scl) {
-  ptx::pdl_wait();
-  const int is = blockIdx.x * blockDim.x + threadIdx.x;
-  if (is >= nslice) return;
-  double s = 0.0;
-  const int64_t npar = off[is + 1] - off[is];
-  if (npar > 0) {
-    s = fc * vacimp * current[is] * xks * delz;
-    s /= 4.0 * eev * (double)npar * dgrid * dgrid;
-  }
-  scl[is] = s;
 }
 
 // ------------------------------------------------------------- host side ---
@@ -930,20 +935,18 @@ int adi_batch_launch(g4b_ctx* c, cudaStream_t st, int mode, bool px, const AdiBa
 int fp64_deposit(g4b_field* f, g4b_beam* b, const g4b_step* st, double fc) {
   g4b_ctx* c = f->ctx;
   const int harm = f->harm;
-  {
-    LaunchScope ls(c, "slice_scl");
-    G4B_CUDA_TRY(launch_pdl(slice_scl_kernel, (unsigned)((b->nslice + 127) / 128), 128, 0,
-                            c->stream, b->nslice, b->d_off, b->d_current, fc, f->xks, f->dgrid,
-                            st->delz, kVacimp, kEev, b->d_scl));
-  }
-  if (int rc = check_launch(c, "slice_scl_kernel")) return rc;
   DepositArgs da{};
   da.x = b->x;
   da.y = b->y;
   da.gamma = b->gamma;
   da.theta = b->theta;
   da.off = b->d_off;
-  da.scl = b->d_scl;
+  da.current = b->d_current;
+  da.fc = fc;
+  da.xks = f->xks;
+  da.delz = st->delz;
+  da.vacimp = kVacimp;
+  da.eev = kEev;
   da.src = static_cast<double2*>(f->src);
   da.desc = f->desc;
   da.src_cap = (size_t)f->ngrid * f->ld;

@@ -658,7 +658,6 @@ int g4b_beam_create(g4b_ctx* c, int nslice, const int64_t* off, int precision,
   if (e == cudaSuccess) e = dev_alloc(c, (void**)&b->d_off, (nslice + 1) * sizeof(int64_t));
   if (e == cudaSuccess) e = dev_alloc(c, (void**)&b->d_current, nslice * sizeof(double));
   if (e == cudaSuccess) e = dev_alloc(c, (void**)&b->d_eloss, nslice * sizeof(double));
-  if (e == cudaSuccess) e = dev_alloc(c, (void**)&b->d_scl, nslice * sizeof(double));
   if (e == cudaSuccess)
     e = dev_alloc(c, (void**)&b->d_chunks, std::max(1, b->nchunk) * sizeof(int4));
   if (e == cudaSuccess)
@@ -674,7 +673,7 @@ int g4b_beam_create(g4b_ctx* c, int nslice, const int64_t* off, int precision,
     g4b_beam_destroy(b);
     return cuda_fail(e, "g4b_beam_create: device allocation");
   }
-  b->bytes = np * 6 * sizeof(double) + (nslice + 1) * 8 + 3 * nslice * 8 +
+  b->bytes = np * 6 * sizeof(double) + (nslice + 1) * 8 + 2 * nslice * 8 +
              chunks.size() * sizeof(int4);
   *out = b;
   return G4B_OK;
@@ -684,7 +683,7 @@ int g4b_beam_destroy(g4b_beam* b) {
   if (!b) return G4B_OK;
   ctx_quiesce(b->ctx);
   void* ptrs[] = {b->x, b->y, b->px, b->py, b->gamma, b->theta, b->d_off,
-                  b->d_current, b->d_eloss, b->d_scl, b->d_chunks, b->d_pez};
+                  b->d_current, b->d_eloss, b->d_chunks, b->d_pez};
   for (void* p : ptrs) dev_free(b->ctx, p);
   ctx_release(b->ctx);
   delete b;

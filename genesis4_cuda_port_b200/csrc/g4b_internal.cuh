@@ -108,7 +108,6 @@ struct g4b_beam {
   double *gamma = nullptr, *theta = nullptr;
   double* d_current = nullptr;
   double* d_eloss = nullptr;
-  double* d_scl = nullptr;           // per-slice source scale
   // per-particle loss (space charge + slice loss); the push reads it in
   // place of d_eloss while use_pez is set
   double* d_pez = nullptr;
