@@ -2386,9 +2386,9 @@ struct g4b_batch {
   // concurrent branches of a step: the beam diagnostics beside the
   // deposition and ADI passes; the ADI kernels of different row layouts
   // beside one another
-  static constexpr int kAux = 4;
+  static constexpr int kAux = 12;
   cudaStream_t aux[kAux] = {};
-  cudaEvent_t ev_fork[2] = {}, ev_diag = nullptr, ev_adi[kNumM] = {};
+  cudaEvent_t ev_fork[2] = {}, ev_diag = nullptr, ev_adi[kAux] = {};
   // graph of one step for the current composition and shapes
   cudaGraphExec_t gexec = nullptr;
   bool graph_valid = false;
@@ -2627,37 +2627,43 @@ int batch_launch(g4b_batch* b, bool timed) {
     return rc;
   }
   ev(2);
-  for (int pass = 0; pass < 2; ++pass) {
-    int ngroups = 0;
-    for (int m = 0; m < kNumM; ++m) ngroups += b->counts.adi[m] > 0;
-    const bool par = fork && ngroups > 1;
-    if (par) G4B_CUDA_TRY(cudaEventRecord(b->ev_fork[1], c->stream));
-    int gi = 0;
-    for (int m = 0; m < kNumM; ++m) {
-      if (b->counts.adi[m] == 0) continue;
-      AdiBatchArgs a;
-      a.args = reinterpret_cast<const AdiPassArgs*>(b->d_args + (pass ? b->off_ay : b->off_ax));
-      a.maps = reinterpret_cast<const CUtensorMap*>(b->d_args + (pass ? b->off_my : b->off_mx));
-      a.items = reinterpret_cast<const int4*>(b->d_items + b->off_adi[m]);
-      a.nitems = reinterpret_cast<const int*>(b->d_args) + 4 + m;
-      const int g = std::min(b->grid[2], b->counts.adi[m]);
-      // groups round-robin over the main stream and the branch streams
-      // 1..kAux-1 (stream 0 of the branches carries the diagnostics)
-      cudaStream_t st = c->stream;
-      if (par && gi % g4b_batch::kAux != 0) {
-        st = b->aux[gi % g4b_batch::kAux];
-        G4B_CUDA_TRY(cudaStreamWaitEvent(st, b->ev_fork[1], 0));
-      }
-      if (int rc = adi_batch_launch(c, st, kMList[m], pass == 0, a,
-                                    pass ? b->smem_y[m] : b->smem_x[m], g))
-        return rc;
-      if (st != c->stream) G4B_CUDA_TRY(cudaEventRecord(b->ev_adi[gi], st));
-      ++gi;
+  auto adi = [&](cudaStream_t st, int m, int pass) {
+    AdiBatchArgs a;
+    a.args = reinterpret_cast<const AdiPassArgs*>(b->d_args + (pass ? b->off_ay : b->off_ax));
+    a.maps = reinterpret_cast<const CUtensorMap*>(b->d_args + (pass ? b->off_my : b->off_mx));
+    a.items = reinterpret_cast<const int4*>(b->d_items + b->off_adi[m]);
+    a.nitems = reinterpret_cast<const int*>(b->d_args) + 4 + m;
+    return adi_batch_launch(c, st, kMList[m], pass == 0, a, pass ? b->smem_y[m] : b->smem_x[m],
+                            std::min(b->grid[2], b->counts.adi[m]));
+  };
+  int groups[kNumM], ngroups = 0;
+  for (int m = 0; m < kNumM; ++m)
+    if (b->counts.adi[m] > 0) groups[ngroups++] = m;
+  if (fork && ngroups > 1) {
+    // A group's pass Y waits for its own pass X alone: chains, round-robin over
+    // the main stream and the branch streams 1..kAux-1 (stream 0 of the
+    // branches carries the diagnostics).  A group of a few slices is bound by
+    // its rows' latency, so chains gain by running at once: us per step of 32
+    // runs of 9 row layouts, pass by pass over 4 streams 128, chains over 4
+    // streams 124, over 6 122, a stream each 117.
+    G4B_CUDA_TRY(cudaEventRecord(b->ev_fork[1], c->stream));
+    for (int gi = 0; gi < ngroups; ++gi) {
+      const int k = gi % g4b_batch::kAux;
+      cudaStream_t st = k ? b->aux[k] : c->stream;
+      if (k && gi == k) G4B_CUDA_TRY(cudaStreamWaitEvent(st, b->ev_fork[1], 0));
+      for (int pass = 0; pass < 2; ++pass)
+        if (int rc = adi(st, groups[gi], pass)) return rc;
     }
-    if (par)
-      for (int k = 0; k < gi; ++k)
-        if (k % g4b_batch::kAux != 0) G4B_CUDA_TRY(cudaStreamWaitEvent(c->stream, b->ev_adi[k], 0));
-    ev(3 + pass);
+    for (int k = 1; k < std::min(ngroups, g4b_batch::kAux); ++k) {
+      G4B_CUDA_TRY(cudaEventRecord(b->ev_adi[k], b->aux[k]));
+      G4B_CUDA_TRY(cudaStreamWaitEvent(c->stream, b->ev_adi[k], 0));
+    }
+  } else {
+    for (int pass = 0; pass < 2; ++pass) {
+      for (int gi = 0; gi < ngroups; ++gi)
+        if (int rc = adi(c->stream, groups[gi], pass)) return rc;
+      ev(3 + pass);
+    }
   }
   if (fork && sp.parts == 0) G4B_CUDA_TRY(cudaStreamWaitEvent(c->stream, b->ev_diag, 0));
   {

@@ -200,6 +200,35 @@ def test_both_row_layouts_solve_the_same_system(ctx):
     b.close()
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_more_row_layouts_than_concurrent_branches(ctx, graph):
+    """Sixteen row layouts in a batch: some branches carry two chains of an ADI
+    pass X and its pass Y."""
+    lanes16 = [100 + m for m in (5, 7, 9, 11, 13, 15, 17, 21)]
+    lanes32 = [3, 5, 7, 9, 11, 13, 15, 17]
+    cfgs, want = [], []
+    for n in (75, 101, 130, 170, 201, 240, 260, 330):
+        cfgs += 2 * [dict(nslice=1, npart=512, ngrid=n, taper=0.0, dgam=0.0, time_run=False,
+                          nsteps=4)]
+        want += [next(m for m in lanes16 if 16 * (m - 100) >= n),
+                 next(m for m in lanes32 if 32 * m >= n)]
+    assert len(set(want)) > 12
+    runs = [_make(ctx, k, cfg) for k, cfg in enumerate(cfgs)]
+    batch = dev.Batch(ctx, len(runs))
+    for r, m in zip(runs, want):
+        r.set_layouts([m])
+        batch.attach(r, 0, 4)
+    batch.step(4, graph=graph)
+    ctx.synchronize()
+    for k, (r, cfg, m) in enumerate(zip(runs, cfgs, want)):
+        alone = _make(ctx, k, cfg)
+        alone.set_layouts([m])
+        alone.advance(0, 4, graph=False)
+        _same(_result(r, 4), _result(alone, 4))
+        alone.close()
+    batch.close()
+
+
 # the deposition and the beam diagnostics of a slice are split by the number of
 # slices in the launch (dep_split: shared tile up to 21 slices, two CTAs of 512
 # or 256 threads per slice up to 147, one CTA above); widths 1 and 6 make tiles
