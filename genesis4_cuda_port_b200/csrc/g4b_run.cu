@@ -1370,6 +1370,21 @@ static DepSplit dep_split(int nslice, int sm_count) {
   return parts >= 7 ? DepSplit{parts, 512} : DepSplit{2, 2 * nslice <= sm_count ? 512 : 256};
 }
 
+// The same for the slices of a batch, whose particle counts differ: a large slice
+// in a narrow CTA is the whole launch's length, so pairs of 512 threads up to four
+// slices per SM, the hardware dealing them out as SMs come free; beyond, the
+// persistent kernels (32 warps per SM) win on slices of one size.  Measured, us
+// per step (pairs of 256 threads to 147 slices and persistent kernels above):
+//   steady-state runs of 2048-32768 particles: 100 of them 222 (322), 140 259
+//   (343), 148 279 (412), 256 436 (515), 500 753 (838);
+//   runs of 100 slices of 8192: two 209 (253), four 370 (425); four runs of 200
+//   slices of 4096 463 (448).
+static DepSplit dep_split_batch(int nslice, int sm_count) {
+  const DepSplit s = dep_split(nslice, sm_count);
+  if (s.T == 512) return s;
+  return nslice <= 4 * sm_count ? DepSplit{2, 512} : DepSplit{0, 0};
+}
+
 // fn(integral constant NB, integral constant T) of a split launch
 template <typename Fn>
 static void dep_dispatch(bool one, int T, Fn fn) {
@@ -2588,8 +2603,8 @@ int batch_launch(g4b_batch* b, bool timed) {
   }
   if (int rc = check_launch(c, "beam_batch_kernel")) return rc;
   ev(1);
-  // few slices in all: several CTAs per slice, the diagnostics beside them
-  const DepSplit sp = dep_split(b->counts.dep, c->sm_count);
+  // several CTAs per slice, the diagnostics beside them, up to four slices per SM
+  const DepSplit sp = dep_split_batch(b->counts.dep, c->sm_count);
   {
     DepBatchArgs a{reinterpret_cast<const DepArgs*>(b->d_args + b->off_dd),
                    reinterpret_cast<const int2*>(b->d_items + b->off_dep), counts + 1};

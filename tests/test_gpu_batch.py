@@ -230,11 +230,11 @@ def test_more_row_layouts_than_concurrent_branches(ctx, graph):
 
 
 # the deposition and the beam diagnostics of a slice are split by the number of
-# slices in the launch (dep_split: shared tile up to 21 slices, two CTAs of 512
-# or 256 threads per slice up to 147, one CTA above); widths 1 and 6 make tiles
+# slices in the launch (dep_split, dep_split_batch: shared tile up to 21 slices,
+# two CTAs per slice up to 147 in a run and 592 in a batch, one CTA above); widths 1 and 6 make tiles
 # of one band and of several, the slices start at odd offsets
 @pytest.mark.parametrize("width", [1.0, 6.0])
-@pytest.mark.parametrize("fill", [18, 19, 71, 72, 144, 145])
+@pytest.mark.parametrize("fill", [18, 19, 71, 72, 144, 145, 589, 590])
 def test_results_do_not_depend_on_how_the_slices_are_split(ctx, width, fill):
     ns, ngrid, gm, n = 3, 151, 160e-6, 5
     off, parts = synth.beam(ns, 1500, seed=11, ragged=True)
