@@ -2380,6 +2380,7 @@ struct g4b_batch {
   // work lists
   std::vector<int2> beam_items, dep_items;
   std::vector<int4> adi_items[kNumM];
+  std::vector<int> modes;       // ADI row layout each [slot][field] is listed under
   size_t items_cap = 0, h_items_cap[2] = {0, 0};
   unsigned char* d_items = nullptr;
   unsigned char* h_items[2] = {nullptr, nullptr};  // pinned, alternating
@@ -2474,6 +2475,7 @@ int batch_rebuild(g4b_batch* b) {
     for (int f = 0; f < r->nfield; ++f) {
       g4b_field* F = r->fs[f].f;
       const int mi = m_index(F->mode);
+      b->modes[s * kRunFields + f] = F->mode;
       if (mi < 0) return fail(G4B_ERR_RANGE, "g4b_batch: unsupported grid");
       const int nband = (F->ngrid + F->band_rows - 1) / F->band_rows;
       for (int sl = 0; sl < r->nslice; ++sl)
@@ -2537,6 +2539,19 @@ int batch_rebuild(g4b_batch* b) {
   b->dirty = false;
   b->graph_valid = false;
   return G4B_OK;
+}
+
+// Has g4b_run_set_layouts switched a listed run's row layout since the last
+// rebuild?  Its bands are then listed under another kernel than the one that
+// its tables, which batch_stage takes from the layout in force, belong to.
+bool batch_layouts_changed(const g4b_batch* b) {
+  for (int s = 0; s < b->max_runs; ++s) {
+    const g4b_run* r = b->runs[s];
+    if (!r || b->next[s] >= b->last[s]) continue;
+    for (int f = 0; f < r->nfield; ++f)
+      if (r->fs[f].f->mode != b->modes[s * kRunFields + f]) return true;
+  }
+  return false;
 }
 
 // Resolve this step's arguments of every active run into the staging buffer.
@@ -2713,6 +2728,7 @@ int g4b_batch_create(g4b_ctx* c, int max_runs, g4b_batch** out) {
   b->runs.assign(max_runs, nullptr);
   b->next.assign(max_runs, 0);
   b->last.assign(max_runs, 0);
+  b->modes.assign((size_t)max_runs * kRunFields, 0);
   batch_default_grids(b);
   cudaFuncSetAttribute(deposit_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)dep_smem(kDepCells2));
@@ -2931,7 +2947,7 @@ int g4b_batch_step(g4b_batch* b, int nsteps, int use_graph) {
   g4b_ctx* c = b->ctx;
   G4B_CUDA_TRY(cudaSetDevice(c->device));
   for (int k = 0; k < nsteps; ++k) {
-    if (b->dirty)
+    if (b->dirty || batch_layouts_changed(b))
       if (int rc = batch_rebuild(b)) return rc;
     if (b->counts.fin == 0) return G4B_OK;
     if (int rc = batch_stage(b)) return rc;

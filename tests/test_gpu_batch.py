@@ -273,3 +273,30 @@ def test_results_do_not_depend_on_how_the_slices_are_split(ctx, width, fill):
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
     for o in (batch, run, filler, alone):
         o.close()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_layout_switched_after_attaching_takes_effect(ctx, graph):
+    """set_layouts on a run that a batch already steps (from a captured graph
+    too): the later steps equal those of an alone run switched at that step."""
+    cfgs = [dict(nslice=2, npart=512, ngrid=n, taper=0.0, dgam=0.0, time_run=False, nsteps=9)
+            for n in (101, 151, 201, 240)]
+    other = [5, 111, 7, 9]  # by default 16 x 7, 32 x 5, 16 x 13, 16 x 15
+    runs = [_make(ctx, k, cfg) for k, cfg in enumerate(cfgs)]
+    batch = dev.Batch(ctx, len(runs))
+    for r in runs:
+        batch.attach(r, 0, 9)
+    batch.step(5, graph=graph)
+    for r, m in zip(runs, other):
+        assert r.layouts() != [m]
+        r.set_layouts([m])
+    batch.step(4, graph=graph)
+    ctx.synchronize()
+    for k, (r, cfg, m) in enumerate(zip(runs, cfgs, other)):
+        alone = _make(ctx, k, cfg)
+        alone.advance(0, 5, graph=False)
+        alone.set_layouts([m])
+        alone.advance(5, 4, graph=False)
+        _same(_result(r, 9), _result(alone, 9))
+        alone.close()
+    batch.close()
