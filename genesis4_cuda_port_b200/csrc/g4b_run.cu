@@ -1181,9 +1181,8 @@ __device__ __forceinline__ void deposit_slice(const DepArgs& a, const int bs, un
 // Part `rank` of C of a slice: the particles [rank, rank + 1) / C into the
 // slice's DepTile; the CTA whose count comes last reads it, writes the source
 // and leaves the tile zero for the next launch.  A field without a prediction,
-// one whose prediction fails and one larger than its tile are done by that CTA
-// in shared memory.
-
+// one whose prediction fails, one without a finite charge and one larger than
+// its tile are done by that CTA in shared memory.
 template <int T>
 __device__ __forceinline__ void deposit_part(const DepArgs& a, const int bs, const int rank,
                                              const int C, unsigned char* smem) {
@@ -1243,7 +1242,8 @@ __device__ __forceinline__ void deposit_part(const DepArgs& a, const int bs, con
       *t.qmax = 0;
       *t.done = 0;
     }
-    if (M > d.m_use || !(qm <= d.q_use)) {
+    // also without a finite positive charge, which that form reports
+    if (M > d.m_use || !(qm > 0.f && qm <= d.q_use)) {
       deposit_field<T, false, kDepCells1>(a, F, d, smem);
     } else if (tid == 0) {
       F.mpred[bs] = M;

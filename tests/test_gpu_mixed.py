@@ -11,6 +11,7 @@ import pytest
 
 from genesis4_cuda_port_b200 import device as dev
 from genesis4_cuda_port_b200 import workloads
+from genesis4_cuda_port_b200._lib import G4BError
 from oracle import pyoracle as orc
 from tests import synth
 
@@ -296,3 +297,39 @@ def test_steady_state_pz_and_bunching_gates(ctx):
     rel = np.max(np.abs(pzm - pz_ref) / pz_ref)
     assert rel < P_TOL, rel
     assert np.max(np.abs(bzm - bz_ref)) < B_TOL
+
+
+@pytest.mark.parametrize("nslice", [2, 30, 160])
+def test_charges_that_are_not_finite_are_reported_and_deposit_nothing(nslice):
+    """A step whose undulator gradient makes 1 + 2 gradx dx negative for every
+    particle has no finite charge weight: in every split of the deposition the
+    step that meets it raises the device error and adds no source."""
+    c = dev.Context(0)
+    ngrid, gridmax = 33, 150e-6
+    off, parts = synth.beam(nslice, 256, seed=31)
+    # x stays within 0.15 mm: gradx dx in [-0.69, -0.51], the push's own
+    # polynomial 1 + gradx dx stays positive
+    steps = [synth.und_step(), synth.und_step(ax=1e-3, gradx=600.0)]
+    fc = synth.coupling()
+
+    def go(last):
+        run = dev.Run(c, off, fields=[(1, ngrid, gridmax)], lambda0=synth.LAMBDA0,
+                      gamma_ref=synth.GAMMA0, time_run=False)
+        run.upload_beam(parts)
+        run.upload_field(0, synth.field(nslice, ngrid, gridmax, seed=32, amplitude=1e11))
+        run.set_current(synth.CURRENT)
+        run.set_lattice(steps, [[fc], [last]], [0.0, 0.0])
+        run.advance(0, 1, graph=False)
+        c.synchronize()  # the first step is in order
+        run.advance(1, 1, graph=False)
+        return run
+
+    bad = go(fc)
+    with pytest.raises(G4BError, match="fixed-point range"):
+        c.synchronize()
+    none = go(0.0)
+    c.synchronize()
+    assert np.array_equal(bad.download_field(0)[0], none.download_field(0)[0])
+    for r in (bad, none):
+        r.close()
+    c.close()
