@@ -118,59 +118,90 @@ __device__ __forceinline__ void px_rhs(C (&v)[M], const C* tile, int ld, int row
   }
 }
 
+// The row solve's coefficients: in the single-run kernels a parameter (operands
+// from the constant bank), in the batched ones an image in global memory that
+// differs from item to item.  There each is loaded where it is used (a
+// broadcast from L1), volatile so that the compiler does not keep all M + 2
+// powers in registers from their first use to their last: that spilled up to
+// 1360 bytes per thread in pass Y.  Pass Y of 64 slices, us, plain loads -> now:
+// 255^2 39 -> 25, 400^2 82 -> 60, 500^2 174 -> 90, 700^2 232 -> 145, 880^2 591 ->
+// 314.
+template <typename C>
+struct RowParam {
+  const RowConst<C>& k;
+  __device__ __forceinline__ C P(int m) const { return k.P[m]; }
+  __device__ __forceinline__ C A(int t) const { return k.A[t]; }
+  __device__ __forceinline__ C cb() const { return k.cb; }
+  __device__ __forceinline__ int nscan() const { return k.nscan; }
+};
+struct RowImage {
+  const RowConst<float2>* k;
+  static __device__ __forceinline__ float2 load(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+  }
+  __device__ __forceinline__ float2 P(int m) const { return load(&k->P[m]); }
+  __device__ __forceinline__ float2 A(int t) const { return load(&k->A[t]); }
+  __device__ __forceinline__ float2 cb() const { return load(&k->cb); }
+  __device__ __forceinline__ int nscan() const { return __ldg(&k->nscan); }
+};
+
 // The tridiagonal solve (1 - i r d2) u = R of one row held by a group of L
 // lanes, M consecutive elements each (lane gl: elements gl*M .. gl*M+M-1, of
 // which the first jn lie in the row; R is zero in the others).  wall: the
 // lanes' q^(gl M) / (1 - q^(2n+2)), then their q^(2n+2-(gl+1)M) / (1 - q^(2n+2)).
-template <typename T, int M, int L, typename C>
-__device__ __forceinline__ void row_solve(C (&v)[M], const RowConst<C>& K, const C* wall, int gl,
-                                          int jn, T r) {
+template <typename T, int M, int L, typename C, typename KC>
+__device__ __forceinline__ void row_solve(C (&v)[M], const KC K, const C* wall, int gl, int jn,
+                                          T r) {
   constexpr int kScan = L == 32 ? 5 : 4;  // log2 L
   const C we = wall[gl], wd = wall[L + gl];
-  v[0] = cmul(K.cb, v[0]);
+  const C cb = K.cb();
+  v[0] = cmul(cb, v[0]);
 #pragma unroll
   for (int j = 1; j < M; ++j) {
     C t;
     t.x = fma(-r, v[j - 1].y, v[j].x);
     t.y = fma(r, v[j - 1].x, v[j].y);
-    v[j] = cmul(K.cb, t);
+    v[j] = cmul(cb, t);
   }
   C b = v[M - 1];
 #pragma unroll
   for (int t = 0; t < kScan; ++t) {
-    if (t >= K.nscan) break;
+    if (t >= K.nscan()) break;
     const C o = shfl_up_c<L>(b, 1 << t);
-    if (gl >= 1 << t) b = cfma(K.A[t], o, b);
+    if (gl >= 1 << t) b = cfma(K.A(t), o, b);
   }
   C yin = shfl_up_c<L>(b, 1);
   if (gl == 0) yin = C{0, 0};
 #pragma unroll
-  for (int j = 0; j < M; ++j) v[j] = cfma(K.P[j + 1], yin, v[j]);
+  for (int j = 0; j < M; ++j) v[j] = cfma(K.P(j + 1), yin, v[j]);
   if (jn < M) {  // u is zero from n on
 #pragma unroll
     for (int j = 0; j < M; ++j)
       if (j >= jn) v[j] = C{0, 0};
   }
+  const C q = K.P(1);
 #pragma unroll
-  for (int j = M - 2; j >= 0; --j) v[j] = cfma(K.P[1], v[j + 1], v[j]);
+  for (int j = M - 2; j >= 0; --j) v[j] = cfma(q, v[j + 1], v[j]);
   b = v[0];
 #pragma unroll
   for (int t = 0; t < kScan; ++t) {
-    if (t >= K.nscan) break;
+    if (t >= K.nscan()) break;
     const C o = shfl_down_c<L>(b, 1 << t);
-    if (gl + (1 << t) < L) b = cfma(K.A[t], o, b);
+    if (gl + (1 << t) < L) b = cfma(K.A(t), o, b);
   }
   C uin = shfl_down_c<L>(b, 1);
   if (gl == L - 1) uin = C{0, 0};
   // the wall at k = -1, from lane 0's first element
-  C u0 = cfma(K.P[M], uin, v[0]);
+  C u0 = cfma(K.P(M), uin, v[0]);
   u0.x = -__shfl_sync(0xffffffffu, u0.x, 0, L);
   u0.y = -__shfl_sync(0xffffffffu, u0.y, 0, L);
   const C c = cmul(we, u0);
   uin.x -= fma(wd.x, u0.x, -(wd.y * u0.y));
   uin.y -= fma(wd.x, u0.y, wd.y * u0.x);
 #pragma unroll
-  for (int j = 0; j < M; ++j) v[j] = cfma(K.P[j + 2], c, cfma(K.P[M - j], uin, v[j]));
+  for (int j = 0; j < M; ++j) v[j] = cfma(K.P(j + 2), c, cfma(K.P(M - j), uin, v[j]));
 }
 
 // R' = u' + i r d2x(u') + S (src/Core/FieldSolverADICUDA.cpp:279-323) of a
@@ -203,14 +234,17 @@ __device__ __forceinline__ void px_rprime(C (&v)[M], int gl, T r, unsigned long 
 // three tiles still fit the SM's shared memory); FP32 10 warps of 32-lane rows or 5 warps of two
 // 16-lane rows each (10 rows per band either way; smaller CTAs of 16-lane
 // rows keep six on an SM so that one CTA's loads and stores overlap the
-// others' solves).
+// others' solves).  FP32 rows of 32 x 33 get the registers of one CTA per SM:
+// at 96 the batched form spills (64 slices of 880^2, X / Y: 387 / 326 -> 373 /
+// 314 us).
 template <typename T, int L> struct BandW {
   static constexpr int value = sizeof(T) == 8 ? 9 : (L == 16 ? 5 : 10);
 };
 template <typename T, int M, int L> struct AdiBlocks {
   static constexpr int value =
       sizeof(T) == 8 ? (M <= 7 ? 3 : 2)
-                     : (L == 16 ? (M <= 9 ? 8 : (M <= 17 ? 6 : 4)) : (M <= 9 ? 4 : 2));
+                     : (L == 16 ? (M <= 9 ? 8 : (M <= 17 ? 6 : 4))
+                                : (M <= 9 ? 4 : (M <= 25 ? 2 : 1)));
 };
 
 // One band of W rows (pass X) or W transposed columns (pass Y) of slice s.
@@ -220,10 +254,11 @@ template <typename T, int M, int L> struct AdiBlocks {
 // phase this band waits on.  Returns false, with nothing solved or stored, if
 // the band's rows did not arrive within the bounded wait (the device error
 // flag then says so); the result is the same in every thread of the CTA.
-template <typename T, int M, bool PX, int L, typename C = typename CT<T>::type>
-__device__ __forceinline__ bool adi_band(const AdiPassArgs& a, const RowConst<C>& K,
+template <typename T, int M, bool PX, int L, typename KC>
+__device__ __forceinline__ bool adi_band(const AdiPassArgs& a, const KC K,
                                          const CUtensorMap* tm_out, int s, int band,
                                          unsigned char* smem, uint64_t* bar, uint32_t parity) {
+  using C = typename CT<T>::type;
   constexpr int R = 32 / L;                     // rows per warp
   constexpr int W = BandW<T, L>::value * R;     // rows per band
   const int n = a.n, ld = a.ld;
@@ -424,7 +459,8 @@ __global__ void __launch_bounds__(BandW<T, L>::value * 32, AdiBlocks<T, M, L>::v
   }
   __syncthreads();
   ptx::pdl_wait();
-  adi_band<T, M, PX, L>(a, K, &tm_out, blockIdx.x / a.nband, blockIdx.x % a.nband, smem, &bar, 0u);
+  adi_band<T, M, PX, L>(a, RowParam<typename CT<T>::type>{K}, &tm_out, blockIdx.x / a.nband,
+                        blockIdx.x % a.nband, smem, &bar, 0u);
 }
 
 // Persistent form over a work list of (run, slice, band) items of many runs
@@ -448,9 +484,8 @@ __global__ void __launch_bounds__(BandW<T, L>::value * 32, AdiBlocks<T, M, L>::v
     // a band whose rows never arrived leaves the barrier's phase open: stop
     // (the error flag reports it) rather than wait on it again
     const AdiPassArgs& a = b.args[w.x];
-    if (!adi_band<T, M, PX, L>(a, *static_cast<const RowConst<typename CT<T>::type>*>(a.tab), tm,
-                               w.y, w.z, smem, &bar, parity))
-      return;
+    const RowImage K{static_cast<const RowConst<float2>*>(a.tab)};
+    if (!adi_band<T, M, PX, L>(a, K, tm, w.y, w.z, smem, &bar, parity)) return;
     parity ^= 1u;
     __syncthreads();
   }

@@ -300,3 +300,28 @@ def test_a_layout_switched_after_attaching_takes_effect(ctx, graph):
         _same(_result(r, 9), _result(alone, 9))
         alone.close()
     batch.close()
+
+
+@pytest.mark.parametrize("ngrid, layouts", [(33, (105, 3)), (351, (11, 125)), (400, (125, 13)),
+                                            (528, (133, 17)), (672, (21,)), (700, (25,)),
+                                            (880, (33,))])
+def test_batched_rows_equal_single_rows_in_the_longest_layouts(ctx, ngrid, layouts):
+    """The batched row solve reads its coefficients from an image in memory,
+    the single-run one from its parameters: the same bits, to the widest grid."""
+    cfg = dict(nslice=1, npart=256, ngrid=ngrid, taper=0.0, dgam=0.0, time_run=False, nsteps=3)
+    for layout in layouts:
+        got = []
+        for batched in (False, True):
+            run = _make(ctx, 3, cfg)
+            run.set_layouts([layout])
+            if batched:
+                batch = dev.Batch(ctx, 1)
+                batch.attach(run, 0, 3)
+                batch.step(3, graph=False)
+                ctx.synchronize()
+                batch.close()
+            else:
+                run.advance(0, 3, graph=False)
+            got.append(_result(run, 3))
+            run.close()
+        _same(*got)
