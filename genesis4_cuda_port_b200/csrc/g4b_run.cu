@@ -29,7 +29,6 @@
 #include <map>
 #include <new>
 #include <tuple>
-#include <type_traits>
 #include <vector>
 
 #include "g4b_internal.cuh"
@@ -733,9 +732,10 @@ __global__ void __launch_bounds__(kDiagThreads, 2)
 // are processed in row bands.
 //
 // A slice belongs to one CTA, which holds a band in shared memory; in runs of
-// few slices C CTAs take 1/C of its particles each and add to a tile in global
-// memory (DepTile), and the last of them to finish writes the source.  The
-// integer sums, hence the bits, are the same for every C.
+// few slices C CTAs share it (deposit_part): its particles, added to a tile in
+// global memory (DepTile) of which the last to finish writes the source, or the
+// bands of a large tile.  The integer sums and the scale, hence the bits, are the
+// same however a slice is shared.
 constexpr int kDepThreads = 512;
 constexpr double kDepUnit = 1073741824.0;  // 2^30
 constexpr int kDepMaxWidth = 896;     // tile width bound: mixed ngrid <= 880
@@ -745,13 +745,15 @@ constexpr int kDepMaxWidth = 896;     // tile width bound: mixed ngrid <= 880
 constexpr int kDepCells2 = 9216, kDepCells1 = 18432;
 constexpr size_t dep_smem(int cells) { return (size_t)(3 * cells + kDepMaxWidth) * 4; }
 // Tile of one slice: `cells` sums im 2^32 + re, the counts per base cell
-// (one row more), the bits of the largest charge weight and the CTAs done.
+// (one row more), the bits of the largest charge weight, the CTAs done and, of a
+// slice shared by bands, the largest number of contributions to a cell.
 constexpr int kDepTileCells = 65536;  // at most
 struct DepTile {
   unsigned long long* sum;
   int* hist;
   int* qmax;
   unsigned* done;
+  int* mmax;
 };
 __host__ __device__ constexpr size_t dep_tile_bytes(int cells) {
   return (size_t)cells * 8 + (size_t)(cells + kDepMaxWidth) * 4 + 128;
@@ -762,6 +764,7 @@ __device__ __forceinline__ DepTile dep_tile(unsigned char* tiles, int cells, int
   t.hist = reinterpret_cast<int*>(t.sum + cells);
   t.qmax = t.hist + cells + kDepMaxWidth;
   t.done = reinterpret_cast<unsigned*>(t.qmax + 1);
+  t.mmax = t.qmax + 2;
   return t;
 }
 
@@ -1088,16 +1091,31 @@ __device__ __noinline__ float dep_rare(const DepArgs& a, const DepSlice d, const
   return q;
 }
 
+// True in the CTA that comes last of the C that share a slice: what the others
+// wrote before is then visible to it, and each has read the prediction.
+__device__ __forceinline__ bool dep_last(const DepTile& t, const int C) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(t.done, 1u) == (unsigned)C - 1u;
+  __syncthreads();
+  if (last) __threadfence();
+  return last != 0;
+}
+
 // One field of a slice by a whole CTA, band by band of at most CELLS cells in
 // shared memory; FOUR: by dep_pass4.  With a prediction one pass takes counts,
 // qmax and contributions at the scale of the predicted bounds; it is kept if
 // neither counted bound exceeds its prediction (then no cell sum can have
 // overflowed and no charge was capped), else the contributions are redone at
 // the exact scale 2^30 / (M qmax).  Without one, a first pass only counts.  M
-// and qmax are the slice's, whatever its bands.
+// and qmax are the slice's, whatever its bands.  With C > 1 (and a prediction)
+// CTA `rank` of C takes the bands rank, rank + C, ..., and the last of them to
+// finish goes on with the slice's M and qmax, alone.
 template <int T, bool FOUR, int CELLS>
 __device__ __forceinline__ void deposit_field(const DepArgs& a, const DepField& F,
-                                              const DepSlice& d, unsigned char* smem) {
+                                              const DepSlice& d, unsigned char* smem, int rank = 0,
+                                              int C = 1) {
   const int tid = threadIdx.x, bw = d.bw;
   int* are = reinterpret_cast<int*>(smem);        // [hb * bw] real parts
   int* aim = are + CELLS;                         // [hb * bw] imaginary parts
@@ -1114,7 +1132,7 @@ __device__ __forceinline__ void deposit_field(const DepArgs& a, const DepField& 
   for (;;) {
     const float Sf = (float)(kDepUnit / B);
     const double unscale = d.scl * (B * (1.0 / kDepUnit));
-    for (int yb = 0; yb < d.bh; yb += hband) {
+    for (int yb = rank * hband; yb < d.bh; yb += C * hband) {
       const int hb = min(hband, d.bh - yb), nout = hb * bw;
       __syncthreads();
       if (count) zero(hist, (hb + 1) * bw);
@@ -1150,6 +1168,24 @@ __device__ __forceinline__ void deposit_field(const DepArgs& a, const DepField& 
     }
     if (!count) break;
     dep_max<T>(M, qm);
+    if (C > 1) {
+      const DepTile t = dep_tile(F.tiles, F.tile_cells, d.bs);
+      if (tid == 0) {
+        atomicMax(t.mmax, M);
+        atomicMax(t.qmax, __float_as_int(qm));
+      }
+      if (!dep_last(t, C)) return;
+      M = __ldcg(t.mmax);
+      qm = __int_as_float(__ldcg(t.qmax));
+      __syncthreads();
+      if (tid == 0) {
+        *t.mmax = 0;
+        *t.qmax = 0;
+        *t.done = 0;
+      }
+      rank = 0;
+      C = 1;
+    }
     if (M == 0 || !(qm > 0.f) || !(qm < 3.0e38f)) {
       if (M > 0) atomicOr(a.err, kErrFixedRange);  // non-finite charge
       float2* out = F.src + (size_t)d.target * F.cap;
@@ -1178,15 +1214,48 @@ __device__ __forceinline__ void deposit_slice(const DepArgs& a, const int bs, un
   }
 }
 
-// Part `rank` of C of a slice: the particles [rank, rank + 1) / C into the
-// slice's DepTile; the CTA whose count comes last reads it, writes the source
-// and leaves the tile zero for the next launch.  A field without a prediction,
-// one whose prediction fails, one without a finite charge and one larger than
-// its tile are done by that CTA in shared memory.
+// Part `rank` of C of a slice in runs of few slices, by one of three ways:
+//   tile: each CTA adds its 1/C of the particles to the slice's DepTile; the one
+//   whose count comes last reads it, writes the source and leaves the tile zero
+//   for the next launch;
+//   bands: the bands of a tile of several are shared out (deposit_field);
+//   alone: CTA 0 does a tile of one band in shared memory.
+// A shared field without a prediction, one whose prediction fails and one without
+// a finite charge are done by the CTA that comes last, alone.
+// Where the lines lie (us per graph step; [ ]: two CTAs per slice, bands dealt in
+// turn).  Adds to L2 cost a particle more than adds to shared memory, four times
+// over where its beamlet is not four neighbours of one slice, and the tile costs
+// its reading; the bands cost a pass over all particles each.
+//   One band, tile / alone: 1 x 2048 (129^2) 20.1 / 19.3 [21.6], 1 x 3000 (151^2)
+//   20.1 / 21.9, 12 x 8192 (201^2) 28.2 / 31.8 [33.4], 12 x 32768 66.2 / 69.0 [70];
+//   from 13 slices by the grouping (dep_grouped): beamlets of four, 16 x 32768 46
+//   / 64 [71], 21 x 8192 32.1 / 32.9 [36.2]; others, 16 x 16384 (151^2) 48 / 41
+//   [42], 21 x 32768 105 / 69 [74].
+//   Several bands, tile / bands: 1 x 6000 (255^2) 57 / 31 [67], 21 x 6000 76 / 41
+//   [78], 1 x 60000 58 / 80 [223], 8 x 60000 105 / 105 [273]; more than 65536
+//   cells, alone / bands: 1 x 6000 (401^2) 123 / 33 [113], 21 x 159 / 72 [154].
+constexpr int kDepShareNp = 2560, kDepShareC = 11;
+constexpr int kDepShareNp2 = 32768, kDepShareC2 = 16;
+
+// Do the first 32 groups of four particles of a slice mostly share a cell (the
+// beamlets of a quiet start)?  The same answer in every warp.
+__device__ __forceinline__ bool dep_grouped(const DepSlice& d) {
+  const int p = 4 * (threadIdx.x & 31);  // d.np is larger
+  int cell[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const float2 xy = d.xy[p + u];
+    int ix, iy;
+    float wx, wy;
+    cell[u] = cell_f(d.mf, xy.x, xy.y, ix, iy, wx, wy) ? iy * d.mf.n + ix : -1;
+  }
+  const bool same = cell[0] == cell[1] && cell[0] == cell[2] && cell[0] == cell[3];
+  return __popc(__ballot_sync(0xffffffffu, same)) >= 24;
+}
+
 template <int T>
 __device__ __forceinline__ void deposit_part(const DepArgs& a, const int bs, const int rank,
                                              const int C, unsigned char* smem) {
-  __shared__ int last;
   const int tid = threadIdx.x;
   for (int fi = 0; fi < a.nfield; ++fi) {
     const DepField& F = a.f[fi];
@@ -1194,61 +1263,60 @@ __device__ __forceinline__ void deposit_part(const DepArgs& a, const int bs, con
     if (!F.do_source || !dep_setup(a, F, bs, rank == 0, d)) continue;
     const int bw = d.bw, nout = d.bh * bw, nbase = (d.bh + 1) * bw;
     const DepTile t = dep_tile(F.tiles, F.tile_cells, bs);
-    // true in the CTA of the slice that comes here last (every CTA has then
-    // read the prediction, which that one replaces)
-    auto is_last = [&]() {
-      __threadfence();
-      __syncthreads();
-      if (tid == 0) last = atomicAdd(t.done, 1u) == (unsigned)C - 1u;
-      __syncthreads();
-      if (last) __threadfence();
-      return last != 0;
-    };
-    if (!d.predicted() || nout > F.tile_cells) {
-      if (is_last()) {
-        if (tid == 0) *t.done = 0;
-        deposit_field<T, false, kDepCells1>(a, F, d, smem);
+    const bool bands = nout > kDepCells1;
+    const bool tile = bands ? C >= kDepShareC2 && d.np >= kDepShareNp2 && nout <= F.tile_cells
+                            : d.np >= kDepShareNp && (C >= kDepShareC || dep_grouped(d));
+    int r = 0, c = 1;  // deposit_field's share, unless the tile does
+    if (!bands && !tile) {
+      if (rank > 0) continue;  // CTA 0's
+    } else if (!d.predicted()) {
+      if (!dep_last(t, C)) continue;
+      if (tid == 0) *t.done = 0;
+    } else if (!tile) {
+      r = rank;
+      c = C;
+    } else {
+      const int share = (((d.np + 3) >> 2) + C - 1) / C * 4, plow = rank * share;
+      float qm = 0.f;
+      dep_pass<T, true>(a, d, plow, min(d.np, plow + share), d.by0, d.bh, nullptr, nullptr, t.sum,
+                        t.hist, true, true, (float)(kDepUnit / d.bound()), d.q_use, qm);
+      for (int o = 16; o > 0; o >>= 1) qm = fmaxf(qm, __shfl_xor_sync(0xffffffffu, qm, o));
+      if ((tid & 31) == 0 && qm > 0.f) atomicMax(t.qmax, __float_as_int(qm));
+      if (!dep_last(t, C)) continue;
+      float2* out = F.src + (size_t)d.target * F.cap;
+      const double unscale = d.scl * (d.bound() * (1.0 / kDepUnit));
+      int M = 0;
+      for (int o = 2 * tid; o < nout; o += 2 * T) {
+        const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(t.sum + o));
+        const int x = o - (int)(((float)o + 0.5f) * d.inv_bw) * bw;
+        const int2 up = __ldcg(reinterpret_cast<const int2*>(t.hist + o)),
+                   dn = __ldcg(reinterpret_cast<const int2*>(t.hist + o + bw));
+        const int left = x > 0 ? __ldcg(t.hist + o - 1) + __ldcg(t.hist + o + bw - 1) : 0;
+        const int2 re = make_int2((int)(unsigned)v.x, (int)(unsigned)v.y);
+        dep_write(out + o, re,
+                  make_int2((int)((v.x - re.x) >> 32), (int)((v.y - re.y) >> 32)), unscale);
+        M = max(M, max(left + up.x + dn.x, up.x + dn.x + up.y + dn.y));
       }
-      continue;
+      qm = __int_as_float(__ldcg(t.qmax));
+      dep_max<T>(M, qm);  // (every cell has been read)
+      for (int o = 2 * tid; o < nbase; o += 2 * T) {
+        if (o < nout) *reinterpret_cast<int4*>(t.sum + o) = make_int4(0, 0, 0, 0);
+        *reinterpret_cast<int2*>(t.hist + o) = make_int2(0, 0);
+      }
+      if (tid == 0) {
+        *t.qmax = 0;
+        *t.done = 0;
+      }
+      // without a finite positive charge too deposit_field goes on: it reports that
+      if (M <= d.m_use && qm > 0.f && qm <= d.q_use) {
+        if (tid == 0) {
+          F.mpred[bs] = M;
+          F.qpred[bs] = qm;
+        }
+        continue;
+      }
     }
-    const int share = (((d.np + 3) >> 2) + C - 1) / C * 4, plow = rank * share;
-    float qm = 0.f;
-    dep_pass<T, true>(a, d, plow, min(d.np, plow + share), d.by0, d.bh, nullptr, nullptr, t.sum,
-                      t.hist, true, true, (float)(kDepUnit / d.bound()), d.q_use, qm);
-    for (int o = 16; o > 0; o >>= 1) qm = fmaxf(qm, __shfl_xor_sync(0xffffffffu, qm, o));
-    if ((tid & 31) == 0 && qm > 0.f) atomicMax(t.qmax, __float_as_int(qm));
-    if (!is_last()) continue;
-    float2* out = F.src + (size_t)d.target * F.cap;
-    const double unscale = d.scl * (d.bound() * (1.0 / kDepUnit));
-    int M = 0;
-    for (int o = 2 * tid; o < nout; o += 2 * T) {
-      const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(t.sum + o));
-      const int x = o - (int)(((float)o + 0.5f) * d.inv_bw) * bw;
-      const int2 up = __ldcg(reinterpret_cast<const int2*>(t.hist + o)),
-                 dn = __ldcg(reinterpret_cast<const int2*>(t.hist + o + bw));
-      const int left = x > 0 ? __ldcg(t.hist + o - 1) + __ldcg(t.hist + o + bw - 1) : 0;
-      const int2 re = make_int2((int)(unsigned)v.x, (int)(unsigned)v.y);
-      dep_write(out + o, re,
-                make_int2((int)((v.x - re.x) >> 32), (int)((v.y - re.y) >> 32)), unscale);
-      M = max(M, max(left + up.x + dn.x, up.x + dn.x + up.y + dn.y));
-    }
-    qm = __int_as_float(__ldcg(t.qmax));
-    dep_max<T>(M, qm);  // (every cell has been read)
-    for (int o = 2 * tid; o < nbase; o += 2 * T) {
-      if (o < nout) *reinterpret_cast<int4*>(t.sum + o) = make_int4(0, 0, 0, 0);
-      *reinterpret_cast<int2*>(t.hist + o) = make_int2(0, 0);
-    }
-    if (tid == 0) {
-      *t.qmax = 0;
-      *t.done = 0;
-    }
-    // also without a finite positive charge, which that form reports
-    if (M > d.m_use || !(qm > 0.f && qm <= d.q_use)) {
-      deposit_field<T, false, kDepCells1>(a, F, d, smem);
-    } else if (tid == 0) {
-      F.mpred[bs] = M;
-      F.qpred[bs] = qm;
-    }
+    deposit_field<T, true, kDepCells1>(a, F, d, smem, r, c);
   }
 }
 
@@ -1271,7 +1339,7 @@ struct DepDiagLaunch {
   int parts;
 };
 
-template <int NB, int T>
+template <int NB, int T, bool SHARED>
 __device__ __forceinline__ void deposit_diag_part(const DepArgs& d, const BeamDiagArgs& b,
                                                   const int bs, const int part, const int parts,
                                                   unsigned char* smem) {
@@ -1280,19 +1348,20 @@ __device__ __forceinline__ void deposit_diag_part(const DepArgs& d, const BeamDi
     diag_groups<NB>(b, bs, threadIdx.x >> 5, T / 32, G);
     __syncthreads();
     diag_record<NB, T>(b, bs, G);
-  } else if (parts == 2) {
-    deposit_slice<T, true, T == 512 ? kDepCells1 : kDepCells2>(d, bs, smem);
-  } else {
+  } else if (SHARED) {
     deposit_part<T>(d, bs, part, parts - 1, smem);
+  } else {
+    deposit_slice<T, true, T == 512 ? kDepCells1 : kDepCells2>(d, bs, smem);
   }
 }
 
-template <int NB, int T>
+template <int NB, int T, bool SHARED>
 __global__ void __launch_bounds__(T, 512 / T)
     deposit_diag_kernel(const __grid_constant__ DepDiagLaunch a) {
   extern __shared__ __align__(128) unsigned char smem[];
   ptx::pdl_wait();
-  deposit_diag_part<NB, T>(a.d, a.b, blockIdx.x / a.parts, blockIdx.x % a.parts, a.parts, smem);
+  deposit_diag_part<NB, T, SHARED>(a.d, a.b, blockIdx.x / a.parts, blockIdx.x % a.parts, a.parts,
+                                   smem);
 }
 
 // Batched forms: items[i] = (run, slice of that run).
@@ -1319,13 +1388,13 @@ struct DiagBatchArgs {
   const int* nitems;
 };
 
-template <int NB, int T>
-__global__ void __launch_bounds__(T, 512 / T)
+template <int NB, bool SHARED>
+__global__ void __launch_bounds__(512, 1)
     deposit_diag_batch_kernel(const __grid_constant__ DepBatchArgs b, const BeamDiagArgs* diag,
                               const int parts) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int2 w = b.items[blockIdx.x / parts];
-  deposit_diag_part<NB, T>(b.args[w.x], diag[w.x], w.y, blockIdx.x % parts, parts, smem);
+  deposit_diag_part<NB, 512, SHARED>(b.args[w.x], diag[w.x], w.y, blockIdx.x % parts, parts, smem);
 }
 
 template <int NB>
@@ -1345,29 +1414,41 @@ __global__ void __launch_bounds__(kDiagThreads, 2)
 
 // How a launch over `nslice` slices is split.  parts > 0: that many CTAs per
 // slice, one of them for the diagnostics, of T threads: one CTA of 512 per SM
-// or two of 256; parts > 2: the deposition shared out over a tile in L2.  Else
+// or two of 256; parts > 2: the deposition shared out (deposit_part).  Else
 // one CTA per slice for the deposition and the diagnostics in a kernel of their
 // own: beside it, or in a branch of the graph where the slices fill the GPU
-// twice.  Measured, us per graph step of 8192 particles per slice (before: two
-// CTAs per slice below 296 slices, 256 threads of four particles above):
-//   slices  1 (151^2) 23.2 (28.3), 8 (201^2) 29.0, 16 33.0, 24 37.0 (two parts:
-//   26.3, 31.8, 34.4, 37.0: the adds to L2 cost more per particle than those to
-//   shared memory, so seven parts is where sharing stops to pay);
-//   50 48.6 (50.2), 64 55.3 (58.7), 100 82.2 (83.4), 147 104.5 (106.9);
-//   200 138 (143), 290 180 (191); 1024: the deposition 97 us (121).
-// A deposition waits on its loads, conversions and shared-memory atomics in
-// turn, so what pays is warps per SM: 32 with a particle per lane (64
+// twice.  A deposition waits on its loads, conversions and shared-memory atomics
+// in turn, so what pays is warps per SM: 32 with a particle per lane (64
 // registers) where two CTAs share an SM; four particles per thread at 128
-// registers where there is one.
+// registers where there is one.  A pair of 256 threads has half the band and half
+// the threads for a tile of several bands, and saves time only on small slices.
+// Measured, us per graph step, two CTAs per slice with bands dealt in turn /
+// pairs of 256 / of 512 / one CTA per slice:
+//   22 x 8192 (201^2) 37.9 / - / 33.4 / -, 74 x 8192 63 / 73 / 52 / 80;
+//   75 x 2048 (129^2) 31 / 29 / 31 / 30, 147 x 500 (65^2) 24 / 22 / 26 / 26;
+//   75 x 8192 69 / 62 / 60 / 61, 75 x 6000 (255^2, four bands) 141 / 173 / 110 /
+//   142, 90 x 32768 165 / 182 / 137 / 167, 75 x 3000 (151^2) 43 / 40 / 41 / 41;
+//   110 x 8192 87 / 79 / 77 / 75, 123 x 3000 56 / 53 / 57 / 52, 147 x 6000 (255^2)
+//   199 / 236 / 188 / 184, 147 x 32768 219 / 223 / 200 / 199;
+//   200 x 8192 139 / 136 / 139 / 128; 1024: the deposition 97 us (121).
 constexpr int kSplitMaxParts = 17;
 struct DepSplit {
   int parts, T;
   size_t smem() const { return dep_smem(T == 512 ? kDepCells1 : kDepCells2); }
 };
-static DepSplit dep_split(int nslice, int sm_count) {
-  if (nslice >= sm_count) return {0, 0};
+// Shared out: up to 21 slices.
+static DepSplit dep_split_few(int nslice, int sm_count) {
   const int parts = std::min(kSplitMaxParts, sm_count / nslice);
-  return parts >= 7 ? DepSplit{parts, 512} : DepSplit{2, 2 * nslice <= sm_count ? 512 : 256};
+  return parts >= 7 ? DepSplit{parts, 512} : DepSplit{0, 0};
+}
+// max_np: particles of the largest slice.
+static DepSplit dep_split(int nslice, int max_np, int sm_count) {
+  const DepSplit few = dep_split_few(nslice, sm_count);
+  if (few.parts > 0) return few;
+  if (2 * nslice <= sm_count) return {2, 512};
+  if (nslice < sm_count && max_np <= 2048) return {2, 256};
+  if (3 * nslice < 2 * sm_count) return {2, 512};
+  return {0, 0};
 }
 
 // The same for the slices of a batch, whose particle counts differ: a large slice
@@ -1380,19 +1461,22 @@ static DepSplit dep_split(int nslice, int sm_count) {
 //   runs of 100 slices of 8192: two 209 (253), four 370 (425); four runs of 200
 //   slices of 4096 463 (448).
 static DepSplit dep_split_batch(int nslice, int sm_count) {
-  const DepSplit s = dep_split(nslice, sm_count);
-  if (s.T == 512) return s;
+  const DepSplit few = dep_split_few(nslice, sm_count);
+  if (few.parts > 0) return few;
   return nslice <= 4 * sm_count ? DepSplit{2, 512} : DepSplit{0, 0};
 }
 
-// fn(integral constant NB, integral constant T) of a split launch
-template <typename Fn>
-static void dep_dispatch(bool one, int T, Fn fn) {
-  using std::integral_constant;
-  if (one && T == 512) fn(integral_constant<int, 1>(), integral_constant<int, 512>());
-  else if (one) fn(integral_constant<int, 1>(), integral_constant<int, 256>());
-  else if (T == 512) fn(integral_constant<int, kMaxBunch>(), integral_constant<int, 512>());
-  else fn(integral_constant<int, kMaxBunch>(), integral_constant<int, 256>());
+// The kernels of a split: one bunching harmonic or any number.
+using DepDiagKernel = void (*)(DepDiagLaunch);
+static DepDiagKernel dep_diag_kernel(bool one, DepSplit s) {
+  if (s.parts > 2) return one ? deposit_diag_kernel<1, 512, true> : deposit_diag_kernel<kMaxBunch, 512, true>;
+  if (s.T == 512) return one ? deposit_diag_kernel<1, 512, false> : deposit_diag_kernel<kMaxBunch, 512, false>;
+  return one ? deposit_diag_kernel<1, 256, false> : deposit_diag_kernel<kMaxBunch, 256, false>;
+}
+using DepDiagBatchKernel = void (*)(DepBatchArgs, const BeamDiagArgs*, int);
+static DepDiagBatchKernel dep_diag_batch_kernel(bool one, DepSplit s) {
+  if (s.parts > 2) return one ? deposit_diag_batch_kernel<1, true> : deposit_diag_batch_kernel<kMaxBunch, true>;
+  return one ? deposit_diag_batch_kernel<1, false> : deposit_diag_batch_kernel<kMaxBunch, false>;
 }
 
 // ---------------------------------------------------------- diag finalize --
@@ -1797,7 +1881,7 @@ int launch_single(g4b_run* r, const StepArgs& L) {
   // the deposition and the ADI passes, on SMs those leave idle, joined before
   // the finalize) is for large runs: a fork per step takes a graph long to
   // instantiate.
-  const DepSplit sp = dep_split(r->nslice, c->sm_count);
+  const DepSplit sp = dep_split(r->nslice, (int)r->max_np, c->sm_count);
   const bool one = r->desc.nbunch == 1;
   const bool branch = r->nslice >= 2 * c->sm_count && r->capturing;
   if (branch) {
@@ -1814,12 +1898,8 @@ int launch_single(g4b_run* r, const StepArgs& L) {
   if (sp.parts > 0) {
     LaunchScope ls(c, "run_deposit_diag");
     const DepDiagLaunch dl{L.dd, L.bd, sp.parts};
-    cudaError_t e = cudaSuccess;
-    dep_dispatch(one, sp.T, [&](auto nb, auto t) {
-      e = launch_pdl(deposit_diag_kernel<decltype(nb)::value, decltype(t)::value>,
-                     (unsigned)(r->nslice * sp.parts), (unsigned)sp.T, sp.smem(), c->stream, dl);
-    });
-    G4B_CUDA_TRY(e);
+    G4B_CUDA_TRY(launch_pdl(dep_diag_kernel(one, sp), (unsigned)(r->nslice * sp.parts),
+                            (unsigned)sp.T, sp.smem(), c->stream, dl));
   } else {
     LaunchScope ls(c, "run_deposit");
     G4B_CUDA_TRY(launch_pdl(branch ? deposit_kernel<false> : deposit_kernel<true>,
@@ -1957,7 +2037,7 @@ int g4b_run_create(g4b_ctx* c, const g4b_run_desc* d, const int64_t* off, g4b_ru
     A((void**)&F.d_qpred, d->nslice * sizeof(float));
     F.tile_cells = std::min((F.f->ngrid * F.f->ld + 3) / 4 * 4, kDepTileCells);
     const size_t tiles =
-        dep_split(d->nslice, c->sm_count).parts > 2 ? d->nslice * dep_tile_bytes(F.tile_cells) : 0;
+        dep_split_few(d->nslice, c->sm_count).parts > 0 ? d->nslice * dep_tile_bytes(F.tile_cells) : 0;
     if (tiles) A((void**)&F.d_tiles, tiles);
     A((void**)&F.d_part, (size_t)d->nslice * F.nband * 9 * 8);
     if (e != cudaSuccess) {
@@ -1985,12 +2065,10 @@ int g4b_run_create(g4b_ctx* c, const g4b_run_desc* d, const int64_t* off, g4b_ru
     return cuda_fail(e, "g4b_run_create: device allocation");
   }
   r->step_doubles = (size_t)d->nslice * (r->rec_beam + 9 * d->nfield);
-  for (int k = 0; k < 4; ++k)
-    dep_dispatch(k & 1, k & 2 ? 512 : 256, [&](auto nb, auto t) {
-      cudaFuncSetAttribute(deposit_diag_kernel<decltype(nb)::value, decltype(t)::value>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)DepSplit{2, decltype(t)::value}.smem());
-    });
+  for (const DepSplit s : {DepSplit{3, 512}, DepSplit{2, 512}, DepSplit{2, 256}})
+    for (const bool one : {false, true})
+      cudaFuncSetAttribute(dep_diag_kernel(one, s), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)s.smem());
   cudaFuncSetAttribute(deposit_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)dep_smem(kDepCells2));
   cudaFuncSetAttribute(deposit_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2625,11 +2703,9 @@ int batch_launch(g4b_batch* b, bool timed) {
                    reinterpret_cast<const int2*>(b->d_items + b->off_dep), counts + 1};
     LaunchScope ls(c, "batch_deposit");
     if (sp.parts > 0)
-      dep_dispatch(b->nb_kind == 1, sp.T, [&](auto nb, auto t) {
-        deposit_diag_batch_kernel<decltype(nb)::value, decltype(t)::value>
-            <<<b->counts.dep * sp.parts, sp.T, sp.smem(), c->stream>>>(
-                a, reinterpret_cast<const BeamDiagArgs*>(b->d_args + b->off_bd), sp.parts);
-      });
+      dep_diag_batch_kernel(b->nb_kind == 1, sp)<<<b->counts.dep * sp.parts, sp.T, sp.smem(),
+                                                   c->stream>>>(
+          a, reinterpret_cast<const BeamDiagArgs*>(b->d_args + b->off_bd), sp.parts);
     else
       deposit_batch_kernel<<<b->grid[1], kDepThreads, dep_smem(kDepCells2), c->stream>>>(a);
   }
@@ -2732,12 +2808,10 @@ int g4b_batch_create(g4b_ctx* c, int max_runs, g4b_batch** out) {
   batch_default_grids(b);
   cudaFuncSetAttribute(deposit_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)dep_smem(kDepCells2));
-  for (int k = 0; k < 4; ++k)
-    dep_dispatch(k & 1, k & 2 ? 512 : 256, [&](auto nb, auto t) {
-      cudaFuncSetAttribute(deposit_diag_batch_kernel<decltype(nb)::value, decltype(t)::value>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)DepSplit{2, decltype(t)::value}.smem());
-    });
+  for (const DepSplit s : {DepSplit{3, 512}, DepSplit{2, 512}})
+    for (const bool one : {false, true})
+      cudaFuncSetAttribute(dep_diag_batch_kernel(one, s),
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem());
   if (int rc = batch_layout(b)) {
     g4b_batch_destroy(b);
     return rc;

@@ -325,3 +325,64 @@ def test_batched_rows_equal_single_rows_in_the_longest_layouts(ctx, ngrid, layou
             got.append(_result(run, 3))
             run.close()
         _same(*got)
+
+
+# the splits of a single run: up to 21 slices shared by several CTAs (tile: 3001
+# and 33001 particles; alone: 1500, or 13 slices and more; bands: width 6, and
+# 301^2 for a box above the tile's 65536 cells), pairs of 512 threads to 74 and of
+# 256 to 147 (up to 2048 particles, else of 512 to 98), one CTA per slice above.
+# The second step focuses x to half its width, so that in every split the bounds
+# taken from the step before fail and the deposition is redone.
+@pytest.mark.parametrize("ngrid, npart, width, counts", [
+    (151, 1500, 1.0, (1, 12, 13, 21, 22, 74, 75, 147, 148, 295, 296)),
+    (151, 1500, 6.0, (1, 13, 21, 22, 75, 147, 148, 296)),
+    (151, 3001, 1.0, (1, 12, 13, 22, 75, 98, 99, 148)),
+    (151, 3001, 6.0, (1, 21, 22, 75, 98, 99)),
+    (151, 40000, 6.0, (1, 8, 9, 22, 99)),
+    (301, 2999, 8.0, (1, 21, 22, 75, 99)),
+])
+@pytest.mark.parametrize("nbunch", [1, 3])
+def test_a_slice_does_not_depend_on_the_slices_beside_it(ctx, ngrid, npart, width, counts, nbunch):
+    gm, n = 160e-6, 4
+    sizes = [npart - 1, npart // 2 | 1, npart]  # the second and third start at odd offsets
+    off, parts = synth.beam(3, sizes, seed=21)
+    for k in ("x", "y"):
+        parts[k] = np.clip(parts[k] * width, -0.99 * gm, 0.99 * gm)
+    for k in ("x", "y", "px", "py", "gamma"):  # the first slice in beamlets of four
+        parts[k][:sizes[0]] = np.repeat(parts[k][:sizes[0] // 4 + 1], 4)[:sizes[0]]
+    k60 = (np.pi / (3 * synth.LAMBDA_U)) ** 2  # 60 degrees of phase advance
+    steps = [synth.und_step(), synth.und_step(qf=k60), synth.und_step(), synth.und_step()]
+
+    def go(which, ns, graph):
+        """These of the three slices, spread over a run of ns; the others hold 64."""
+        order = [0, ns // 2, ns - 1][:len(which)]
+        few = synth.beam(1, 64, seed=22)[1]
+        cols = [few] * ns
+        for i, s in zip(which, order):
+            cols[s] = {k: parts[k][off[i]:off[i + 1]] for k in parts}
+        p = {k: np.concatenate([c[k] for c in cols]) for k in parts}
+        o = np.concatenate([[0], np.cumsum([len(c["x"]) for c in cols])])
+        run = dev.Run(ctx, o, fields=[(1, ngrid, gm)], lambda0=synth.LAMBDA0,
+                      gamma_ref=synth.GAMMA0, time_run=False, nbunch=nbunch)
+        run.upload_beam(p)
+        run.upload_field(0, None)
+        run.set_current(synth.CURRENT)
+        run.set_lattice(steps, [[synth.coupling()]] * n, [0.0] * n)
+        run.advance(0, n, graph=graph)
+        beam = run.download_beam()
+        field = run.download_field(0)[0]
+        hist = [run.history(i) for i in range(n)]
+        run.close()
+        return [([beam[k][o[s]:o[s + 1]] for k in beam], field[s],
+                 [(b[s], f[:, s]) for b, f in hist]) for s in order]
+
+    want = go((0, 1, 2), 3, False)
+    assert all(np.any(w[1]) for w in want)
+    for ns in counts:
+        got = go((0, 1, 2), ns, ns % 2 == 0) if ns > 1 else [go((i,), 1, False)[0] for i in range(3)]
+        for g, w in zip(got, want):
+            for a, b in zip(g[0], w[0]):
+                assert np.array_equal(a, b), ns
+            assert np.array_equal(g[1], w[1]), ns
+            for (b1, f1), (b2, f2) in zip(g[2], w[2]):
+                assert np.array_equal(b1, b2) and np.array_equal(f1, f2), ns
