@@ -2495,6 +2495,7 @@ namespace {
 const int kTuneBeam[4] = {4, 8, 16, 32};
 const int kTuneDep[4] = {2, 4, 6, 8};
 const int kTuneAdi[4] = {2, 4, 6, 8};
+constexpr int kDepBatchCtas = 2;  // the untuned deposition's
 
 int batch_layout(g4b_batch* b) {
   size_t o = align_up<BatchCounts>(sizeof(BatchCounts));
@@ -2783,7 +2784,7 @@ int batch_launch(g4b_batch* b, bool timed) {
 void batch_default_grids(g4b_batch* b) {
   const int sm = b->ctx->sm_count;
   b->grid[0] = 2 * kStepBlocks * sm;
-  b->grid[1] = 2 * sm;
+  b->grid[1] = kDepBatchCtas * sm;
   b->grid[2] = 4 * sm;
   b->grid[3] = sm;
 }
@@ -3045,7 +3046,14 @@ int g4b_batch_step(g4b_batch* b, int nsteps, int use_graph) {
       b->tune_idx++;
       if (--b->tune_left == 0) {
         const int* cand[3] = {kTuneBeam, kTuneDep, kTuneAdi};
+        // a deposition split over several CTAs per slice takes no notice of its
+        // grid: the default stays for a later composition
+        const bool split = dep_split_batch(b->counts.dep, sm).parts > 0;
         for (int q = 0; q < 3; ++q) {
+          if (q == 1 && split) {
+            b->grid[1] = kDepBatchCtas * sm;
+            continue;
+          }
           int best = 0;
           for (int j = 1; j < 4; ++j)
             if (b->tune_ms[q][j] < b->tune_ms[q][best]) best = j;

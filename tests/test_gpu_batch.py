@@ -386,3 +386,20 @@ def test_a_slice_does_not_depend_on_the_slices_beside_it(ctx, ngrid, npart, widt
             assert np.array_equal(g[1], w[1]), ns
             for (b1, f1), (b2, f2) in zip(g[2], w[2]):
                 assert np.array_equal(b1, b2) and np.array_equal(f1, f2), ns
+
+
+def test_tuner_leaves_the_deposition_grid_that_a_split_ignores(ctx):
+    """Few slices take several CTAs each, whatever the tuned grid: timings of
+    that launch say nothing about it, so it keeps its default."""
+    batch = dev.Batch(ctx, 2)
+    default = batch.shapes()
+    run = _make(ctx, 3, CONFIGS[3])
+    batch.attach(run, 0, 7)
+    for _ in range(5):  # repeated: timings picked one of four grids by chance
+        batch.tune()
+        batch.step(4, graph=False)
+        assert batch.shapes()["deposit"] == default["deposit"]
+        batch.detach(0)
+        batch.attach(run, 0, 7)
+    batch.close()
+    run.close()

@@ -299,14 +299,14 @@ def test_steady_state_pz_and_bunching_gates(ctx):
     assert np.max(np.abs(bzm - bz_ref)) < B_TOL
 
 
-@pytest.mark.parametrize("nslice", [2, 30, 160])
-def test_charges_that_are_not_finite_are_reported_and_deposit_nothing(nslice):
+@pytest.mark.parametrize("nslice, npart", [(2, 256), (2, 3000), (30, 256), (160, 256)])
+def test_charges_that_are_not_finite_are_reported_and_deposit_nothing(nslice, npart):
     """A step whose undulator gradient makes 1 + 2 gradx dx negative for every
     particle has no finite charge weight: in every split of the deposition the
     step that meets it raises the device error and adds no source."""
     c = dev.Context(0)
     ngrid, gridmax = 33, 150e-6
-    off, parts = synth.beam(nslice, 256, seed=31)
+    off, parts = synth.beam(nslice, npart, seed=31)
     # x stays within 0.15 mm: gradx dx in [-0.69, -0.51], the push's own
     # polynomial 1 + gradx dx stays positive
     steps = [synth.und_step(), synth.und_step(ax=1e-3, gradx=600.0)]
