@@ -5,20 +5,22 @@
 // order (warp xor tree, then warps in index order).  A slice is split over
 // `parts` CTAs where there are fewer slices than the GPU holds CTAs; every CTA
 // writes one record, and the host, which is what the results are for, adds the
-// parts in order.  The entry points' records go straight to pinned host memory,
-// so a call is one launch and one synchronisation (before: one CTA per slice, a
-// device buffer and two or three copies to pageable memory; 60 FP64 steps of one
-// slice with both diagnostics every step 11.4 -> 6.3 ms).  Per launch, beam /
-// field: 1 slice of 8192 and 151^2 24 / 24 -> 13 / 11 us, 256 slices of 8192 and
-// 201^2 45 / 60 -> 39 / 44 us, 300 slices of 5000 with four harmonics 61 -> 43 us.
-// Bound by the latency of the loads and, with several harmonics, by the FP64
-// pipe.
+// parts pairwise.  The entry points' records go straight to pinned host memory,
+// a slice of one part in the caller's layout, so a call is one launch and one
+// synchronisation.  A call, us, one CTA per slice with a device buffer and two or
+// three copies to pageable memory -> now, beam / field: 1 slice of 8192 and 151^2
+// 73 / 48 -> 32 / 25, 148 of 5000 and 129^2 65 / 47 -> 41 / 34, 1024 of 4096 and
+// 101^2 126 / 102 -> 87 / 74, 4096 of 500 and 65^2 166 / 120 -> 123 / 109; 300 of
+// 5000 with four harmonics 102 -> 75.  Bound by the latency of the loads and, with
+// several harmonics, by the FP64 pipe.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
-#include <vector>
 
 #include "g4b_internal.cuh"
 
@@ -26,6 +28,7 @@ namespace g4b {
 
 constexpr int kDiagThreads = 256;
 constexpr int kDiagWarps = kDiagThreads / 32;
+constexpr int kBeamDiagCtas = 2, kFieldDiagCtas = 8;  // per SM, before a slice is not split
 
 enum class Red { Sum, Min, Max };
 
@@ -40,24 +43,30 @@ __device__ __forceinline__ double warp_red(double v, Red op) {
 struct BeamRecArgs {
   const int64_t* off;
   const double *x, *y, *px, *py, *gamma, *theta;
-  double* rec;  // [nslice][parts][23 + 2 nharm]
-  int nharm, need_aux, parts;
+  // parts > 1: [nslice][parts][23 + 2 nharm]; else the caller's three arrays,
+  // [nslice][23], then re and im [nslice][nharm] each
+  double* rec;
+  int nslice, nharm, need_aux, parts;
 };
 
 // g4_beam_slice_reduce_kernel (src/Core/DiagnosticCUDA.cpp:188-303); HP
-// harmonics accumulated per pass over the particles, the higher ones from one
-// sincos by multiplication with e^{i theta}.  U particles in flight per thread.
+// harmonics accumulated per pass over the particles, each by its own sincos
+// corrected for the rounding of k theta.  Multiplying e^{i theta} up instead is
+// a sincos for all, 300 slices of 5000 with four harmonics 36 us against 54, but
+// its errors add up: at the eighth harmonic rms 1.3e-17 of the particles against
+// 2.5e-18 (4.4e-18 without the correction, and 6e-16 at phases of 300).  More
+// than four harmonics at once leave one CTA of registers per SM: 300 x 5000 with
+// eight 126 us a call against 108.
 template <int HP>
-__global__ void __launch_bounds__(kDiagThreads, HP <= 4 ? 2 : 1)
+__global__ void __launch_bounds__(kDiagThreads, 2)
     beam_diag_kernel(const __grid_constant__ BeamRecArgs a) {
-  constexpr int U = HP == 1 ? 4 : 2;
+  constexpr int U = HP == 1 ? 4 : 2;  // particles in flight per thread
   __shared__ double part[kDiagWarps][23 + 2 * HP];
   ptx::pdl_wait();
-  const int is = blockIdx.x / a.parts, ip = blockIdx.x % a.parts;
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  const int is = blockIdx.x / a.parts, ip = blockIdx.x % a.parts;
   const int64_t q0 = a.off[is], all = a.off[is + 1] - q0, per = (all + a.parts - 1) / a.parts;
   const int64_t p0 = q0 + min(all, ip * per), p1 = q0 + min(all, (ip + 1) * per);
-  double* rec = a.rec + (size_t)blockIdx.x * (23 + 2 * a.nharm);
   double v[23];
 #pragma unroll
   for (int k = 0; k < 13; ++k) v[k] = 0.0;
@@ -113,20 +122,16 @@ __global__ void __launch_bounds__(kDiagThreads, HP <= 4 ? 2 : 1)
             v[21] = fmin(v[21], gv); v[22] = fmax(v[22], gv);
           }
         }
-        double s1, c1;
-        sincos(lt[u], &s1, &c1);
-        double s = s1, c = c1;
-        if (hb > 0) sincos((double)(hb + 1) * lt[u], &s, &c);
 #pragma unroll
         for (int h = 0; h < HP; ++h) {
           if (h >= hn) break;
-          br[h] += c;
-          bi[h] += s;
-          if (h + 1 < HP) {
-            const double t = fma(c, c1, -s * s1);
-            s = fma(s, c1, c * s1);
-            c = t;
-          }
+          const double k = (double)(hb + h + 1), ph = k * lt[u];
+          double err = fma(k, lt[u], -ph);  // of the product's rounding
+          if (fabs(err) > 0x1p-27) err = 0.0;  // (phases above 2^26: as rounded)
+          double sh, ch;
+          sincos(ph, &sh, &ch);
+          br[h] += fma(-err, sh, ch);
+          bi[h] += fma(err, ch, sh);
         }
       }
     }
@@ -156,26 +161,32 @@ __global__ void __launch_bounds__(kDiagThreads, HP <= 4 ? 2 : 1)
         const double t = part[i][k];
         r = op == Red::Sum ? r + t : (op == Red::Min ? fmin(r, t) : fmax(r, t));
       }
-      rec[k < 23 ? k : k + 2 * hb] = r;
+      if (a.parts > 1) {
+        a.rec[(size_t)blockIdx.x * (23 + 2 * a.nharm) + (k < 23 ? k : k + 2 * hb)] = r;
+      } else if (k < 23) {
+        a.rec[(size_t)is * 23 + k] = k >= 13 && !a.need_aux ? 0.0 : r;
+      } else {
+        double* b = a.rec + (size_t)a.nslice * (23 + (k % 2 ? 0 : a.nharm));
+        b[(size_t)is * a.nharm + hb + (k - 23) / 2] = r;
+      }
     }
     __syncthreads();
   }
 }
 
-// g4_field_slice_reduce_kernel (src/Core/DiagnosticCUDA.cpp:305-363): records
-// [nslice][parts][9], seven sums and (in the first part) the centre cell; part
-// ip takes the rows of its warps, parts * 8 rows apart.
+// g4_field_slice_reduce_kernel (src/Core/DiagnosticCUDA.cpp:305-363): seven sums
+// and the centre cell, [nslice][parts][7], then [nslice][2]; part ip takes the
+// rows of its warps, parts * 8 rows apart.
 template <typename C>
 __global__ void __launch_bounds__(kDiagThreads)
     field_diag_kernel(int nslice, int n, int ld, int first, int parts, const C* cells,
                       double* rec) {
   __shared__ double part[kDiagWarps][7];
   ptx::pdl_wait();
-  const int is0 = blockIdx.x / parts, ip = blockIdx.x % parts;
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  const int is0 = blockIdx.x / parts, ip = blockIdx.x % parts;
   const C* c = cells + (size_t)is0 * n * ld;
   const int is = (nslice + is0 - first) % nslice;
-  rec += ((size_t)is * parts + ip) * 9;
   const double shift = -0.5 * (double)(n - 1);
   double v[7] = {0, 0, 0, 0, 0, 0, 0};
   // a warp per row: coalesced row reads with no index division, the row's
@@ -213,12 +224,13 @@ __global__ void __launch_bounds__(kDiagThreads)
   if (tid < 7) {
     double r = part[0][tid];
     for (int i = 1; i < kDiagWarps; ++i) r += part[i][tid];
-    rec[tid] = r;
+    rec[((size_t)is * parts + ip) * 7 + tid] = r;
   } else if (tid == 32 && ip == 0) {
     const int ic = (n * n - 1) / 2;
     const C u = c[(size_t)(ic / n) * ld + (ic % n)];
-    rec[7] = u.x;
-    rec[8] = u.y;
+    double* center = rec + (size_t)nslice * parts * 7 + 2 * (size_t)is;
+    center[0] = u.x;
+    center[1] = u.y;
   }
 }
 
@@ -258,7 +270,9 @@ int diag_host(size_t n, double** out) {
 int diag_parts(g4b_ctx* c, int nslice, int per_sm, int64_t most) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(most, per_sm * c->sm_count / nslice));
 }
-int field_parts(g4b_field* f) { return diag_parts(f->ctx, f->nslice, 8, (f->ngrid + 15) / 16); }
+int field_parts(g4b_field* f) {
+  return diag_parts(f->ctx, f->nslice, kFieldDiagCtas, (f->ngrid + 15) / 16);
+}
 
 int launch_field_diag(g4b_field* f, int parts, double* rec) {
   g4b_ctx* c = f->ctx;
@@ -277,18 +291,32 @@ int launch_field_diag(g4b_field* f, int parts, double* rec) {
   return check_launch(c, "field_diag_kernel");
 }
 
-// The parts' field records into the caller's arrays.
-void gather_field(const double* rec, int nslice, int parts, double* stats, double* center) {
-  for (int s = 0; s < nslice; ++s) {
-    const double* r = rec + (size_t)s * parts * 9;
-    for (int k = 0; k < 7; ++k) {
-      double t = r[k];
-      for (int p = 1; p < parts; ++p) t += r[9 * p + k];
-      stats[(size_t)s * 7 + k] = t;
+// Adds the first n values (N where it is known) of the parts' records of one
+// slice into the first part's, pairwise: added one after another they would
+// round as often as there are parts.
+template <int N>
+inline void add_parts(double* r, int parts, size_t stride, int n = N) {
+  for (int d = 1; d < parts; d *= 2)
+    for (int p = 0; p + d < parts; p += 2 * d) {
+      double* __restrict__ a = r + p * stride;
+      const double* __restrict__ b = a + d * stride;
+      for (int k = 0; k < (N ? N : n); ++k) a[k] += b[k];
     }
-    center[2 * s] = r[7];
-    center[2 * s + 1] = r[8];
-  }
+}
+
+size_t field_rec(int nslice, int parts) { return (size_t)nslice * (7 * parts + 2); }
+
+// The field records into the caller's arrays; the parts' are overwritten.
+void gather_field(double* rec, int nslice, int parts, double* stats, double* center) {
+  if (parts == 1)
+    std::memcpy(stats, rec, (size_t)nslice * 7 * sizeof(double));
+  else
+    for (int s = 0; s < nslice; ++s) {
+      double* r = rec + (size_t)s * parts * 7;
+      add_parts<7>(r, parts, 7);
+      std::memcpy(stats + (size_t)s * 7, r, 7 * sizeof(double));
+    }
+  std::memcpy(center, rec + (size_t)nslice * parts * 7, (size_t)nslice * 2 * sizeof(double));
 }
 }  // namespace
 
@@ -340,33 +368,41 @@ int g4b_diag_beam(g4b_beam* b, int nharm, int need_aux, double* stats, double* b
   g4b_ctx* c = b->ctx;
   G4B_CUDA_TRY(cudaSetDevice(c->device));
   const int ns = b->nslice, nrec = 23 + 2 * nharm;
-  const int parts = diag_parts(c, ns, 2, (b->max_slice_np + 511) / 512);
+  const int parts = diag_parts(c, ns, kBeamDiagCtas, (b->max_slice_np + 511) / 512);
   double* rec = nullptr;
   if (int rc = diag_host((size_t)ns * parts * nrec, &rec)) return rc;
   {
     LaunchScope ls(c, "diag_beam");
-    const BeamRecArgs a{b->d_off, b->x,     b->y,  b->px, b->py, b->gamma,
-                        b->theta, rec, nharm, need_aux, parts};
-    auto kern = nharm == 1 ? beam_diag_kernel<1>
-                           : (nharm <= 4 ? beam_diag_kernel<4> : beam_diag_kernel<8>);
+    const BeamRecArgs a{b->d_off, b->x, b->y,  b->px, b->py,    b->gamma,
+                        b->theta, rec,  ns,    nharm, need_aux, parts};
+    auto kern = nharm == 1 ? beam_diag_kernel<1> : beam_diag_kernel<4>;
     G4B_CUDA_TRY(launch_pdl(kern, (unsigned)(ns * parts), kDiagThreads, 0, c->stream, a));
   }
   if (int rc = check_launch(c, "beam_diag_kernel")) return rc;
   G4B_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  if (parts == 1) {
+    const size_t nb = (size_t)ns * nharm;
+    std::memcpy(stats, rec, (size_t)ns * 23 * sizeof(double));
+    std::memcpy(bre, rec + (size_t)ns * 23, nb * sizeof(double));
+    std::memcpy(bim, rec + (size_t)ns * 23 + nb, nb * sizeof(double));
+    return G4B_OK;
+  }
   for (int s = 0; s < ns; ++s) {
-    const double* r = rec + (size_t)s * parts * nrec;
-    double* st = stats + (size_t)s * 23;
-    for (int k = 0; k < nrec; ++k) {
-      const bool sum = k < 13 || k >= 23, lo = (k - 13) % 2 == 0;
-      double t = r[k];
-      for (int p = 1; p < parts; ++p) {
-        const double u = r[(size_t)p * nrec + k];
-        t = sum ? t + u : (lo ? std::fmin(t, u) : std::fmax(t, u));
+    double* r = rec + (size_t)s * parts * nrec;
+    add_parts<13>(r, parts, nrec);
+    add_parts<0>(r + 23, parts, nrec, 2 * nharm);
+    for (int p = 1; p < parts; ++p) {
+      const double* u = r + (size_t)p * nrec;
+      for (int k = 13; k < 23; k += 2) {
+        r[k] = std::fmin(r[k], u[k]);
+        r[k + 1] = std::fmax(r[k + 1], u[k + 1]);
       }
-      if (k < 23)
-        st[k] = k >= 13 && !need_aux ? 0.0 : t;
-      else
-        (k % 2 ? bre : bim)[(size_t)s * nharm + (k - 23) / 2] = t;
+    }
+    std::memcpy(stats + (size_t)s * 23, r, 23 * sizeof(double));
+    if (!need_aux) std::fill_n(stats + (size_t)s * 23 + 13, 10, 0.0);
+    for (int h = 0; h < nharm; ++h) {
+      bre[(size_t)s * nharm + h] = r[23 + 2 * h];
+      bim[(size_t)s * nharm + h] = r[24 + 2 * h];
     }
   }
   return G4B_OK;
@@ -378,7 +414,7 @@ int g4b_diag_field(g4b_field* f, double* stats, double* center) {
   G4B_CUDA_TRY(cudaSetDevice(c->device));
   const int parts = field_parts(f);
   double* rec = nullptr;
-  if (int rc = diag_host((size_t)f->nslice * parts * 9, &rec)) return rc;
+  if (int rc = diag_host(field_rec(f->nslice, parts), &rec)) return rc;
   if (int rc = launch_field_diag(f, parts, rec)) return rc;
   G4B_CUDA_TRY(cudaStreamSynchronize(c->stream));
   gather_field(rec, f->nslice, parts, stats, center);
@@ -399,14 +435,16 @@ int g4b_diag_field_static(g4b_field* f, double* stats, double* center) {
   G4B_CUDA_TRY(cudaSetDevice(c->device));
   double* rec = nullptr;
   if (int rc = static_diag_scratch(c->device, &rec)) return rc;
-  // the records of every part fit: nslice * parts <= max(nslice, 8 CTAs per SM)
+  // the records of every part fit: 7 nslice parts + 2 nslice <= 9 x 4096
   const int parts = std::min(field_parts(f), kStaticDiagMaxSlices / f->nslice);
   if (int rc = launch_field_diag(f, parts, rec)) return rc;
-  std::vector<double> host((size_t)f->nslice * parts * 9);
-  G4B_CUDA_TRY(cudaMemcpyAsync(host.data(), rec, host.size() * sizeof(double),
-                               cudaMemcpyDeviceToHost, c->stream));
+  const size_t n = field_rec(f->nslice, parts);
+  const std::unique_ptr<double[]> host(new (std::nothrow) double[n]);
+  if (!host) return fail(G4B_ERR_NOMEM, "g4b_diag_field_static: host allocation");
+  G4B_CUDA_TRY(cudaMemcpyAsync(host.get(), rec, n * sizeof(double), cudaMemcpyDeviceToHost,
+                               c->stream));
   G4B_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  gather_field(host.data(), f->nslice, parts, stats, center);
+  gather_field(host.get(), f->nslice, parts, stats, center);
   return G4B_OK;
 }
 

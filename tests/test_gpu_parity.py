@@ -326,3 +326,58 @@ def test_diagnostics_split_over_ctas(ctx, nslice, npart, ngrid, nharm):
     rs, rc = orc.diag_field(f0, nslice // 2)
     assert np.max(np.abs(st - rs) / np.max(np.abs(rs), 0)) < 8 * ngrid ** 2 * 2.0 ** -53
     assert np.array_equal(cen, rc)
+
+
+# One particle per slice, so each sum is one cosine or sine: within the 2 ulp of
+# CUDA's sincos and the rounding of the correction for the product h theta, 3 x
+# 2^-53, at every harmonic and phase (the product itself is exact in 64 bits).
+@pytest.mark.parametrize("nharm", [1, 4, 5, 9])
+@pytest.mark.parametrize("span", [0.1, 3.2, 400.0])
+def test_bunching_harmonics_are_single_sines(ctx, nharm, span):
+    ns = 1000
+    off, parts = synth.beam(ns, 1, seed=nharm)
+    parts["theta"] = np.random.default_rng(nharm).uniform(-span, span, ns)
+    beam = _beam(ctx, off, parts)
+    _, re, im = beam.diagnostics(nharm, True)
+    for h in range(nharm):
+        ph = parts["theta"].astype(np.longdouble) * (h + 1)
+        assert np.max(np.abs(re[:, h] - np.cos(ph))) <= 3 * 2.0 ** -53
+        assert np.max(np.abs(im[:, h] - np.sin(ph))) <= 3 * 2.0 ** -53
+    beam.close()
+
+
+# split slices (up to 148), whole ones in the caller's layout above; sums of up to
+# 700 terms round 9 (terms per thread) + 5 + 8 + 9 (parts) times at most, the
+# field's of 33^2 up to 5 + 33 + 5 + 8 + 3
+@pytest.mark.parametrize("ns", [1, 148, 149, 600])
+@pytest.mark.parametrize("nharm, aux", [(1, True), (5, False)])
+def test_diagnostics_of_split_and_whole_slices(ctx, ns, nharm, aux):
+    off, parts = synth.beam(ns, 700, seed=ns, ragged=True)
+    beam = _beam(ctx, off, parts)
+    st, re, im = beam.diagnostics(nharm, aux)
+    p = {k: v.astype(np.longdouble) for k, v in parts.items()}
+    cols = [p["gamma"], p["gamma"] ** 2, p["x"], p["x"] ** 2, p["y"], p["y"] ** 2, p["px"],
+            p["px"] ** 2, p["py"], p["py"] ** 2, p["x"] * p["px"], p["y"] * p["py"]]
+    cols += [f(p["theta"] * (h + 1)) for h in range(nharm) for f in (np.cos, np.sin)]
+    got = [st[:, k] for k in range(12)] + [a[:, h] for h in range(nharm) for a in (re, im)]
+    assert np.array_equal(st[:, 12], np.diff(off))
+    for s in range(ns):
+        o = slice(off[s], off[s + 1])
+        for v, g in zip(cols, got):
+            assert abs(g[s] - v[o].sum()) <= (31 + 3) * 2.0 ** -53 * np.abs(v[o]).sum() + 1e-300
+        for k, (name, lo, hi) in enumerate((("x", 1e5, -1e5), ("px", 1e5, -1e5), ("y", 1e5, -1e5),
+                                            ("py", 1e5, -1e5), ("gamma", 1e7, 1.0))):
+            want = (min([lo, *parts[name][o]]), max([hi, *parts[name][o]])) if aux else (0.0, 0.0)
+            assert tuple(st[s, 13 + 2 * k:15 + 2 * k]) == want
+    n = 33
+    fld = dev.FieldState(ctx, ns, n, 150e-6, synth.LAMBDA0)
+    cells = synth.field(ns, n, 150e-6, seed=5, amplitude=1e11)
+    fld.upload(cells)
+    stats, center = fld.diagnostics()
+    u, d = cells.astype(np.clongdouble), np.arange(n) - np.longdouble(0.5 * (n - 1))
+    w = u.real ** 2 + u.imag ** 2
+    for k, v in enumerate((w, w * d, w * d * d, w * d[:, None], w * d[:, None] ** 2, u.real, u.imag)):
+        assert np.all(np.abs(stats[:, k] - v.sum((1, 2))) <= 58 * 2.0 ** -53 * np.abs(v).sum((1, 2)))
+    assert np.array_equal(center, np.stack([cells.real, cells.imag], -1)[:, n // 2, n // 2])
+    for o in (fld, beam):
+        o.close()
