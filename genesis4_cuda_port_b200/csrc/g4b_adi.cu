@@ -40,6 +40,7 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <limits>
 #include <new>
 #include <utility>
 #include <vector>
@@ -1029,33 +1030,51 @@ void row_tables(double r, int n, int M, int L, RowConst<C>& K, std::vector<unsig
   using T = decltype(C{}.x);
   const cld ir(0.0L, r), beta = (cld(1.0L, 2.0L * r) + std::sqrt(cld(1.0L, 4.0L * r))) / 2.0L;
   const cld q = ir / beta;
+  // products of long doubles by their parts (std::complex's operator tests for
+  // NaN), each table by recurrence: at most a few dozen roundings of 2^-64
+  auto mul = [](cld a, cld b) {
+    return cld(a.real() * b.real() - a.imag() * b.imag(),
+               a.real() * b.imag() + a.imag() * b.real());
+  };
   auto power = [&](long long m) {  // q^m by squaring
     cld p = 1.0L, s = q;
-    for (; m > 0; m >>= 1, s *= s)
-      if (m & 1) p *= s;
+    for (; m > 0; m >>= 1, s = mul(s, s))
+      if (m & 1) p = mul(p, s);
     return p;
   };
-  auto round = [](cld z) {
+  // (what is below half the smallest denormal by a comparison: a conversion
+  // that underflows takes 150 ns, most of a table's time)
+  constexpr long double tiny = std::numeric_limits<T>::denorm_min() / 4.0L;
+  auto round1 = [](long double x) {
+    return std::fabs(x) < tiny ? std::copysign((T)0, (T)(x < 0 ? -1 : 1)) : (T)x;
+  };
+  auto round = [&](cld z) {
     C c;
-    c.x = (T)z.real();
-    c.y = (T)z.imag();
+    c.x = round1(z.real());
+    c.y = round1(z.imag());
     return c;
   };
   K = RowConst<C>{};
-  for (int m = 0; m < kRowMaxM + 2; ++m) K.P[m] = round(power(m));
+  cld p = 1.0L, qM = 1.0L;
+  for (int m = 0; m < kRowMaxM + 2; ++m, p = mul(p, q)) {
+    K.P[m] = round(p);
+    if (m == M) qM = p;
+  }
   K.cb = round(1.0L / beta);
   // scan steps whose multiplier rounds to zero are left out (no more than that:
   // the field far outside the beam is a power of q, small but exact)
-  for (int t = 0; (1 << t) < L; ++t) {
-    K.A[t] = round(power((long long)M << t));
+  p = qM;
+  for (int t = 0; (1 << t) < L; ++t, p = mul(p, p)) {
+    K.A[t] = round(p);
     if (K.A[t].x != 0 || K.A[t].y != 0) K.nscan = t + 1;
   }
   std::vector<C> wall(2 * L, C{0, 0});
-  const cld den = 1.0L - power(2LL * n + 2);
-  for (int l = 0; l < L && l * M < n; ++l) {
-    wall[l] = round(power((long long)l * M) / den);
-    wall[L + l] = round(power(2LL * n + 2 - (long long)(l + 1) * M) / den);
-  }
+  const cld inv = 1.0L / (1.0L - power(2LL * n + 2));
+  const int lanes = (n + M - 1) / M;
+  p = inv;
+  for (int l = 0; l < lanes; ++l, p = mul(p, qM)) wall[l] = round(p);
+  p = mul(power(2LL * n + 2 - (long long)lanes * M), inv);
+  for (int l = lanes - 1; l >= 0; --l, p = mul(p, qM)) wall[L + l] = round(p);
   image.resize(sizeof K + wall.size() * sizeof(C));
   std::memcpy(image.data(), &K, sizeof K);
   std::memcpy(image.data() + sizeof K, wall.data(), wall.size() * sizeof(C));
