@@ -404,54 +404,58 @@ __global__ void __launch_bounds__(kColLines * kLineT, MODE == kColSrc ? 2 : 3)
   }
 }
 
-// Spectrum of the propagation kernel for a step length: c_t = (1/n) sum_k
+// The propagation kernel for a step length and its spectrum: c_t = (1/n) sum_k
 // exp(i k1_k dz) exp(2 pi i k t / n) with the one-axis phases k1 (FP64 cos and
 // sin as the reference's propagator kernel, src/Core/FieldSolverFFTCUDA.cpp:
-// 157-188), laid out as h_m = c_m, h_(512-m) = c_(n-m), and its 512-point
+// 157-188), then, laid out as h_m = c_m, h_(512-m) = c_(n-m), its 512-point
 // transform / 512, both summed with compensation (every step repeats this
-// table's errors, so they are kept below the transforms' own rounding).  Each
-// CTA forms c and 512 / gridDim.x of the outputs, kKernSplit threads per
-// output.
-constexpr int kKernThreads = 256, kKernSplit = 8, kKernGrid = kFftM * kKernSplit / kKernThreads;
+// table's errors, so they are kept below the transforms' own rounding).  A warp
+// per sum and a launch each: a CTA that forms all of c itself takes n^2 terms.
+// 201^2, per change of step length: 20 us in one launch, now 8 (a cluster of
+// eight CTAs that exchange c 16; the propagator table of a full transform pair,
+// n^2 cosines and sines, 4, in front of field steps of twice the time).
+constexpr int kKernThreads = 256, kKernWarps = kKernThreads / 32;
 __device__ __forceinline__ void csum(double2& s, double2& c, double2 v) {
   ptx::csum_add(s.x, c.x, v.x);
   ptx::csum_add(s.y, c.y, v.y);
 }
+__device__ __forceinline__ double2 csum_total(double2 s, double2 c) {
+  ptx::csum_warp(s.x, c.x, 32);
+  ptx::csum_warp(s.y, c.y, 32);
+  return make_double2(s.x + c.x, s.y + c.y);
+}
 __global__ void __launch_bounds__(kKernThreads)
-    fft_kernel_spectrum(const double* k1, const double2* wn, const double2* tw, double delz, int n,
-                        double2* hc) {
-  __shared__ double2 p[kFftMaxN], c[kFftMaxN], w[kFftMaxN];
-  const int tid = threadIdx.x;
+    fft_kernel_taps(const double* k1, const double2* wn, double delz, int n, double2* taps) {
+  __shared__ double2 p[kFftMaxN];
+  const int tid = threadIdx.x, lane = tid & 31;
   ptx::pdl_wait();
   if (tid < n) {
     const double ph = k1[tid] * delz;
     p[tid] = make_double2(cos(ph), sin(ph));
-    w[tid] = wn[tid];  // exp(2 pi i j / n)
   }
   __syncthreads();
-  if (tid < n) {
-    double2 acc = make_double2(0.0, 0.0), err = acc;
-    int j = 0;  // k t mod n
-    for (int k = 0; k < n; ++k) {
-      csum(acc, err, zmul(p[k], w[j]));
-      j += tid;
-      if (j >= n) j -= n;
-    }
-    c[tid] = make_double2((acc.x + err.x) / (double)n, (acc.y + err.y) / (double)n);
-  }
-  __syncthreads();
-  const int out = blockIdx.x * (kKernThreads / kKernSplit) + tid / kKernSplit, part = tid % kKernSplit;
+  const int t = blockIdx.x * kKernWarps + tid / 32;
+  if (t >= n) return;
+  double2 acc = make_double2(0.0, 0.0), err = acc;
+  for (int k = lane; k < n; k += 32) csum(acc, err, zmul(p[k], __ldg(wn + k * t % n)));
+  acc = csum_total(acc, err);
+  if (lane == 0) taps[t] = make_double2(acc.x / (double)n, acc.y / (double)n);
+}
+__global__ void __launch_bounds__(kKernThreads)
+    fft_kernel_spectrum(const double2* taps, const double2* tw, int n, double2* hc) {
+  const int lane = threadIdx.x & 31;
+  ptx::pdl_wait();
+  const int out = blockIdx.x * kKernWarps + threadIdx.x / 32;
   const int t = out & (kLineT - 1), s = out / kLineT;
   const int k = (t >> 3) + 8 * (t & 7) + 64 * brev3(s);
   double2 acc = make_double2(0.0, 0.0), err = acc;
-  for (int m = part; m < n; m += kKernSplit) {
+  for (int m = lane; m < n; m += 32) {
     const double2 e = __ldg(tw + ((k * m) & (kFftM - 1)));
-    csum(acc, err, zmul(c[m], e));
-    if (m > 0) csum(acc, err, zmulc(c[n - m], e));
+    csum(acc, err, zmul(taps[m], e));
+    if (m > 0) csum(acc, err, zmulc(taps[n - m], e));
   }
-  ptx::csum_warp(acc.x, err.x, kKernSplit);
-  ptx::csum_warp(acc.y, err.y, kKernSplit);
-  if (part == 0) hc[out] = make_double2((acc.x + err.x) / kFftM, (acc.y + err.y) / kFftM);
+  acc = csum_total(acc, err);
+  if (lane == 0) hc[out] = make_double2(acc.x / kFftM, acc.y / kFftM);
 }
 
 }  // namespace
@@ -620,7 +624,8 @@ int g4b_fft_init(g4b_fft* s, double delz, double dgrid, double xks, int ngrid) {
     if (int rc = upload(c, &s->wn, wn)) return rc;
     if (int rc = upload(c, &s->k1, k1)) return rc;
     if (int rc = upload(c, &s->sig_t, sig_t)) return rc;
-    if (!s->hc) G4B_CUDA_TRY(dev_alloc(c, (void**)&s->hc, kFftM * sizeof(double2)));
+    if (!s->hc)  // the spectrum, then the kernel itself
+      G4B_CUDA_TRY(dev_alloc(c, (void**)&s->hc, (kFftM + kFftMaxN) * sizeof(double2)));
     s->prop_delz = std::nan("");
     s->filter = s->want_filter && shape_ok;
     s->ngrid = n;
@@ -629,10 +634,17 @@ int g4b_fft_init(g4b_fft* s, double delz, double dgrid, double xks, int ngrid) {
     s->ready = true;
   }
   if (!(s->prop_delz == delz)) {
+    double2* taps = s->hc + kFftM;
+    {
+      LaunchScope ls(c, "fft_kernel_taps");
+      G4B_CUDA_TRY(launch_pdl(fft_kernel_taps, (unsigned)((s->ngrid + kKernWarps - 1) / kKernWarps),
+                              kKernThreads, 0, c->stream, s->k1, s->wn, delz, s->ngrid, taps));
+    }
+    if (int rc = check_launch(c, "fft_kernel_taps")) return rc;
     {
       LaunchScope ls(c, "fft_kernel_spectrum");
-      G4B_CUDA_TRY(launch_pdl(fft_kernel_spectrum, kKernGrid, kKernThreads, 0, c->stream, s->k1,
-                              s->wn, s->tw, delz, s->ngrid, s->hc));
+      G4B_CUDA_TRY(launch_pdl(fft_kernel_spectrum, kFftM / kKernWarps, kKernThreads, 0, c->stream,
+                              taps, s->tw, s->ngrid, s->hc));
     }
     if (int rc = check_launch(c, "fft_kernel_spectrum")) return rc;
     s->prop_delz = delz;
