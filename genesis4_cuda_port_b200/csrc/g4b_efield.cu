@@ -313,9 +313,32 @@ struct g4b_efield {
   double rmax = 0, lambda = 0, ks = 0;
   int ngrid = 0, nz = 0, nphi = 0;
   size_t smem = 0;
+  int resident[4] = {-1, -1, -1, -1};  // clusters of 1, 2, 4, 8 CTAs the GPU holds at once
 };
 
 namespace {
+// Clusters the GPU holds at once: fewer than CTAs per SM times SMs over the size,
+// for a cluster takes its SMs from one GPC.
+int resident_clusters(g4b_efield* e) {
+  for (int k = 0; k < 4 && e->resident[k] < 0; ++k) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1u << k);
+    cfg.blockDim = dim3(kScThreads);
+    cfg.dynamicSmemBytes = e->smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1u << k;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    G4B_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, short_range_kernel, &cfg));
+    e->resident[k] = std::max(1, n);
+  }
+  return G4B_OK;
+}
+
 int ensure_pez(g4b_beam* b) {
   if (b->d_pez) return G4B_OK;
   G4B_CUDA_TRY(dev_alloc(b->ctx, (void**)&b->d_pez,
@@ -396,10 +419,21 @@ int g4b_efield_short_range(g4b_efield* e, g4b_beam* b, double gammaz2) {
   G4B_CUDA_TRY(cudaFuncSetAttribute(short_range_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)e->smem));
-  // the largest cluster with which the slices still fit three CTAs per SM, of at
-  // least 512 particles each
-  int C = 8;
-  while (C > 1 && ((int64_t)b->nslice * C > 3 * c->sm_count || b->max_slice_np < 512 * C)) C >>= 1;
+  // the largest cluster of at least 512 particles per CTA with which the slices
+  // still run at once (a slice more, and the last clusters run alone: 8192
+  // particles with one mode, 55 slices in clusters of 8 / 4 82 / 52 us, 111 in 4 / 2
+  // 99 / 71; one CTA per slice 139).  Where single CTAs take a second round, pairs
+  // if that makes it shorter: large slices, the more of them the more CTAs share
+  // an SM (200 slices of 8192 with 45 modes, one CTA per SM, 981 / 841 us; 600 of
+  // 8192 with one mode, three, 266 / 246, but of 4096 137 / 153)
+  if (int rc = resident_clusters(e)) return rc;
+  const auto rounds = [&](int k) { return (b->nslice + e->resident[k] - 1) / e->resident[k]; };
+  int C = 1;
+  for (int k = 1; k < 4; ++k)
+    if (rounds(k) == 1 && b->max_slice_np >= (512 << k)) C = 1 << k;
+  if (rounds(0) == 2 && rounds(1) < 4 &&
+      (int64_t)b->max_slice_np * c->sm_count >= (int64_t)2560 * e->resident[0])
+    C = 2;
   const unsigned grid = (unsigned)(C * std::max(1, std::min(b->nslice, c->sm_count * 8)));
   {
     LaunchScope ls(c, "short_range");

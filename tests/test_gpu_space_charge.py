@@ -202,3 +202,22 @@ def test_deck_with_space_charge_changes_the_energy_spread():
     assert np.all(np.isfinite(b))
     np.testing.assert_array_equal(a[0], b[0])  # step 0: before any push
     assert np.max(np.abs(b[-1] - a[-1])) > 1e-6 * np.max(np.abs(a[-1]))
+
+
+def test_short_range_pairs_where_single_ctas_take_a_second_round(ctx):
+    """45 modes of 100 cells take an SM's shared memory: 150 slices do not run at
+    once with a CTA each and go as pairs (the tolerance of the test above)."""
+    nslice = 150
+    off, p = _bunched(nslice, 2600, seed=17)
+    cur = np.linspace(2500.0, 800.0, nslice)
+    beam = dev.BeamState(ctx, off, synth.GAMMA0)
+    beam.upload(p)
+    beam.set_current(cur)
+    sc = dev.EFieldSolver(ctx, 2.3, 100, 5, 4, synth.LAMBDA0)
+    sc.short_range(beam, GZ2)
+    got = beam.particle_ez()
+    want = orc.short_range(off, p, cur, GZ2, rmax=2.3, ngrid=100, nz=5, nphi=4,
+                           lambda0=synth.LAMBDA0)
+    assert np.max(np.abs(got - want)) < 1e-9 * np.max(np.abs(want))
+    for o in (sc, beam):
+        o.close()
