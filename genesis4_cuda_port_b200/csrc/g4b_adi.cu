@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(kDepFp64Threads, 1) deposit_slice_kernel(const
         const double f = dep_faw2(a, lx[u], ly[u]), g = fabs(lg[u]);
         m.fmx = f > m.fmx ? f : m.fmx;
         m.gmn = g < m.gmn ? g : m.gmn;
-        if (!(f >= 0.0 && f < 1e300 && g > 1e-290)) m.fmx = INFINITY;  // no finite weight
+        if (!(f >= 0.0 && g > 0.0)) m.fmx = INFINITY;  // no finite weight
         m.ixmin = min(m.ixmin, ix);
         m.ixmax = max(m.ixmax, ix);
         m.iymin = min(m.iymin, iy);
@@ -655,7 +655,8 @@ __global__ void __launch_bounds__(kDepFp64Threads, 1) deposit_slice_kernel(const
     m.cnt = 0;  // lane 0's values are copies of this warp's: they add no extreme
   }
   m.warp_reduce();
-  const double qmax = m.fmx < INFINITY ? sqrt(m.fmx) / m.gmn : INFINITY;
+  double qmax = sqrt(m.fmx) / m.gmn;
+  if (!(qmax <= 1e300)) qmax = INFINITY;  // taken up to there (m.gmn infinite: no charge)
 
   const bool any = m.cnt > 0 && qmax > 0.0;
   if (any && !(qmax < INFINITY) && tid == 0) atomicOr(a.err, kErrFixedRange);

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from genesis4_cuda_port_b200 import device as dev
+from genesis4_cuda_port_b200._lib import G4BError
 from oracle import pyoracle as orc
 from tests import synth
 
@@ -381,3 +382,30 @@ def test_diagnostics_of_split_and_whole_slices(ctx, ns, nharm, aux):
     assert np.array_equal(center, np.stack([cells.real, cells.imag], -1)[:, n // 2, n // 2])
     for o in (fld, beam):
         o.close()
+
+
+def test_deposition_takes_every_weight_up_to_its_limit(ctx):
+    """Charge weights up to 1e300 are taken: with gamma 2^-980 of its value and
+    the current 2^-200 the source is 2^780 times as large, bit for bit; a weight
+    above the limit is reported."""
+    ngrid, gridmax = 33, 150e-6
+    off, parts = synth.beam(2, 500, seed=61)
+    step, got = synth.und_step(), []
+    for eg, ec in ((0, 0), (-980, -200), (-1020, -200)):
+        p = dict(parts, gamma=parts["gamma"] * 2.0 ** eg)
+        beam = _beam(ctx, off, p, np.full(2, synth.CURRENT * 2.0 ** ec))
+        fld = dev.FieldState(ctx, 2, ngrid, gridmax, synth.LAMBDA0)
+        fld.upload(np.zeros((2, ngrid, ngrid), np.complex128))
+        adi = dev.FieldSolverADICUDA(ctx)
+        adi.init(step.delz, fld.dgrid, fld.xks, ngrid)
+        adi.advance(fld, beam, step, fc=synth.coupling())
+        if eg == -1020:
+            with pytest.raises(G4BError, match="fixed-point range"):
+                ctx.synchronize()
+        else:
+            ctx.synchronize()
+            got.append(fld.download())
+        for o in (adi, fld, beam):
+            o.close()
+    assert np.max(np.abs(got[0])) > 0
+    assert np.array_equal(got[1] * 2.0 ** -780, got[0])
