@@ -538,8 +538,9 @@ struct DiagGroups {
 
 // This lane's sum of one unit: quantity lane / (32 / Q).  The lanes are added
 // in a butterfly that halves the quantities a lane carries at every level: 15
-// exchanges for 16 quantities where a tree per quantity takes 80.
-template <int NB>
+// exchanges for 16 quantities where a tree per quantity takes 80.  L2: loads past
+// L1 (see beam_diag_kernel).
+template <int NB, bool L2>
 __device__ __forceinline__ double diag_unit(const BeamDiagArgs& a, const float2* xyp,
                                             const float2* pxyp, const float* dgp,
                                             const double* thp, const int np, const int p0,
@@ -553,10 +554,10 @@ __device__ __forceinline__ double diag_unit(const BeamDiagArgs& a, const float2*
   for (int u = 0; u < kDiagU; ++u) {
     const int p = p0 + 32 * u + lane;
     if (p < np) {
-      lxy[u] = xyp[p];
-      lpp[u] = pxyp[p];
-      ldg[u] = dgp[p];
-      lth[u] = thp[p];
+      lxy[u] = L2 ? __ldcg(xyp + p) : xyp[p];
+      lpp[u] = L2 ? __ldcg(pxyp + p) : pxyp[p];
+      ldg[u] = L2 ? __ldcg(dgp + p) : dgp[p];
+      lth[u] = L2 ? __ldcg(thp + p) : thp[p];
     }
   }
   double v[Q];
@@ -613,7 +614,7 @@ __device__ __forceinline__ double diag_unit(const BeamDiagArgs& a, const float2*
 }
 
 // The groups of slice bs by warp w of nw.
-template <int NB>
+template <int NB, bool L2 = false>
 __device__ __forceinline__ void diag_groups(const BeamDiagArgs& a, const int bs, const int w,
                                             const int nw, DiagGroups<NB>& G) {
   constexpr int Q = DiagGroups<NB>::Q;
@@ -626,7 +627,7 @@ __device__ __forceinline__ void diag_groups(const BeamDiagArgs& a, const int bs,
   for (int g = w; g < kDiagGroups; g += nw) {
     double s = 0.0, c = 0.0;
     for (int u0 = g * kDiagUnit; u0 < np; u0 += kDiagGroups * kDiagUnit)
-      ptx::csum_add(s, c, diag_unit<NB>(a, a.xy + p0, a.pxy + p0, a.dg + p0, a.th + p0, np, u0,
+      ptx::csum_add(s, c, diag_unit<NB, L2>(a, a.xy + p0, a.pxy + p0, a.dg + p0, a.th + p0, np, u0,
                                         mn, mx));
     if (lane % (32 / Q) == 0) G.sum[g][lane / (32 / Q)] = make_double2(s, c);
   }
@@ -697,10 +698,14 @@ __global__ void __launch_bounds__(kDiagThreads, 2)
     beam_diag_kernel(const __grid_constant__ BeamDiagArgs a) {
   __shared__ DiagGroups<NB> G;
   // launched beside the deposition (deposit_kernel): the beam step, whose
-  // output it reads, is complete; the wait for the deposition at its end makes
-  // this kernel's completion imply the deposition's
+  // output it reads, is complete, since the deposition waited for it before it
+  // let this kernel start; but that wait ordered only the deposition's own
+  // reads, so the particles are read from L2 (diag_unit), where the beam step's
+  // writes are, and not through an L1 that may hold older lines.  The wait for
+  // the deposition at its end makes this kernel's completion imply the
+  // deposition's
   if (!BESIDE) ptx::pdl_wait();
-  diag_groups<NB>(a, blockIdx.x, threadIdx.x >> 5, kDiagThreads / 32, G);
+  diag_groups<NB, BESIDE>(a, blockIdx.x, threadIdx.x >> 5, kDiagThreads / 32, G);
   __syncthreads();
   diag_record<NB, kDiagThreads>(a, blockIdx.x, G);
   if (BESIDE) ptx::pdl_wait();
