@@ -518,13 +518,21 @@ struct BeamDiagArgs {
 // Beam diagnostics (DiagnosticCUDA.cpp:102-125): FP64 sums, the minima and
 // maxima in FP32 (exact for FP32 state).  The order of the sums is fixed by
 // the slice alone, so any number of CTAs gives the same bits: a
-// unit of kDiagUnit consecutive particles is summed by one warp (eight per
+// unit of diag_unit_size consecutive particles is summed by one warp (those of a
 // lane in order, then the lanes in a tree), unit j belongs to group j mod
 // kDiagGroups, a group adds its units in order and the groups are added in a
 // tree, both with compensation (csum_*).
 constexpr int kDiagThreads = 256;
-constexpr int kDiagU = 8;             // particles of a unit per lane, all in flight
-constexpr int kDiagUnit = 32 * kDiagU;
+// Particles of a unit: eight per lane, or with several bunching harmonics, whose
+// butterfly of 32 quantities costs as much as three particles, sixteen, in flight
+// by fours (no spills then).  By the run's own harmonics, not the kernel's NB: in a
+// batch a run of one harmonic shares a kernel with others.  16384 particles per
+// slice and eight harmonics, us per step, eight at once / sixteen in fours [one CTA
+// per slice with a tree at its end]: 1 slice 43 / 34 [50], 99 107 / 87 [97], 200 170
+// / 145 [179]; 1024 particles per warp leave slices of 2048 too few warps.
+template <int NB> __device__ __forceinline__ int diag_unit_size(const int nbunch) {
+  return NB == 1 || nbunch == 1 ? 256 : 512;
+}
 constexpr int kDiagGroups = 32;
 constexpr int kDiagSums = 12;         // x, x^2, y, y^2, px, px^2, py, py^2, x px, y py, dg, dg^2
 
@@ -547,54 +555,63 @@ __device__ __forceinline__ double diag_unit(const BeamDiagArgs& a, const float2*
                                             float (&mn)[5], float (&mx)[5]) {
   constexpr int Q = DiagGroups<NB>::Q;
   const int lane = threadIdx.x & 31;
-  float2 lxy[kDiagU], lpp[kDiagU];
-  float ldg[kDiagU];
-  double lth[kDiagU];
-#pragma unroll
-  for (int u = 0; u < kDiagU; ++u) {
-    const int p = p0 + 32 * u + lane;
-    if (p < np) {
-      lxy[u] = L2 ? __ldcg(xyp + p) : xyp[p];
-      lpp[u] = L2 ? __ldcg(pxyp + p) : pxyp[p];
-      ldg[u] = L2 ? __ldcg(dgp + p) : dgp[p];
-      lth[u] = L2 ? __ldcg(thp + p) : thp[p];
-    }
-  }
+  constexpr int U = NB <= 2 ? 8 : 4;  // particles in flight per lane
   double v[Q];
 #pragma unroll
   for (int k = 0; k < Q; ++k) v[k] = 0.0;
+  auto add = [&](const int base) {
+    float2 lxy[U], lpp[U];
+    float ldg[U];
+    double lth[U];
 #pragma unroll
-  for (int u = 0; u < kDiagU; ++u) {
-    if (p0 + 32 * u + lane >= np) break;
-    const double x = lxy[u].x, y = lxy[u].y, px = lpp[u].x, py = lpp[u].y;
-    const double d = ldg[u];
-    v[0] += x; v[1] = __fma_rn(x, x, v[1]);
-    v[2] += y; v[3] = __fma_rn(y, y, v[3]);
-    v[4] += px; v[5] = __fma_rn(px, px, v[5]);
-    v[6] += py; v[7] = __fma_rn(py, py, v[7]);
-    v[8] = __fma_rn(x, px, v[8]); v[9] = __fma_rn(y, py, v[9]);
-    v[10] += d; v[11] = __fma_rn(d, d, v[11]);
-    if (a.need_aux) {
-      const float f[5] = {lxy[u].x, lpp[u].x, lxy[u].y, lpp[u].y, ldg[u]};
-#pragma unroll
-      for (int i = 0; i < 5; ++i) {
-        mn[i] = fminf(mn[i], f[i]);
-        mx[i] = fmaxf(mx[i], f[i]);
+    for (int u = 0; u < U; ++u) {
+      const int p = base + 32 * u + lane;
+      if (p < np) {
+        lxy[u] = L2 ? __ldcg(xyp + p) : xyp[p];
+        lpp[u] = L2 ? __ldcg(pxyp + p) : pxyp[p];
+        ldg[u] = L2 ? __ldcg(dgp + p) : dgp[p];
+        lth[u] = L2 ? __ldcg(thp + p) : thp[p];
       }
     }
-    float s1, c1;
-    __sincosf(reduce_angle(lth[u]), &s1, &c1);
-    float ch = c1, sh = s1;
 #pragma unroll
-    for (int h = 0; h < NB; ++h) {
-      if (h >= a.nbunch) break;
-      v[kDiagSums + 2 * h] += ch;
-      v[kDiagSums + 2 * h + 1] += sh;
-      const float nc = __fmaf_rn(ch, c1, -__fmul_rn(sh, s1));
-      const float ns = __fmaf_rn(sh, c1, __fmul_rn(ch, s1));
-      ch = nc;
-      sh = ns;
+    for (int u = 0; u < U; ++u) {
+      if (base + 32 * u + lane >= np) break;
+      const double x = lxy[u].x, y = lxy[u].y, px = lpp[u].x, py = lpp[u].y;
+      const double d = ldg[u];
+      v[0] += x; v[1] = __fma_rn(x, x, v[1]);
+      v[2] += y; v[3] = __fma_rn(y, y, v[3]);
+      v[4] += px; v[5] = __fma_rn(px, px, v[5]);
+      v[6] += py; v[7] = __fma_rn(py, py, v[7]);
+      v[8] = __fma_rn(x, px, v[8]); v[9] = __fma_rn(y, py, v[9]);
+      v[10] += d; v[11] = __fma_rn(d, d, v[11]);
+      if (a.need_aux) {
+        const float f[5] = {lxy[u].x, lpp[u].x, lxy[u].y, lpp[u].y, ldg[u]};
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+          mn[i] = fminf(mn[i], f[i]);
+          mx[i] = fmaxf(mx[i], f[i]);
+        }
+      }
+      float s1, c1;
+      __sincosf(reduce_angle(lth[u]), &s1, &c1);
+      float ch = c1, sh = s1;
+#pragma unroll
+      for (int h = 0; h < NB; ++h) {
+        if (h >= a.nbunch) break;
+        v[kDiagSums + 2 * h] += ch;
+        v[kDiagSums + 2 * h + 1] += sh;
+        const float nc = __fmaf_rn(ch, c1, -__fmul_rn(sh, s1));
+        const float ns = __fmaf_rn(sh, c1, __fmul_rn(ch, s1));
+        ch = nc;
+        sh = ns;
+      }
     }
+  };
+  if constexpr (NB == 1) {
+    add(p0);
+  } else {
+#pragma unroll 1
+    for (int base = p0; base < min(p0 + diag_unit_size<NB>(a.nbunch), np); base += 32 * U) add(base);
   }
 #pragma unroll
   for (int o = 16, h = Q / 2; o > 0; o >>= 1, h >>= 1) {
@@ -621,12 +638,13 @@ __device__ __forceinline__ void diag_groups(const BeamDiagArgs& a, const int bs,
   const int lane = threadIdx.x & 31;
   const int64_t p0 = a.off[bs];
   const int np = (int)(a.off[bs + 1] - p0);  // at most kRunMaxNp per slice
+  const int unit = diag_unit_size<NB>(a.nbunch);
   // minima / maxima of x, px, y, py (reference start values -+1e5) and dg
   float mn[5] = {1.0e5f, 1.0e5f, 1.0e5f, 1.0e5f, INFINITY};
   float mx[5] = {-1.0e5f, -1.0e5f, -1.0e5f, -1.0e5f, -INFINITY};
   for (int g = w; g < kDiagGroups; g += nw) {
     double s = 0.0, c = 0.0;
-    for (int u0 = g * kDiagUnit; u0 < np; u0 += kDiagGroups * kDiagUnit)
+    for (int u0 = g * unit; u0 < np; u0 += kDiagGroups * unit)
       ptx::csum_add(s, c, diag_unit<NB, L2>(a, a.xy + p0, a.pxy + p0, a.dg + p0, a.th + p0, np, u0,
                                         mn, mx));
     if (lane % (32 / Q) == 0) G.sum[g][lane / (32 / Q)] = make_double2(s, c);

@@ -403,3 +403,34 @@ def test_tuner_leaves_the_deposition_grid_that_a_split_ignores(ctx):
         batch.attach(run, 0, 7)
     batch.close()
     run.close()
+
+
+def test_runs_of_different_harmonics_share_a_batch(ctx):
+    """The diagnostics' order of sums follows the run's own number of bunching
+    harmonics: in a batch whose kernel serves several, every run has its bits."""
+    n = 4
+
+    def make(k, nbunch):
+        off, parts = synth.beam(2, [5000, 1111], seed=80 + k)
+        run = dev.Run(ctx, off, fields=[(1, 65, 160e-6)], lambda0=synth.LAMBDA0,
+                      gamma_ref=synth.GAMMA0, time_run=False, nbunch=nbunch)
+        run.upload_beam(parts)
+        run.upload_field(0, None)
+        run.set_current(synth.CURRENT)
+        run.set_lattice([synth.und_step()] * n, [[synth.coupling()]] * n, [0.0] * n)
+        return run
+
+    kinds = [1, 2, 5, 8]
+    batch = dev.Batch(ctx, len(kinds))
+    runs = [make(k, nb) for k, nb in enumerate(kinds)]
+    for r in runs:
+        batch.attach(r, 0, n)
+    batch.step(n, graph=False)
+    ctx.synchronize()
+    for k, (r, nb) in enumerate(zip(runs, kinds)):
+        alone = make(k, nb)
+        alone.advance(0, n, graph=False)
+        _same(_result(r, n), _result(alone, n))
+        alone.close()
+        r.close()
+    batch.close()
