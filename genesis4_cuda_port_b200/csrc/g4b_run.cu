@@ -2520,6 +2520,14 @@ const int kTuneDep[4] = {2, 4, 6, 8};
 const int kTuneAdi[4] = {2, 4, 6, 8};
 constexpr int kDepBatchCtas = 2;  // the untuned deposition's
 
+// The first `n` branch streams (a batch of more row layouts than usual gets the
+// others when it is listed).
+int batch_streams(g4b_batch* b, int n) {
+  for (int k = 0; k < std::min(n, g4b_batch::kAux); ++k)
+    if (!b->aux[k]) G4B_CUDA_TRY(cudaStreamCreateWithFlags(&b->aux[k], cudaStreamNonBlocking));
+  return G4B_OK;
+}
+
 int batch_layout(g4b_batch* b) {
   size_t o = align_up<BatchCounts>(sizeof(BatchCounts));
   const size_t nr = b->max_runs, nf = (size_t)b->max_runs * kRunFields;
@@ -2550,8 +2558,7 @@ int batch_layout(g4b_batch* b) {
   for (auto& e : b->ev_fork) G4B_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (auto& e : b->ev_adi) G4B_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   G4B_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_diag, cudaEventDisableTiming));
-  for (auto& s : b->aux) G4B_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  return G4B_OK;
+  return batch_streams(b, 4);
 }
 
 // Rebuild the work lists after the set of attached, unfinished runs changed.
@@ -2607,6 +2614,9 @@ int batch_rebuild(g4b_batch* b) {
     b->off_adi[m] = need;
     need = align_up<int4>(need + b->adi_items[m].size() * sizeof(int4));
   }
+  int ngroups = 0;
+  for (int m = 0; m < kNumM; ++m) ngroups += b->counts.adi[m] > 0;
+  if (int rc = batch_streams(b, ngroups)) return rc;
   need = std::max<size_t>(need, 256);
   if (need > b->items_cap) {  // stream-ordered: the old lists' readers finish first
     dev_free(b->ctx, b->d_items);
