@@ -41,14 +41,15 @@
 // and C.
 //
 // Bound: the FP64 pipe (about 530 FP64 instructions per thread and line, half
-// an SM clock each) and the exchanges (64 16-byte accesses per thread, two
-// clocks each) take about the same time, some 600 clocks per line together
-// when overlapped; measured, 1024 slices of 201^2 (CUDA events): rows 0.61 ms,
-// columns 0.93 ms, against 1.27 + 2.31 + 1.59 ms for the forward, middle and
-// inverse passes of a full transform pair with a line per warp (sixteen values
-// per thread, 128 registers); cuFFT's forward and inverse pair takes 4.99 ms.
-// The field step with its source: 5.48 -> 1.84 ms.  The order of the spectrum (thread t, slot s) -> k = t / 8 +
-// 8 (t % 8) + 64 brev3(s) is seen by the pointwise multiply alone.
+// an SM clock per warp each) and the exchanges (64 16-byte accesses per thread,
+// four clocks per warp each) take about the same time, some 600 clocks per line
+// together when overlapped; measured, 1024 slices of 201^2 (CUDA events): rows
+// 0.61 ms, columns 0.93 ms, against 1.27 + 2.31 + 1.59 ms for the forward, middle
+// and inverse passes of a full transform pair with a line per warp (sixteen
+// values per thread, 128 registers); cuFFT's forward and inverse pair takes 4.99
+// ms.  The field step with its source: 5.48 -> 1.74 ms.  The order of the spectrum
+// (thread t, slot s) -> k = t / 8 + 8 (t % 8) + 64 brev3(s) is seen by the
+// pointwise multiply alone.
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -327,11 +328,12 @@ __global__ void __launch_bounds__(kRowLines * kLineT, 2)
 // Columns, four per CTA, through a shared tile of the plane's rows (64-byte
 // segments in global memory; entry (row, c) of the tile at row * 4 +
 // (c ^ row / 2 % 4), so that the threads of a line read its rows without bank
-// conflicts).  Three CTAs per SM (96 slices of 201^2: 94 us with the tile
-// copied by cp.async, 101 us through registers; eight columns per CTA 107 us
-// at one and 130 us at two CTAs per SM); the two transforms of kColSrc at two
-// (124 against 132 us for 64 slices of 255^2).  kColConv: u's columns convolved in place; kColAdd: + 2 S;
-// kColSrc: the columns of st forward, times 2 filter, back, in place.
+// conflicts).  Three CTAs per SM, 80 registers with 64-84 bytes of spills (96
+// slices of 201^2: 94 us with the tile copied by cp.async, 101 us through
+// registers; eight columns per CTA 107 us at one and 130 us at two CTAs per SM);
+// the two transforms of kColSrc at two (124 against 132 us for 64 slices of
+// 255^2).  kColConv: u's columns convolved in place; kColAdd: + 2 S; kColSrc: the
+// columns of st forward, times 2 filter, back, in place.
 enum { kColConv, kColAdd, kColSrc };
 __device__ __forceinline__ int col_swz(int y) { return (y >> 1) & 3; }
 template <int MODE>

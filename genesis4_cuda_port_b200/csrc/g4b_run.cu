@@ -12,13 +12,13 @@
 //                  cells (integer atomics, order independent);
 //   K2 deposit : per slice, the deterministic exact-integer deposition of
 //                  every field's source into a compact tile, and the beam
-//                  diagnostics (FP64 sums): a branch of the captured graph
-//                  beside the deposition in runs that fill the GPU, in the
-//                  deposition's CTAs (first) in smaller runs;
+//                  diagnostics (FP64 sums) into the history buffer: a branch of
+//                  the captured graph or a kernel beside the deposition in
+//                  runs of many slices, CTAs of the same launch in smaller ones;
 //   K3/K4 ADI passes per field (pass Y also zeroes the planes this step's
 //                  slippage zeroes and writes field-diagnostic partials);
-//   K5 diag_finalize : per-slice beam and field diagnostics into the history
-//                  buffer.
+//   K5 diag_finalize : per-slice field diagnostics into the history buffer;
+//                  resets the slices' boxes.
 // The theta derivative ks(1-1/b) + ku is evaluated cancellation-free in FP64
 // as ku - ks*eps/(b(1+b)), eps = btper0/gamma^2 (the two ~ku terms cancel to
 // the detuning).  Slippage is the host's integer index model: `first` and the
