@@ -64,13 +64,16 @@ namespace {
 constexpr int kFftM = 512;       // convolution length
 constexpr int kFftMaxN = 256;    // 2 n - 1 <= 512
 constexpr int kLineT = 64;       // threads per line
+constexpr int kTwA = kFftM;              // W_512^(k t), k = 1, 2, 4, t < 64
+constexpr int kTwB = kTwA + 3 * kLineT;  // W_64^(k t), k = 1, 2, 4, t < 8
+constexpr int kTwAll = kTwB + 3 * 8;
 constexpr int kRowLines = 4;     // lines per CTA along x
 constexpr int kColLines = 4;     // lines per CTA along y (64-byte row segments)
 constexpr int kXbRow = 9;                   // padded row of eight
 constexpr int kXb = 8 * 8 * kXbRow;         // exchange buffer of a line (double2)
 
 struct FftArgs {
-  const double2* tw;      // W_512^j, j < 512
+  const double2* tw;      // W_512^j, j < 512, the lines' factors (kTwA, kTwB), W_512^j's second words
   const double2* chirp;   // w_j, j < n
   const double2* hc;      // FFT_512 of the propagation kernel / 512, slot * 64 + t
   const double2* hf;      // FFT_512(conj w) / 512
@@ -96,21 +99,26 @@ __device__ __forceinline__ double2 zmulc(double2 a, double2 b) {
 }
 __host__ __device__ constexpr int brev3(int k) { return ((k & 1) << 2) | (k & 2) | ((k & 4) >> 2); }
 
-constexpr double kS = 0.70710678118654752440;
+// t / sqrt2 with sqrt2 / 2 as two words: every transform of every step meets the
+// first one's error, always the same way (24 source-free steps at 151^2, a
+// Gaussian beam: 8.8e-15 rms without the second, 4.0e-15 with it; 256 slices of
+// 201^2: 400 and 413 us).
+constexpr double kS = 0.70710678118654752440, kSl = -4.8336466567264565e-17;
+__device__ __forceinline__ double by_s(double t) { return fma(kS, t, kSl * t); }
 
 __device__ __forceinline__ double2 mul_w1(double2 z) {  // x (1 - i)/sqrt2
-  return make_double2(kS * (z.x + z.y), kS * (z.y - z.x));
+  return make_double2(by_s(z.x + z.y), by_s(z.y - z.x));
 }
 __device__ __forceinline__ double2 mul_w2(double2 z) { return make_double2(z.y, -z.x); }  // x (-i)
 __device__ __forceinline__ double2 mul_w3(double2 z) {  // x (-1 - i)/sqrt2
-  return make_double2(kS * (z.y - z.x), -kS * (z.x + z.y));
+  return make_double2(by_s(z.y - z.x), by_s(-z.x - z.y));
 }
 __device__ __forceinline__ double2 mul_c1(double2 z) {  // x (1 + i)/sqrt2
-  return make_double2(kS * (z.x - z.y), kS * (z.x + z.y));
+  return make_double2(by_s(z.x - z.y), by_s(z.x + z.y));
 }
 __device__ __forceinline__ double2 mul_c2(double2 z) { return make_double2(-z.y, z.x); }  // x i
 __device__ __forceinline__ double2 mul_c3(double2 z) {  // x (-1 + i)/sqrt2
-  return make_double2(-kS * (z.x + z.y), kS * (z.x - z.y));
+  return make_double2(by_s(-z.x - z.y), by_s(z.x - z.y));
 }
 
 // 8-point DFT of v[0..7] (radix-2, decimation in frequency): X[k] lands in
@@ -181,12 +189,18 @@ __device__ __forceinline__ void idft8(double2 (&v)[8]) {
   }
 }
 
-// Slot s holds k = brev3(s): times w^k (CONJ: its conjugate).
+// Slot s holds k = brev3(s): times w^k (CONJ: its conjugate).  w, w^2 and w^4
+// are table entries, the others products of them: every step repeats a factor's
+// error, and with all powers from w alone, up to seven times its own, they were
+// most of what the solver lost over a run (24 source-free steps at 101^2, a
+// Gaussian beam: 2.0e-14 rms against 7.5e-15, and 5.0e-15 with every power from
+// the table).  256 slices of 201^2: 409 us with one entry, 400 with three, 437
+// with seven.
 template <bool CONJ>
 __device__ __forceinline__ double2 tmul(double2 z, double2 w) { return CONJ ? zmulc(z, w) : zmul(z, w); }
-template <bool CONJ>
-__device__ __forceinline__ void twiddle8(double2 (&v)[8], double2 w1) {
-  const double2 w2 = zmul(w1, w1), w4 = zmul(w2, w2);
+template <bool CONJ, int STRIDE>
+__device__ __forceinline__ void twiddle8(double2 (&v)[8], const double2* w) {
+  const double2 w1 = __ldg(w), w2 = __ldg(w + STRIDE), w4 = __ldg(w + 2 * STRIDE);
   v[brev3(1)] = tmul<CONJ>(v[brev3(1)], w1);
   v[brev3(2)] = tmul<CONJ>(v[brev3(2)], w2);
   v[brev3(4)] = tmul<CONJ>(v[brev3(4)], w4);
@@ -202,7 +216,7 @@ struct Line {
   int t;             // thread of the line
   int bar;           // named barrier of its two warps
   double2* xb;       // its exchange buffer
-  double2 wa, wb;    // W_512^t, W_64^(t % 8)
+  const double2 *wa, *wb;  // powers of W_512^t and of W_64^(t % 8)
   __device__ __forceinline__ void sync() const {
     asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kLineT) : "memory");
   }
@@ -212,8 +226,8 @@ __device__ __forceinline__ Line make_line(const FftArgs& a, int line, double2* x
   L.t = threadIdx.x & (kLineT - 1);
   L.bar = 1 + line;
   L.xb = xall + line * kXb;
-  L.wa = __ldg(a.tw + L.t);
-  L.wb = __ldg(a.tw + 8 * (L.t & 7));
+  L.wa = a.tw + kTwA + L.t;
+  L.wb = a.tw + kTwB + (L.t & 7);
   return L;
 }
 
@@ -227,14 +241,14 @@ __device__ __forceinline__ void conv512(double2 (&v)[8], const Line& L, const do
   double2* grp = L.xb + hi * 8 * kXbRow + lo;     // entry (k0, 0, j0)
   double2* row = L.xb + hi * 8 * kXbRow + lo * kXbRow;  // entry (k0, k1, 0)
   dft8<true>(v);
-  twiddle8<false>(v, L.wa);
+  twiddle8<false, kLineT>(v, L.wa);
 #pragma unroll
   for (int s = 0; s < 8; ++s) own[brev3(s) * 8 * kXbRow] = v[s];
   L.sync();
 #pragma unroll
   for (int j = 0; j < 8; ++j) v[j] = grp[j * kXbRow];
   dft8<false>(v);
-  twiddle8<false>(v, L.wb);
+  twiddle8<false, 8>(v, L.wb);
 #pragma unroll
   for (int s = 0; s < 8; ++s) grp[brev3(s) * kXbRow] = v[s];
   __syncwarp();
@@ -249,14 +263,14 @@ __device__ __forceinline__ void conv512(double2 (&v)[8], const Line& L, const do
   __syncwarp();
 #pragma unroll
   for (int s = 0; s < 8; ++s) v[s] = grp[brev3(s) * kXbRow];
-  twiddle8<true>(v, L.wb);
+  twiddle8<true, 8>(v, L.wb);
   idft8<false>(v);
 #pragma unroll
   for (int j = 0; j < 8; ++j) grp[j * kXbRow] = v[j];
   L.sync();
 #pragma unroll
   for (int s = 0; s < 8; ++s) v[s] = own[brev3(s) * 8 * kXbRow];
-  twiddle8<true>(v, L.wa);
+  twiddle8<true, kLineT>(v, L.wa);
   idft8<true>(v);
 }
 
@@ -410,22 +424,36 @@ __global__ void __launch_bounds__(kColLines * kLineT, MODE == kColSrc ? 2 : 3)
 // exp(i k1_k dz) exp(2 pi i k t / n) with the one-axis phases k1 (FP64 cos and
 // sin as the reference's propagator kernel, src/Core/FieldSolverFFTCUDA.cpp:
 // 157-188), then, laid out as h_m = c_m, h_(512-m) = c_(n-m), its 512-point
-// transform / 512, both summed with compensation (every step repeats this
-// table's errors, so they are kept below the transforms' own rounding).  A warp
-// per sum and a launch each: a CTA that forms all of c itself takes n^2 terms.
-// 201^2, per change of step length: 20 us in one launch, now 8 (a cluster of
+// transform / 512.  Every step repeats this table's errors, so the roots of unity
+// and c carry a second word, products their rounding error, and the sums are
+// compensated: beyond the phases' own rounding the spectrum is rounded once.  A
+// warp per sum and a launch each: a CTA that forms all of c itself takes n^2 terms.
+// 201^2, per change of step length: 20 us in one launch, now 10 (a cluster of
 // eight CTAs that exchange c 16; the propagator table of a full transform pair,
 // n^2 cosines and sines, 4, in front of field steps of twice the time).
 constexpr int kKernThreads = 256, kKernWarps = kKernThreads / 32;
-__device__ __forceinline__ void csum(double2& s, double2& c, double2 v) {
-  ptx::csum_add(s.x, c.x, v.x);
-  ptx::csum_add(s.y, c.y, v.y);
-}
-__device__ __forceinline__ double2 csum_total(double2 s, double2 c) {
-  ptx::csum_warp(s.x, c.x, 32);
-  ptx::csum_warp(s.y, c.y, 32);
-  return make_double2(s.x + c.x, s.y + c.y);
-}
+struct CSum {
+  double s = 0.0, c = 0.0;
+  // + (a + al) (b + bl)
+  __device__ __forceinline__ void add(double a, double al, double b, double bl) {
+    const double p = a * b;
+    c += fma(a, bl, fma(al, b, fma(a, b, -p)));
+    ptx::csum_add(s, c, p);
+  }
+  // The lanes' total, rounded to the first word with the rest in the second.
+  __device__ __forceinline__ void total() {
+    ptx::csum_warp(s, c, 32);
+    const double t = s + c;
+    c -= t - s;
+    s = t;
+  }
+  // ... divided by n.
+  __device__ __forceinline__ void divide(double n) {
+    const double q = s / n;
+    c = (fma(-q, n, s) + c) / n;
+    s = q;
+  }
+};
 __global__ void __launch_bounds__(kKernThreads)
     fft_kernel_taps(const double* k1, const double2* wn, double delz, int n, double2* taps) {
   __shared__ double2 p[kFftMaxN];
@@ -438,10 +466,22 @@ __global__ void __launch_bounds__(kKernThreads)
   __syncthreads();
   const int t = blockIdx.x * kKernWarps + tid / 32;
   if (t >= n) return;
-  double2 acc = make_double2(0.0, 0.0), err = acc;
-  for (int k = lane; k < n; k += 32) csum(acc, err, zmul(p[k], __ldg(wn + k * t % n)));
-  acc = csum_total(acc, err);
-  if (lane == 0) taps[t] = make_double2(acc.x / (double)n, acc.y / (double)n);
+  CSum re, im;
+  for (int k = lane; k < n; k += 32) {
+    const double2 w = __ldg(wn + k * t % n), wl = __ldg(wn + n + k * t % n);
+    re.add(p[k].x, 0.0, w.x, wl.x);
+    re.add(-p[k].y, 0.0, w.y, wl.y);
+    im.add(p[k].x, 0.0, w.y, wl.y);
+    im.add(p[k].y, 0.0, w.x, wl.x);
+  }
+  re.total();
+  im.total();
+  if (lane == 0) {
+    re.divide((double)n);
+    im.divide((double)n);
+    taps[t] = make_double2(re.s, im.s);
+    taps[n + t] = make_double2(re.c, im.c);
+  }
 }
 __global__ void __launch_bounds__(kKernThreads)
     fft_kernel_spectrum(const double2* taps, const double2* tw, int n, double2* hc) {
@@ -450,14 +490,26 @@ __global__ void __launch_bounds__(kKernThreads)
   const int out = blockIdx.x * kKernWarps + threadIdx.x / 32;
   const int t = out & (kLineT - 1), s = out / kLineT;
   const int k = (t >> 3) + 8 * (t & 7) + 64 * brev3(s);
-  double2 acc = make_double2(0.0, 0.0), err = acc;
+  CSum re, im;
   for (int m = lane; m < n; m += 32) {
     const double2 e = __ldg(tw + ((k * m) & (kFftM - 1)));
-    csum(acc, err, zmul(taps[m], e));
-    if (m > 0) csum(acc, err, zmulc(taps[n - m], e));
+    const double2 el = __ldg(tw + kTwAll + ((k * m) & (kFftM - 1)));
+    double2 v = taps[m], vl = taps[n + m];
+    re.add(v.x, vl.x, e.x, el.x);
+    re.add(-v.y, -vl.y, e.y, el.y);
+    im.add(v.x, vl.x, e.y, el.y);
+    im.add(v.y, vl.y, e.x, el.x);
+    if (m > 0) {  // h_(512-m): the conjugate factor
+      v = taps[n - m], vl = taps[2 * n - m];
+      re.add(v.x, vl.x, e.x, el.x);
+      re.add(v.y, vl.y, e.y, el.y);
+      im.add(-v.x, -vl.x, e.y, el.y);
+      im.add(v.y, vl.y, e.x, el.x);
+    }
   }
-  acc = csum_total(acc, err);
-  if (lane == 0) hc[out] = make_double2(acc.x / kFftM, acc.y / kFftM);
+  re.total();
+  im.total();
+  if (lane == 0) hc[out] = make_double2(re.s / kFftM, im.s / kFftM);
 }
 
 }  // namespace
@@ -506,6 +558,12 @@ std::vector<double2> permuted_spectrum(const std::vector<cld>& h) {
       out[s * kLineT + t] = make_double2((double)v.real(), (double)v.imag());
     }
   return out;
+}
+
+// A root of unity as two words.
+void split(long double re, long double im, double2& hi, double2& lo) {
+  hi = make_double2((double)re, (double)im);
+  lo = make_double2((double)(re - (long double)hi.x), (double)(im - (long double)hi.y));
 }
 
 template <typename T>
@@ -576,10 +634,14 @@ int g4b_fft_init(g4b_fft* s, double delz, double dgrid, double xks, int ngrid) {
   if (!(s->ready && s->ngrid == ngrid && s->dgrid == dgrid && s->xks == xks)) {
     const int n = ngrid;
     const long double pi = 3.141592653589793238462643383279502884L;
-    std::vector<double2> tw(kFftM), chirp(n), wn(n);
+    std::vector<double2> tw(kTwAll + kFftM), chirp(n), wn(2 * n);  // second words behind
     for (int j = 0; j < kFftM; ++j) {
       const long double ang = -2.0L * pi * j / kFftM;
-      tw[j] = make_double2((double)cosl(ang), (double)sinl(ang));
+      split(cosl(ang), sinl(ang), tw[j], tw[kTwAll + j]);
+    }
+    for (int i = 0; i < 3; ++i) {
+      for (int t = 0; t < kLineT; ++t) tw[kTwA + i * kLineT + t] = tw[t << i];
+      for (int t = 0; t < 8; ++t) tw[kTwB + i * 8 + t] = tw[8 * t << i];
     }
     std::vector<cld> hfw(kFftM, 0), hiw(kFftM, 0);
     for (int j = 0; j < n; ++j) {
@@ -588,7 +650,7 @@ int g4b_fft_init(g4b_fft* s, double delz, double dgrid, double xks, int ngrid) {
       const cld w(cosl(ang), sinl(ang));
       chirp[j] = make_double2((double)w.real(), (double)w.imag());
       const long double turn = 2.0L * pi * (long double)j / n;
-      wn[j] = make_double2((double)cosl(turn), (double)sinl(turn));
+      split(cosl(turn), sinl(turn), wn[j], wn[n + j]);
       hfw[j] = std::conj(w);
       hiw[j] = w;
       if (j > 0) {
@@ -627,7 +689,7 @@ int g4b_fft_init(g4b_fft* s, double delz, double dgrid, double xks, int ngrid) {
     if (int rc = upload(c, &s->k1, k1)) return rc;
     if (int rc = upload(c, &s->sig_t, sig_t)) return rc;
     if (!s->hc)  // the spectrum, then the kernel itself
-      G4B_CUDA_TRY(dev_alloc(c, (void**)&s->hc, (kFftM + kFftMaxN) * sizeof(double2)));
+      G4B_CUDA_TRY(dev_alloc(c, (void**)&s->hc, (kFftM + 2 * kFftMaxN) * sizeof(double2)));
     s->prop_delz = std::nan("");
     s->filter = s->want_filter && shape_ok;
     s->ngrid = n;
