@@ -92,11 +92,16 @@ bool prepare(const g4h_engine_config& cfg, const Undulator& lat, const g4h_job& 
 }
 
 // Device bytes a job will hold (particles 28 B, per plane a + b + source tile,
-// diagnostics history of one step), for admission.
+// diagnostics history of one step), for admission.  Runs of few slices hold a tile
+// of 12 bytes per cell as well, where a slice of more than kTileCells cells keeps
+// only so many; the engine's own line, 21 slices on 148 SMs, moves with the SMs.
 double estimate_bytes(const g4h_job& j) {
+  constexpr double kTileCells = 65536;
+  constexpr int kTileSlices = 32;
   const double n = j.ngrid, ld = n + ((int)n & 1);
   const double planes = 3.0 * j.nslice * n * ld * 8;
-  return 28.0 * j.nslice * j.npart + planes + 4096.0 * j.nslice + (1 << 20);
+  const double tiles = j.nslice <= kTileSlices ? 12.0 * j.nslice * std::min(n * ld, kTileCells) : 0.0;
+  return 28.0 * j.nslice * j.npart + planes + tiles + 8192.0 * j.nslice + (1 << 20);
 }
 
 int create_run(g4b_ctx* ctx, const g4h_engine_config& cfg, const g4h_job& j,
@@ -345,6 +350,15 @@ int g4h_scan(const g4h_engine_config* cfg, const g4h_job* jobs, int njobs,
     set_error(e.what());
     return G4B_ERR_CUDA;
   }
+}
+
+int g4h_job_bytes(const g4h_job* job, double* bytes) {
+  if (!job || !bytes) {
+    set_error("g4h_job_bytes: null argument");
+    return G4B_ERR_ARG;
+  }
+  *bytes = estimate_bytes(*job);
+  return G4B_OK;
 }
 
 // Served request stream with continuous batching.  Request i arrives at

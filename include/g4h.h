@@ -182,6 +182,9 @@ typedef struct g4h_serve_stats {
  * null. */
 int g4h_scan(const g4h_engine_config* cfg, const g4h_job* jobs, int njobs,
              g4h_scan_result* result, double* final_power, double* records);
+/* Device memory that g4h_serve sets aside for a job when it admits it: at least
+ * what its run holds. */
+int g4h_job_bytes(const g4h_job* job, double* bytes);
 /* arrival[njobs] in seconds from the start, non-decreasing; latency[njobs]
  * receives completion - arrival. */
 int g4h_serve(const g4h_engine_config* cfg, const g4h_job* jobs, const double* arrival,

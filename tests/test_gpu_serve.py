@@ -1,8 +1,11 @@
 """Batched scan and served stream (C++ drivers on the batch engine): each
 run's results are the same alone and in the mix, exactly."""
+import ctypes
+
 import numpy as np
 import pytest
 
+from genesis4_cuda_port_b200 import device as dev
 from genesis4_cuda_port_b200 import host, workloads
 
 pytestmark = pytest.mark.gpu
@@ -51,6 +54,23 @@ def test_scan_batched_equals_one_at_a_time():
     assert np.array_equal(p_b, p_s)
     assert np.all(p_b > 0)
     assert all(g > 0 for g in r_b.grids)
+
+
+@pytest.mark.parametrize("nslice,ngrid", [(1, 255), (4, 401), (21, 101), (22, 101), (60, 64)])
+def test_memory_set_aside_covers_the_run(nslice, ngrid):
+    """Admission counts every allocation of the run, the shared tiles of runs of
+    few slices included, and not half as much again."""
+    wl, npart = workloads.sase(), 256
+    job = workloads._job(wl, nslice=nslice, ngrid=ngrid, npart=npart, nsteps=4,
+                         time_run=int(nslice > 1), taper=0.0, seed_power=1e3, seed=1)
+    aside = ctypes.c_double()
+    assert host.load().g4h_job_bytes(ctypes.byref(job), ctypes.byref(aside)) == 0
+    ctx = dev.Context(0)
+    run = dev.Run(ctx, npart * np.arange(nslice + 1), fields=[(1, ngrid, job.gridmax)],
+                  lambda0=wl.lambda0, gamma_ref=wl.gamma0, nbunch=1)
+    held = run.device_bytes()
+    run.close()
+    assert held <= aside.value < 1.5 * held + (1 << 21)
 
 
 def test_served_results_equal_alone():
