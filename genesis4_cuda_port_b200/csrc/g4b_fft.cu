@@ -44,10 +44,10 @@
 // an SM clock per warp each) and the exchanges (64 16-byte accesses per thread,
 // four clocks per warp each) take about the same time, some 600 clocks per line
 // together when overlapped; measured, 1024 slices of 201^2 (CUDA events): rows
-// 0.61 ms, columns 0.93 ms, against 1.27 + 2.31 + 1.59 ms for the forward, middle
+// 0.62 ms, columns 0.94 ms, against 1.27 + 2.31 + 1.59 ms for the forward, middle
 // and inverse passes of a full transform pair with a line per warp (sixteen
 // values per thread, 128 registers); cuFFT's forward and inverse pair takes 4.99
-// ms.  The field step with its source: 5.48 -> 1.74 ms.  The order of the spectrum
+// ms.  The field step with its source: 5.48 -> 1.76 ms.  The order of the spectrum
 // (thread t, slot s) -> k = t / 8 + 8 (t % 8) + 64 brev3(s) is seen by the
 // pointwise multiply alone.
 #include <algorithm>
